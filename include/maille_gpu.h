@@ -48,7 +48,10 @@ typedef enum {
                          solution accumulation, FP64 refinement dots, FP64 factor pivots) */
 } MaillePrecision;
 
-/* Ordering of the free nodes for the level-scheduled IC(0). */
+/* Ordering of the free nodes for the level-scheduled IC(0). With the multicolour orderings the
+ * elastic PCG's preconditioner is IC(0) plus a coarse correction (a trilinear box grid over the mesh
+ * with its Galerkin matrix inverted densely): the same stopping test, statuses and results, in
+ * 5 to 12 times fewer iterations. RCM keeps IC(0) alone, for the reference's iteration counts. */
 typedef enum {
     MAILLE_ORDER_AUTO = 0,           /* the path's measured best: MULTICOLOR_ITERATED for the
                                         elastic solves, MULTICOLOR_BFS for the thermal step */
@@ -210,7 +213,8 @@ int32_t maille_gpu_spmv_device(MailleGpuHandle* h, int32_t precision, int32_t co
  * No counterpart in the reference. */
 int64_t maille_gpu_kernel_launches(void);
 
-/* Raise (1) or clear (0) the cancel flag; checked between PCG iteration chunks. Safe to call
+/* Raise (1) or clear (0) the cancel flag; checked before the PCG's first launch and between its
+ * launches. Safe to call
  * from another thread while a solve runs (the Observer / Flow::Stop role, model.rs:1203-1218). */
 void maille_gpu_cancel(MailleGpuHandle* h, int32_t flag);
 

@@ -13,9 +13,10 @@ import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 SRC = [os.path.join(HERE, "csrc", f) for f in ("setup.cpp", "kernels.cu", "sparse.cu", "persist.cu", "solver.cu", "noalloc.cu",
-                                                        "batch_kernels.cu", "batch.cu", "large_strain.cu", "analysis.cu", "memory.cu", "thermal.cu", "ordering.cu")]
+                                                        "batch_kernels.cu", "batch.cu", "large_strain.cu", "analysis.cu", "memory.cu", "thermal.cu", "ordering.cu", "coarse.cu")]
 HDR = [os.path.join(HERE, "csrc", f) for f in ("common.hpp", "kernels.cuh", "sparse.cuh", "reduce.cuh",
-                                                         "cuda_host.hpp", "batch.cuh", "handle.hpp", "analysis.cuh", "tet.cuh", "ordering.cuh")] + [
+                                                         "cuda_host.hpp", "batch.cuh", "handle.hpp", "analysis.cuh", "tet.cuh", "ordering.cuh",
+                                                         "coarse.cuh", "coarse_dev.cuh")] + [
     os.path.join(HERE, "..", "include", "maille_gpu.h")]
 LIB = os.path.join(HERE, "libmaille_gpu.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")

@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include "analysis.cuh"
+#include "coarse.cuh"
 #include "common.hpp"
 #include "cuda_host.hpp"
 #include "kernels.cuh"
@@ -133,6 +134,7 @@ struct MailleGpuHandle {
     double* ke = nullptr;
     double *K = nullptr, *F = nullptr;
     SellBuf sk;      // K, sliced, for the SpMV
+    Coarse coarse;   // the preconditioner's coarse correction (multicolour orderings)
     PsellBuf pl, pu;  // strictly lower / upper blocks of the factor, packed, for the sweeps
     double *Ks64 = nullptr, *Ls64 = nullptr, *Us64 = nullptr, *D64 = nullptr;
     float *Ks32 = nullptr, *Ls32 = nullptr, *Us32 = nullptr, *D32 = nullptr;

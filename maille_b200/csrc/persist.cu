@@ -36,9 +36,11 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <utility>
 
 #include <cooperative_groups.h>
 
+#include "coarse_dev.cuh"
 #include "cuda_host.hpp"
 #include "reduce.cuh"
 #include "sparse.cuh"
@@ -779,6 +781,7 @@ __global__ void __launch_bounds__(kPW * 32, 2) k_pcg(PcgArgs<T> a, int init) {
             s->iter, s->max_iter, s->done, s->status, s->updates, s->epoch};
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
+    const int32_t gwarp = (int32_t)(blockIdx.x * kPW) + warp, nwarps = (int32_t)(gridDim.x * kPW);
     const bool timed = a.timing != nullptr && blockIdx.x == 0 && threadIdx.x == 0;
     unsigned long long t_last = timed ? gtime() : 0;
     auto mark = [&](int phase) {
@@ -909,8 +912,21 @@ __global__ void __launch_bounds__(kPW * 32, 2) k_pcg(PcgArgs<T> a, int init) {
             grid.sync();
             mark(3);
         }
+        // the coarse correction's restriction of r runs before the backward sweep and is gathered after
+        // it, so the grid barrier between the two is waited for behind the sweep
+        cg::grid_group::arrival_token restricted{};
+        if (a.c.nn) {
+            coarse_restrict<T, 3>(a.c, a.r, gwarp, nwarps);
+            restricted = grid.barrier_arrive();
+        }
         v.epoch += 1;
         loc = sweep<T, false>(a.U, v.epoch, a.Uv, a.D, a.nb, a.r, a.z, stage, ok);
+        if (a.c.nn) {
+            grid.barrier_wait(std::move(restricted));
+            coarse_gather<T, 3>(a.c, tid, nthreads);
+            grid.sync();
+            loc += coarse_apply<T, 3>(a.c, gwarp, nwarps);
+        }
         if (!ok) atomicExch(timeout, 1);
         publish(loc, a.partials, 3, sh);
         grid.sync();
@@ -923,15 +939,29 @@ __global__ void __launch_bounds__(kPW * 32, 2) k_pcg(PcgArgs<T> a, int init) {
         const double rz = grid_total(a.partials, 3);
         v.beta = init ? 0.0 : rz / v.rz;  // iterative.rs:237-239
         v.rz = rz;
-        // p = z + beta p (iterative.rs:240-242)
+        // p = z + beta p (iterative.rs:240-242), z taking its coarse part P y here (y in the staging
+        // buffers' shared memory: every node reads its cell's 8 corners)
+        T* ys = reinterpret_cast<T*>(stage_mem);
+        if (a.c.nn) {
+            for (int32_t k = threadIdx.x; k < 4 * a.c.nn; k += blockDim.x) ys[k] = __ldcg(a.c.y + k);
+            __syncthreads();
+        }
         for (int64_t i = tid; i < a.nb; i += nthreads) {
             double zv[3], pv[4];
             rec_get(a.z, i, zv);
             get4(a.p, i, pv);
+            if (a.c.nn) {
+                T cv[3];
+                coarse_interpolate3(a.c.w, i, ys, a.c.kx + 1, (a.c.kx + 1) * (a.c.ky + 1), cv);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) zv[c] += (double)cv[c];
+            }
 #pragma unroll
             for (int c = 0; c < 3; ++c) pv[c] = (double)(T)(zv[c] + v.beta * pv[c]);
             set4(a.p, i, pv);
         }
+        // the buffers written above are the next bulk copies' targets
+        if (a.c.nn) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         grid.sync();
         mark(5);
         ++it;

@@ -65,6 +65,7 @@ MailleGpuHandle::~MailleGpuHandle() {
     sk.gather(all);
     pl.gather(all);
     pu.gather(all);
+    coarse.gather(all);
     device_free_all(all);
     const double t1 = now_ms();
     pinned_slot_free(h_scal);
@@ -122,6 +123,8 @@ PcgArgs<T> pcg_args(MailleGpuHandle* h, const T* Kv, const T* Lv, const T* Uv, c
     a.partials = h->partials;
     a.timing = h->timing;
     a.claim = h->claim;
+    if constexpr (sizeof(T) == 4) a.c = h->coarse.dev32();
+    else a.c = h->coarse.dev64();
     return a;
 }
 
@@ -140,6 +143,14 @@ int32_t run_pcg_persistent(MailleGpuHandle* h, int32_t* iterations, int32_t* upd
         }
     };
     CK(cudaMemsetAsync(h->claim, 0, 4 * sizeof(int32_t), st));
+    // a flag that is already up stops the solve before its first launch: a whole solve may take fewer
+    // iterations than one launch runs
+    if (h->cancel.load()) {
+        *iterations = 0;
+        *updates = 0;
+        *rel_res = 1.0;
+        return MAILLE_CANCELLED;
+    }
     launch(true);
     int32_t status = MAILLE_OK;
     for (;;) {
@@ -299,6 +310,7 @@ int32_t assemble_factor(MailleGpuHandle* h, Error& err) {
         launch_sell_fill<double>(h->pu.h.steps(), h->pu.src, h->F, h->Us64, st);
         launch_diag_fill<double>(s.nb, h->diag, h->F, h->D64, st);
     }
+    h->coarse.update(h->K, st);
     CK(cudaGetLastError());
     CK(cudaEventRecord(h->ev[3], st));
     return MAILLE_OK;
@@ -360,6 +372,7 @@ int32_t create_impl(const MailleElasticProblem* p, MailleGpuHandle** out, Maille
     // the step 4 % shorter than MULTICOLOR)
     const int ordering = p->ordering == MAILLE_ORDER_AUTO ? MAILLE_ORDER_MULTICOLOR_ITERATED : p->ordering;
     std::vector<int32_t> kept, kept_of;
+    std::vector<double> box(6, 0.0);  // of the nodes, for the coarse grid
     const double t_setup0 = now_ms();
     double t_setup1 = t_setup0;
     bool analysed = false;
@@ -380,6 +393,7 @@ int32_t create_impl(const MailleElasticProblem* p, MailleGpuHandle** out, Maille
         h->h_f.assign(n3, 0.0);
         if (p->f) std::memcpy(h->h_f.data(), p->f, n3 * sizeof(double));
         h->h_f0 = h->h_f;
+        coarse_box(p->coords, 0, p->n_nodes, box.data());
         t_setup1 = now_ms();
     });
     struct Joiner {
@@ -506,6 +520,12 @@ int32_t create_impl(const MailleElasticProblem* p, MailleGpuHandle** out, Maille
             h->pl.upload(pt, s.nb, st);
             h->pu.upload(pt, s.nb, st);
         }
+        // the coarse correction, with the multicolour orderings (RCM stands for the reference's own
+        // iteration counts). MAILLE_COARSE=0: IC(0) alone (a measurement knob)
+        if (ordering != MAILLE_ORDER_RCM && env_int("MAILLE_COARSE", 1) != 0)
+            h->coarse.plan(3, is_mixed(h.get()), s.nb, s.blocks, h->coords, h->perm, h->fixmask, h->row_ptr, h->col,
+                           nullptr, box, {(int64_t)s.nb}, st);
+        tmark("coarse plan");
         CK(cudaEventRecord(h->ev[11], st));  // pattern and layouts on the device
         h->belem = dupload(s.belem.data(), s.belem.size(), st);
         h->bnodes = dupload(s.bnodes.data(), s.bnodes.size(), st);

@@ -15,6 +15,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "coarse.cuh"
+
 namespace maille {
 
 constexpr int kLaneSlots = 4;    // slots (blocks) per lane per step
@@ -81,6 +83,7 @@ struct PcgArgs {
     PcgScalars* s;
     int32_t* claim;  // claim[2]: the sweeps' timeout flag
     double* partials;       // [4 * grid]
+    CoarseDev<T> c;         // the preconditioner's coarse correction (c.nn = 0: none)
     unsigned long long* timing;  // optional [8] ns per phase (block 0): spmv, axpy, update, fwd, bwd, p
 };
 template <typename T, bool MIXED>

@@ -1,0 +1,79 @@
+"""The coarse correction of the IC(0) preconditioner (coarse.cuh): the corrected PCG solves the same
+systems as IC(0) alone, in fewer iterations, over the shapes of its grid: one cell, cells without nodes,
+thin plates and bars, sweep tiles of 64 unknowns that are not full, fixed components, parts that a
+cell holds together, and load cases on one factor."""
+import numpy as np
+import pytest
+
+import maille_b200 as mb
+from maille_b200 import meshgen as mg
+from maille_b200._lib import MAILLE_FP64, MAILLE_MIXED, MAILLE_ORDER_MULTICOLOR
+
+import cases
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return np.linalg.norm(a - b) / np.linalg.norm(b)
+
+
+def box(cells, size, quadratic):
+    p = mg.clamped_cube(cells, quadratic, 50000.0 + 150000.0 * mg.uniform(21, 6 * int(np.prod(cells))), size=size)
+    rollers = np.nonzero(np.abs(p.coords[:, 0]) < 1e-12)[0]
+    p.fixed[3 * rollers] = 1  # rows with one fixed component
+    return p
+
+
+def frame():
+    """Two separate blocks with empty cells between them."""
+    return cases.two_blocks(5)
+
+
+SHAPES = {
+    "cube_below_the_limit": lambda: box((4, 4, 4), (1.0, 1.0, 1.0), False),
+    "cube": lambda: box((9, 9, 9), (1.0, 1.0, 1.0), False),
+    "plate": lambda: box((24, 18, 1), (2.4, 1.8, 0.1), False),
+    "bar": lambda: box((2, 2, 60), (0.1, 0.1, 3.0), False),
+    "ragged_tet10": lambda: box((7, 4, 5), (1.3, 0.7, 1.0), True),
+    "two_blocks": frame,
+}
+
+
+@pytest.mark.parametrize("shape", sorted(SHAPES))
+def test_the_corrected_pcg_solves_the_same_system(gpu, oracle_lib, monkeypatch, shape):
+    # 1e-10 of the oracle at 1e-13, the tolerance of the parity tests
+    p = SHAPES[shape]()
+    ref = oracle_lib.model_solve(p, solver=2, tol=1e-13)
+    m = mb.Model.from_arrays(p.coords, p.conn, p.young, p.poisson, p.fixed, p.imposed, p.loads,
+                             (p.p_elem, p.p_face, p.p_value))
+    m.with_solver(mb.SolverKind.ITERATIVE).with_tolerance(1e-13)
+    iterations = {}
+    for knob in ("0", "1"):
+        monkeypatch.setenv("MAILLE_COARSE", knob)
+        f = m.solve()
+        assert rel(f.displacements, ref["u"]) < 1e-10
+        assert rel(f.reactions, ref["reactions"]) < 1e-10
+        iterations[knob] = f.info["iterations"]
+    # fewer wherever the mesh is several cells from its supports (the plate is clamped on its whole
+    # face: there is nothing for a coarse grid to carry)
+    if shape in ("cube", "bar", "ragged_tet10"):
+        assert iterations["1"] < iterations["0"]
+
+
+@pytest.mark.parametrize("precision,tol,err", [(MAILLE_FP64, 1e-13, 1e-10), (MAILLE_MIXED, 1e-10, 1e-8)])
+def test_new_moduli_renew_the_correction(gpu, oracle_lib, precision, tol, err):
+    p = box((8, 6, 7), (1.0, 0.8, 0.9), True)
+    m = mb.Model.from_arrays(p.coords, p.conn, p.young, p.poisson, p.fixed, p.imposed, p.loads,
+                             (p.p_elem, p.p_face, p.p_value))
+    m.with_solver(mb.SolverKind.ITERATIVE).with_tolerance(tol).with_precision(precision)
+    m.ordering = MAILLE_ORDER_MULTICOLOR
+    with mb.SolverHandle(m) as h:
+        first = h.solve()
+        p.young = 210000.0 * (0.01 + 0.99 * mg.uniform(22, p.n_elems)) ** 3
+        h.refactor(young=p.young)
+        a, b = h.solve(), h.solve()
+    ref = oracle_lib.model_solve(p, solver=2, tol=1e-14)
+    assert rel(a.displacements, ref["u"]) < err
+    assert np.array_equal(a.displacements, b.displacements)
+    assert a.info["iterations"] < 3 * first.info["iterations"]
