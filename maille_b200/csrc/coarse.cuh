@@ -105,7 +105,7 @@ constexpr uint32_t kCoarseBase = (1u << 28) - 1u;
 
 // Host bounding box of the nodes [n0, n1) of xyz into box[6] (min x, y, z, max x, y, z).
 void coarse_box(const double* xyz, int64_t n0, int64_t n1, double box[6]);
-// Cells per axis for `rows` rows in the box.
-void coarse_cells(const double box[6], int64_t rows, int32_t k[3]);
+// Cells per axis for `rows` rows of `dof` unknowns in the box.
+void coarse_cells(int dof, const double box[6], int64_t rows, int32_t k[3]);
 
 }  // namespace maille

@@ -39,17 +39,24 @@ __device__ __forceinline__ void coarse_weights(const T f[3], T w[8]) {
     w[4] = x0 * c; w[5] = x1 * c; w[6] = x0 * d; w[7] = x1 * d;
 }
 
-__device__ __forceinline__ void coarse_load_r(const float* r, int64_t i, float v[3]) {
-    const float4 q = __ldcg(reinterpret_cast<const float4*>(r) + i);
-    v[0] = q.x; v[1] = q.y; v[2] = q.z;
+// the DOF residuals of row i: r is padded to 4 entries a row when DOF is 3, plain when it is 1
+template <int DOF>
+__device__ __forceinline__ void coarse_load_r(const float* r, int64_t i, float* v) {
+    if constexpr (DOF == 3) {
+        const float4 q = __ldcg(reinterpret_cast<const float4*>(r) + i);
+        v[0] = q.x; v[1] = q.y; v[2] = q.z;
+    } else {
+        v[0] = __ldcg(r + i);
+    }
 }
-__device__ __forceinline__ void coarse_load_r(const double* r, int64_t i, double v[3]) {
-    const double2 q = __ldcg(reinterpret_cast<const double2*>(r + 4 * i));
-    v[0] = q.x; v[1] = q.y; v[2] = __ldcg(r + 4 * i + 2);
-}
-template <typename T>
-__device__ __forceinline__ void coarse_load_r(const T* r, int64_t i, T v[1]) {
-    v[0] = __ldcg(r + i);
+template <int DOF>
+__device__ __forceinline__ void coarse_load_r(const double* r, int64_t i, double* v) {
+    if constexpr (DOF == 3) {
+        const double2 q = __ldcg(reinterpret_cast<const double2*>(r + 4 * i));
+        v[0] = q.x; v[1] = q.y; v[2] = __ldcg(r + 4 * i + 2);
+    } else {
+        v[0] = __ldcg(r + i);
+    }
 }
 
 // one halving step of a transposed warp sum: N values a lane, N / 2 after it
@@ -77,7 +84,7 @@ __device__ __noinline__ void coarse_restrict(const CoarseDev<T> c, const T* r, i
             T f[3], w[8], v[DOF];
             uint32_t row;
             coarse_row(c.ws, p, f, row);
-            coarse_load_r(r, (int64_t)row, v);
+            coarse_load_r<DOF>(r, (int64_t)row, v);
             coarse_weights(f, w);
 #pragma unroll
             for (int a = 0; a < 8; ++a)

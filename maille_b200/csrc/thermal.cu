@@ -34,12 +34,14 @@
 #include <string>
 #include <thread>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "analysis.cuh"
+#include "coarse_dev.cuh"
 #include "common.hpp"
 #include "cuda_host.hpp"
 #include "kernels.cuh"
@@ -517,6 +519,7 @@ struct HeatPcg {
     double* x64;                     // [nb + 1] the FP64 solution
     double* r64;                     // [nb + 1] the true residual b - A x64
     double delta;                    // reliable update when ||r|| fell below delta x its last true value
+    CoarseDev<T> c;                  // the preconditioner's coarse correction (c.nn = 0: none)
 };
 
 __device__ __forceinline__ unsigned long long heat_clock() {
@@ -782,6 +785,7 @@ __device__ __forceinline__ void st2(float* p, double a, double b) {
 template <typename T, bool MIXED>
 __global__ void __launch_bounds__(kT, 2) k_heat_pcg(HeatPcg<T> a) {
     __shared__ double sh[kT / 32];
+    extern __shared__ __align__(16) unsigned char coarse_mem[];  // y of the coarse correction
     cg::grid_group grid = cg::this_grid();
     const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
     if (*a.status != 0) {  // gated off before the launch (an earlier failure, or cancelled)
@@ -817,15 +821,58 @@ __global__ void __launch_bounds__(kT, 2) k_heat_pcg(HeatPcg<T> a) {
     heat_publish(loc, a.partials, 3, sh);
     grid.sync();
     const double bnorm = sqrt(heat_total(a.partials, 3));
+    // z = (L L^T)^-1 r by the sweeps, the coarse correction's y = E^-1 P^T r beside them (the barrier
+    // between its restriction and its gather is waited for behind the sweeps); this thread's share
+    // of r . (z + P y)
+    auto precondition = [&]() {
+        cg::grid_group::arrival_token restricted{};
+        const int32_t warp = (int32_t)(tid >> 5), warps = (int32_t)(nth >> 5);
+        if (a.c.nn) {
+            coarse_restrict<T, 1>(a.c, a.r, warp, warps);
+            restricted = grid.barrier_arrive();
+        }
+        double rz = heat_sweeps(a, ++epoch);
+        if (a.c.nn) {
+            grid.barrier_wait(std::move(restricted));
+            coarse_gather<T, 1>(a.c, tid, nth);
+            grid.sync();
+            rz += coarse_apply<T, 1>(a.c, warp, warps);
+        }
+        return rz;
+    };
+    // p = z + P y + beta p, two entries per thread and pass
+    auto update_p = [&](double beta) {
+        T* ys = reinterpret_cast<T*>(coarse_mem);
+        if (a.c.nn) {
+            for (int32_t k = threadIdx.x; k < a.c.nn; k += blockDim.x) ys[k] = __ldcg(a.c.y + k);
+            __syncthreads();
+        }
+        const int32_t sy = a.c.kx + 1, sz = sy * (a.c.ky + 1);
+        for (int64_t i2 = tid; 2 * i2 < a.nb; i2 += nth) {
+            const int64_t i = 2 * i2;
+            const bool two = i + 1 < a.nb;
+            double z0 = (double)__ldcg(&a.zrec[i].x), z1 = two ? (double)__ldcg(&a.zrec[i + 1].x) : 0.0;
+            if (a.c.nn) {
+                z0 += (double)coarse_interpolate1(a.c.w, i, ys, sy, sz);
+                if (two) z1 += (double)coarse_interpolate1(a.c.w, i + 1, ys, sy, sz);
+            }
+            if (two) {
+                const double2 pv = ld2(a.p + i);
+                st2(a.p + i, z0 + beta * pv.x, z1 + beta * pv.y);
+            } else {
+                a.p[i] = (T)(z0 + beta * (double)__ldcg(a.p + i));
+            }
+        }
+    };
     double maxr = bnorm;  // mixed: the last true residual norm
     int32_t status = 0, it = 0;
     double rel = 0.0;
     if (bnorm > 0.0) {
-        loc = heat_sweeps(a, ++epoch);
+        loc = precondition();
         heat_publish(loc, a.partials, 2, sh);
         grid.sync();
         double rz = heat_total(a.partials, 2);
-        for (int64_t i = tid; i < a.nb; i += nth) a.p[i] = (T)__ldcg(&a.zrec[i].x);
+        update_p(0.0);
         grid.sync();
         for (;;) {
             if (__ldcg(a.timeout)) {
@@ -923,7 +970,7 @@ __global__ void __launch_bounds__(kT, 2) k_heat_pcg(HeatPcg<T> a) {
                     break;
                 }
             }
-            loc = heat_sweeps(a, ++epoch);
+            loc = precondition();
             heat_publish(loc, a.partials, 2, sh);
             grid.sync();
             mark(2);
@@ -934,16 +981,7 @@ __global__ void __launch_bounds__(kT, 2) k_heat_pcg(HeatPcg<T> a) {
             const double rz_next = heat_total(a.partials, 2);
             const double beta = rz_next / rz;
             rz = rz_next;
-            for (int64_t i2 = tid; 2 * i2 < a.nb; i2 += nth) {
-                const int64_t i = 2 * i2;
-                if (i + 1 < a.nb) {
-                    const double z0 = (double)__ldcg(&a.zrec[i].x), z1 = (double)__ldcg(&a.zrec[i + 1].x);
-                    const double2 pv = ld2(a.p + i);
-                    st2(a.p + i, z0 + beta * pv.x, z1 + beta * pv.y);
-                } else {
-                    a.p[i] = (T)((double)__ldcg(&a.zrec[i].x) + beta * (double)__ldcg(a.p + i));
-                }
-            }
+            update_p(beta);
             grid.sync();
             mark(3);
         }
@@ -1115,6 +1153,26 @@ bool finite_all(const double* v, int64_t n) {
     return true;
 }
 
+// Whether the coarse correction (coarse.cuh) pays for this step. IC(0) alone carries a correction over
+// the diffusion length of an increment, so its iterations follow lambda = theta dt k / (rho c h^2) (h: the
+// node spacing) until the mesh ends: about 18 sqrt(lambda), at most 4.3 nb^(1/3), at tol 1e-12; with the
+// correction 20 to 30, each a quarter dearer. Measured (Tet4 and Tet10 cubes, IC(0) / corrected):
+// lambda 0.9 20 / 21, 1.8 24 / 20, 4.8 40 / 23, 9.3 57 / 27, 12 52 / 26, 73 103 / 38 (Tet10 40^3); steady
+// 28 / 21 with 294 free nodes, 53 / 23 with 2028, 127 / 30 with 23548. The plan and the inverse cost
+// about as much as 15 iterations once a step.
+bool coarse_pays(const MailleThermalProblem* p, const std::vector<double>& box, int64_t nb) {
+    double k = 0.0, rc = 0.0, vol = 1.0;
+    for (int64_t e = 0; e < p->n_elems; ++e) {
+        k += p->conductivity[e];
+        rc += p->rho_c[e];
+    }
+    for (int a = 0; a < 3; ++a) vol *= std::max(0.0, box[3 + a] - box[a]);
+    const double h2 = std::cbrt(vol / (double)nb) * std::cbrt(vol / (double)nb);
+    const double lambda = rc > 0.0 && h2 > 0.0 ? p->theta * p->time_step * k / (rc * h2) : INFINITY;
+    const double alone = std::min(18.0 * std::sqrt(lambda), 4.3 * std::cbrt((double)nb));
+    return (alone - 32.0) * p->increments >= 15.0;
+}
+
 int32_t check_thermal(const MailleThermalProblem* p, std::string& why) {
     auto bad = [&](const std::string& m) {
         why = m;
@@ -1189,6 +1247,7 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
     const char* host_env = std::getenv("MAILLE_HOST_ORDERING");
     const bool host_ordering = host_env && std::atoi(host_env) != 0;
     std::vector<int32_t> kept, kept_of;
+    std::vector<double> box(6, 0.0);  // of the nodes, for the coarse grid
     std::thread analysis([&] {
         if (host_ordering)
             analysed = analyse(n, npe, ne, p->conn, fixed3.data(), ordering, sym, err, /*pattern=*/false,
@@ -1196,6 +1255,7 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
         else
             analysed = analyse_topology(n, npe, ne, p->conn, fixed3.data(), sym, kept, kept_of, err,
                                         /*boundary_lists=*/false, /*incidence=*/false);
+        coarse_box(p->coords, 0, n, box.data());
         t_setup1 = now_ms();
     });
     struct Joiner {
@@ -1208,6 +1268,7 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
     cudaStream_t st = nullptr;
     cudaEvent_t ev[7] = {};
     DevBufs mem;
+    Coarse coarse;
     Slices sk, sl, su;
     sk.kind = SELL_FULL;
     sl.kind = SELL_LOWER;
@@ -1337,6 +1398,10 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
         sk.upload(pt, nb, st);
         sl.upload(pt, nb, st);
         su.upload(pt, nb, st);
+        if (const char* e = std::getenv("MAILLE_COARSE");
+            ordering != MAILLE_ORDER_RCM && !(e && std::atoi(e) == 0) && coarse_pays(p, box, nb))
+            coarse.plan(1, p->precision == MAILLE_MIXED, nb, pt.blocks, coords, perm, nullptr, pt.row_ptr, pt.col, nullptr,
+                        box, {(int64_t)nb}, st);
         // assembly of the left and right matrices on the free-node pattern
         double* A = mem.take(dalloc<double>((size_t)pt.blocks));
         double* R = mem.take(dalloc<double>((size_t)pt.blocks));
@@ -1369,6 +1434,8 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
             }
         }
         if (shift_used < 0.0) return th_fail(MAILLE_SINGULAR, "Singular: IC(0) failed for every diagonal shift");
+        // the coarse correction, as in the elastic solve (solver.cu)
+        coarse.update(A, st);
         // iteration operands
         auto slots = [&](const Slices& s) { return (int64_t)s.h.steps() * kStepSlots; };
         double* Av = mem.take(dalloc<double>((size_t)slots(sk)));
@@ -1483,7 +1550,8 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
         int per_sm = 0, sms = 0, dev = p->device;
         void* pcg_fn = mixed ? (void*)k_heat_pcg<float, true> : (void*)k_heat_pcg<double, false>;
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pcg_fn, kT, 0));
+        const size_t csmem = coarse.active() ? (size_t)coarse.dev64().nn * (mixed ? 4 : 8) : 0;  // y
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pcg_fn, kT, csmem));
         const int grid = sms * std::min(per_sm, 2);
         if (grid <= 0) return th_fail(MAILLE_CUDA_ERROR, "the PCG kernel does not fit on the device");
         double* partials = mem.take(dalloc<double>((size_t)4 * grid));
@@ -1508,18 +1576,18 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
                 HeatPcg<double> a{nb, sk.dev(), sl.dev(), su.dev(), bwd_slice, Av, Lv, Uv, D, b, x, r, pp, ap,
                                   yrec, zrec, partials, timeout, (unsigned long long)s << 32, tol, max_iter,
                                   d_status + (s - 1), d_iters + (s - 1), d_rel + (s - 1), timing,
-                                  nullptr, nullptr, nullptr, 0.0};
+                                  nullptr, nullptr, nullptr, 0.0, coarse.dev64()};
                 void* args[] = {&a};
-                CK(cudaLaunchCooperativeKernel(pcg_fn, dim3(grid), dim3(kT), args, 0, st));
+                CK(cudaLaunchCooperativeKernel(pcg_fn, dim3(grid), dim3(kT), args, csmem, st));
             } else {
                 // 32-bit tags: increment s starts after the sweeps every earlier increment can take
                 const unsigned long long epoch0 = (unsigned long long)(s - 1) * ((unsigned long long)max_iter + 2);
                 HeatPcg<float> a{nb, sk.dev(), sl.dev(), su.dev(), bwd_slice, Av32, Lv32, Uv32, D32, b, x32, r32,
                                  p32, ap32, yrec32, zrec32, partials, timeout, epoch0, tol, max_iter,
                                  d_status + (s - 1), d_iters + (s - 1), d_rel + (s - 1), timing,
-                                 Av, x, r64, kHeatDelta};
+                                 Av, x, r64, kHeatDelta, coarse.dev32()};
                 void* args[] = {&a};
-                CK(cudaLaunchCooperativeKernel(pcg_fn, dim3(grid), dim3(kT), args, 0, st));
+                CK(cudaLaunchCooperativeKernel(pcg_fn, dim3(grid), dim3(kT), args, csmem, st));
             }
             counted();
             k_heat_scatter<<<grid_of(n), kT, 0, st>>>(n, inv, fixed, imp, x, temps + (size_t)s * n);

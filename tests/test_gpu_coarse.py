@@ -77,3 +77,21 @@ def test_new_moduli_renew_the_correction(gpu, oracle_lib, precision, tol, err):
     assert rel(a.displacements, ref["u"]) < err
     assert np.array_equal(a.displacements, b.displacements)
     assert a.info["iterations"] < 3 * first.info["iterations"]
+
+
+@pytest.mark.parametrize("quadratic,cells,precision", [(False, 5, MAILLE_FP64), (False, 13, MAILLE_FP64),
+                                                       (True, 7, MAILLE_FP64), (True, 7, MAILLE_MIXED)])
+def test_the_thermal_step_takes_the_correction(gpu, oracle_lib, monkeypatch, quadratic, cells, precision):
+    # 1e-9 of the largest temperature, as the thermal parity tests; fewer iterations where the diffusion
+    # length of an increment spans many nodes, the same on the small cube, where the step leaves it out
+    from maille_b200 import thermal as th
+    p = mg.thermal_cube(cells, quadratic, increments=3, time_period=0.6, theta=0.75)
+    ref = oracle_lib.thermal_transient(p, solver=2)
+    iterations = {}
+    for knob in ("0", "1"):
+        monkeypatch.setenv("MAILLE_COARSE", knob)
+        s, out = th.solve_problem(p, f=ref["f"], precision=precision)
+        assert s == 0
+        assert np.abs(out["temps"] - ref["temps"]).max() < 1e-9 * np.abs(ref["temps"]).max()
+        iterations[knob] = int(out["iterations"].sum())
+    assert iterations["1"] < iterations["0"] if cells > 5 else iterations["1"] == iterations["0"]
