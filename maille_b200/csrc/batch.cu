@@ -104,6 +104,7 @@ struct MailleGpuBatch {
     bool any_imposed = false;
     Symbolic sym;
     std::vector<int32_t> row_inst;
+    Coarse coarse;  // the preconditioner's coarse correction, a grid per instance
     // device: inputs (packed numbering)
     double *coords = nullptr, *young = nullptr, *poisson = nullptr, *imposed = nullptr, *f0 = nullptr,
            *f = nullptr;
@@ -309,6 +310,7 @@ int32_t numeric(MailleGpuBatch* b, Error& err) {
     int32_t* dfail = dalloc<int32_t>(1);
     const int32_t status = factorize(b, err, dfail);
     dfree(dfail);
+    if (status == MAILLE_OK) b->coarse.update(b->K, b->st);
     CK(cudaEventRecord(b->ev[7], b->st));
     return status;
 }
@@ -467,6 +469,7 @@ BatchArgs<M, T> batch_args(MailleGpuBatch* b) {
     a.flags = b->flags;
     a.cancel = b->d_cancel;
     a.timing = b->timing;
+    if (b->cfg.threads % 128 == 0) a.c = b->coarse.batch<T>();  // its product works in groups of 4 warps
     return a;
 }
 
@@ -737,6 +740,20 @@ int32_t create_batch(const MailleBatchProblem* p, MailleGpuBatch** out) {
         if (env_int("MAILLE_PHASE_TIMING", 0)) {
             b->timing = dalloc<unsigned long long>(8);
             CK(cudaMemsetAsync(b->timing, 0, 8 * sizeof(unsigned long long), st));
+        }
+        if (env_int("MAILLE_COARSE", 1) != 0) {
+            std::vector<double> box(6 * (size_t)b->n_inst);
+            std::vector<int64_t> rows(b->n_inst, 0);
+            for (int32_t k = 0; k < b->n_inst; ++k)
+                coarse_box(p->coords, b->node_off[k], b->node_off[k + 1], box.data() + 6 * (size_t)k);
+            for (int32_t k : b->row_inst) rows[k]++;
+            struct DevTemp {
+                void* p = nullptr;
+                ~DevTemp() { dfree(p); }
+            } inst;
+            inst.p = dupload(b->row_inst.data(), b->row_inst.size(), st);
+            b->coarse.plan(3, b->mixed(), s.nb, s.blocks, b->coords, b->perm, b->fixmask, b->row_ptr, b->col,
+                           static_cast<const int32_t*>(inst.p), box, rows, st, b->R);
         }
         CK(cudaEventRecord(b->ev[5], st));
         if (numeric(b.get(), err) != MAILLE_OK) return fail(err);

@@ -19,6 +19,8 @@
 
 #include <cuda_runtime.h>
 
+#include "coarse.cuh"
+
 namespace maille {
 
 struct BSellDev {
@@ -63,6 +65,7 @@ struct BatchArgs {
     unsigned int* flags;        // [(nb + 1) G] row-ready epochs per load-case group
     const volatile int32_t* cancel;  // host-mapped cancel flag
     unsigned long long* timing;      // optional [8] ns per phase
+    CoarseBatchDev<T> c;             // the preconditioner's coarse correction (c.nodes = 0: none)
 };
 
 // Lane geometry of one kernel instance.

@@ -25,10 +25,12 @@
 
 #include <atomic>
 #include <cmath>
+#include <utility>
 
 #include <cooperative_groups.h>
 
 #include "batch.cuh"
+#include "coarse_dev.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -272,6 +274,166 @@ __device__ __forceinline__ double ordered_total(const double* part, int64_t base
     return s;
 }
 
+// ---- the coarse correction (coarse.cuh) for R load cases --------------------------------------
+//
+// A lane stands for one (load case, component) of a row, so a row's 3 R values are one contiguous
+// access and no sum crosses lanes; 32 / (3 R) rows go side by side when 3 R is less than 16.
+
+// partial sums of w_a(row) r(row) over a chunk's rows, for the 8 corners of its cell
+template <typename T, int R>
+__device__ __noinline__ void batch_restrict(const CoarseBatchDev<T> c, const uint32_t* done, const T* r, int32_t warp,
+                                            int32_t nwarps) {
+    constexpr int W = 3 * R, SUBS = 32 / W;
+    constexpr uint32_t FULL = (1u << R) - 1u;
+    const int lane = threadIdx.x & 31, v = lane % W, sub = lane / W;
+    for (int32_t k = warp; k < c.nchunks; k += nwarps) {
+        const int4 range = __ldg(c.chunk + k);
+        if (__ldcg(done + range.w) == FULL) continue;
+        T s[8] = {};
+        if (sub < SUBS) {
+#pragma unroll 4
+            for (int32_t p = range.x + sub; p < range.y; p += SUBS) {
+                T f[3], w[8];
+                uint32_t code;
+                coarse_row(c.ws, p, f, code);
+                const T x = __ldcg(r + (int64_t)(code & kCoarseRow) * W + v);
+                coarse_weights(f, w);
+#pragma unroll
+                for (int a = 0; a < 8; ++a) s[a] += w[a] * x;
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < 8; ++a) {
+            T t = s[a];
+#pragma unroll
+            for (int q = 1; q < SUBS; ++q) t += __shfl_sync(FULLW, s[a], (lane + q * W) & 31);
+            if (lane < W) c.part[((int64_t)k * 8 + a) * W + lane] = t;
+        }
+    }
+}
+
+// P^T r of every coarse node, load case and component: its cells' partial sums in order
+template <typename T, int R>
+__device__ __noinline__ void batch_gather(const CoarseBatchDev<T> c, const uint32_t* done, int64_t tid, int64_t nthreads) {
+    constexpr int W = 3 * R;
+    constexpr uint32_t FULL = (1u << R) - 1u;
+    for (int64_t e = tid; e < (int64_t)c.nodes * W; e += nthreads) {
+        const int32_t node = (int32_t)(e / W), v = (int32_t)(e - (int64_t)node * W), inst = __ldg(c.node_inst + node);
+        if (__ldcg(done + inst) == FULL) continue;
+        const CoarseGrid& g = c.grids[inst];
+        const int32_t l = node - g.node0, nx = g.k[0] + 1, ny = g.k[1] + 1;
+        const int32_t gx = l % nx, gy = l / nx % ny, gz = l / (nx * ny);
+        T s = T(0);
+#pragma unroll
+        for (int a = 0; a < 8; ++a) {
+            const int32_t x = gx - (a & 1), y = gy - ((a >> 1) & 1), z = gz - (a >> 2);
+            if (x < 0 || y < 0 || z < 0 || x >= g.k[0] || y >= g.k[1] || z >= g.k[2]) continue;
+            const int32_t cell = g.cell0 + x + g.k[0] * (y + g.k[1] * z);
+            const int32_t k1 = __ldg(c.cell_chunk + cell + 1);
+            for (int32_t k = __ldg(c.cell_chunk + cell); k < k1; ++k) s += __ldcg(c.part + ((int64_t)k * 8 + a) * W + v);
+        }
+        c.rc[e] = s;
+    }
+}
+
+// y = E^-1 P^T r: a group of 4 warps takes kCoarseTileRows rows of one instance's inverse, 4 a warp, for
+// all load cases; P^T r passes through shared memory in pieces of kPiece unknowns, so every value
+// of the inverse is read once and every value of P^T r once a tile. Each warp leaves its share of
+// (P^T r) . y per load case in its own slot.
+constexpr int kPiece = 128;
+template <typename T, int R>
+__device__ __noinline__ void batch_apply(const CoarseBatchDev<T> c, const uint32_t* done, T* smem) {
+    constexpr uint32_t FULL = (1u << R) - 1u;
+    const int lane = threadIdx.x & 31, wp = (threadIdx.x >> 5) & 3, t128 = threadIdx.x & 127;
+    const int group = threadIdx.x >> 7, groups = blockDim.x >> 7;
+    T* x = smem + group * kPiece * R;  // x[c * kPiece + f]
+    for (int32_t t = blockIdx.x * groups + group; t < c.ntiles; t += gridDim.x * groups) {
+        const int2 tile = __ldg(c.tile + t);
+        if (__ldcg(done + tile.x) == FULL) continue;  // the same for the 4 warps: done does not change here
+        const CoarseGrid& g = c.grids[tile.x];
+        const int32_t m = g.m, ld = g.ld, e0 = tile.y + 4 * wp;
+        const T* A = c.inv + g.dense0 + (int64_t)e0 * ld;  // rows beyond m (ld holds them) are zero
+        const T* rc = c.rc + (int64_t)g.node0 * 3 * R;
+        T acc[4][R] = {};
+        for (int32_t f0 = 0; f0 < m; f0 += kPiece) {
+            asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
+            for (int q = t128; q < kPiece * R; q += 128) {
+                const int32_t col = q / kPiece, f = f0 + q % kPiece;
+                x[q] = f < m ? __ldcg(rc + ((int64_t)(f / 3) * R + col) * 3 + f % 3) : T(0);
+            }
+            asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
+#pragma unroll
+            for (int j = 0; j < kPiece / 32; ++j) {
+                const int32_t f = f0 + 32 * j + lane;
+                if (f0 + 32 * j >= ld) break;
+                T av[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) av[q] = __ldg(A + (int64_t)q * ld + f);
+#pragma unroll
+                for (int k = 0; k < R; ++k) {
+                    const T xv = x[k * kPiece + 32 * j + lane];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) acc[q][k] += av[q] * xv;
+                }
+            }
+        }
+        // sums over the lanes; lane k keeps load case k
+        double dot = 0.0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            T mine = T(0);
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                T s = acc[q][k];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULLW, s, o);
+                if (lane == k) mine = s;
+            }
+            const int32_t e = e0 + q;
+            if (lane < R && e < m) {
+                const int64_t at = ((int64_t)(g.node0 + e / 3) * R + lane) * 3 + e % 3;
+                c.y[at] = mine;
+                dot += (double)__ldcg(c.rc + at) * (double)mine;
+            }
+        }
+        if (lane < R) c.dot[((int64_t)t * 4 + wp) * R + lane] = dot;
+    }
+}
+
+// p = z + P y + beta p over the chunks (every row once): the corners' y stay in registers for a
+// chunk's rows
+template <typename T, int R>
+__device__ __noinline__ void batch_update_p(const CoarseBatchDev<T> c, const uint32_t* done, const double* beta, const T* z,
+                                            T* p, int32_t warp, int32_t nwarps) {
+    constexpr int W = 3 * R, SUBS = 32 / W;
+    constexpr uint32_t FULL = (1u << R) - 1u;
+    const int lane = threadIdx.x & 31, v = lane % W, sub = lane / W;
+    for (int32_t k = warp; k < c.nchunks; k += nwarps) {
+        const int4 range = __ldg(c.chunk + k);
+        if (sub >= SUBS || __ldcg(done + range.w) == FULL) continue;
+        const CoarseGrid& g = c.grids[range.w];
+        const int32_t sy = g.k[0] + 1, sz = sy * (g.k[1] + 1);
+        const double bt = __ldcg(beta + (int64_t)range.w * R + v / 3);
+        T y[8];
+#pragma unroll
+        for (int a = 0; a < 8; ++a)
+            y[a] = __ldcg(c.y + (int64_t)(range.z + (a & 1) + ((a >> 1) & 1) * sy + (a >> 2) * sz) * W + v);
+#pragma unroll 4
+        for (int32_t q = range.x + sub; q < range.y; q += SUBS) {
+            T f[3], w[8], s = T(0);
+            uint32_t code;
+            coarse_row(c.ws, q, f, code);
+            const int64_t at = (int64_t)(code & kCoarseRow) * W + v;
+            const T zv = __ldcg(z + at), pv = __ldcg(p + at);
+            coarse_weights(f, w);
+#pragma unroll
+            for (int a = 0; a < 8; ++a) s += w[a] * y[a];
+            if ((code >> (29 + v % 3)) & 1u) s = T(0);
+            p[at] = (T)((double)zv + (double)s + bt * (double)pv);
+        }
+    }
+}
+
 // Marks instance i finished when every column has stopped (lane 0).
 __device__ __forceinline__ void retire_if_done(const BatchState& st, int i, uint32_t before, uint32_t after,
                                                uint32_t full) {
@@ -283,8 +445,10 @@ __global__ void __launch_bounds__(256) k_batch_pcg(BatchArgs<M, T> a, int passes
     using Gm = Geo<R, Q, SUB>;
     constexpr int AB = group_align<T, Q>();
     constexpr uint32_t FULL = (1u << R) - 1u;
+    __shared__ T coarse_mem[2 * kPiece * R];
     cg::grid_group grid = cg::this_grid();
     const BatchState& st = a.st;
+    const bool coarse = a.c.nodes > 0;
     const int lane = threadIdx.x & 31;
     const int rr = lane / Gm::LW, g = (lane / SUB) % Gm::G, q = lane % SUB;
     const int slot0 = 4 * (rr * SUB + q);
@@ -430,8 +594,15 @@ __global__ void __launch_bounds__(256) k_batch_pcg(BatchArgs<M, T> a, int passes
         mark(3);
         if (__ldcg(st.ctrl + 2) != 0) break;
 
-        // ---- backward sweep: z = L_II^-T (y - sum L^T z), and r.z per column ------------------
+        // ---- backward sweep: z = L_II^-T (y - sum L^T z), and r.z per column; the coarse
+        // correction's restriction before it, its gather after it (the barrier between the two is
+        // waited for behind the sweep) -----------------------------------------------------------
         epoch += 1;
+        cg::grid_group::arrival_token restricted{};
+        if (coarse) {
+            batch_restrict<T, R>(a.c, st.done, a.r, warp, nwarps);
+            restricted = grid.barrier_arrive();
+        }
         {
             bool ok = true;
             for (int32_t k0 = warp; k0 < a.U.nslices; k0 += nwarps) {
@@ -482,6 +653,13 @@ __global__ void __launch_bounds__(256) k_batch_pcg(BatchArgs<M, T> a, int passes
             if (!ok) atomicExch(st.ctrl + 2, 1);
             if (MIXED && blockIdx.x == 0 && threadIdx.x == 0) st.ctrl[1] = 0;
         }
+        if (coarse) {
+            grid.barrier_wait(std::move(restricted));
+            batch_gather<T, R>(a.c, st.done, (int64_t)blockIdx.x * blockDim.x + threadIdx.x,
+                               (int64_t)gridDim.x * blockDim.x);
+            grid.sync();
+            batch_apply<T, R>(a.c, st.done, coarse_mem);
+        }
         grid.sync();
         // ---- r.z per column: one warp per instance sums its slots in slot order ---------------
         if (__ldcg(st.ctrl + 2) == 0) {
@@ -489,7 +667,11 @@ __global__ void __launch_bounds__(256) k_batch_pcg(BatchArgs<M, T> a, int passes
                 const uint32_t dm = __ldcg(st.done + inst);
                 if (dm == FULL) continue;
                 const int b0 = __ldg(a.inst_uslot + inst), cnt = __ldg(a.inst_uslot + inst + 1) - b0;
-                const double rz = ordered_total<R>(a.part_u, b0, cnt);
+                double rz = ordered_total<R>(a.part_u, b0, cnt);
+                if (coarse) {
+                    const int t0 = __ldg(a.c.inst_tile + inst), t1 = __ldg(a.c.inst_tile + inst + 1);
+                    rz += ordered_total<R>(a.c.dot, 4 * (int64_t)t0, 4 * (t1 - t0));
+                }
                 if (lane < R) {
                     const int64_t s = (int64_t)inst * R + lane;
                     const bool live = !((dm >> lane) & 1u);
@@ -506,7 +688,8 @@ __global__ void __launch_bounds__(256) k_batch_pcg(BatchArgs<M, T> a, int passes
         first = false;
 
         // ---- p = z + beta p (iterative.rs:240-242) --------------------------------------------
-        for (int32_t t = warp; t < a.ntasks; t += nwarps) {
+        if (coarse) batch_update_p<T, R>(a.c, st.done, st.beta, a.z, a.p, warp, nwarps);
+        for (int32_t t = coarse ? a.ntasks : warp; t < a.ntasks; t += nwarps) {
             const int32_t inst = a.task_inst[t];
             const uint32_t dm = __ldcg(st.done + inst);
             if (dm == FULL) continue;

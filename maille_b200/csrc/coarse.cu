@@ -33,7 +33,8 @@ namespace {
 
 constexpr int kT = 256;
 constexpr int kTile = 64;        // unknowns a sweep step; tile side
-constexpr int kRowChunk = 256;   // rows a restriction chunk
+constexpr int kRowChunk = 256;   // rows a restriction chunk, one row a lane at a time
+constexpr int kBatchChunk = 64;  // rows a chunk of a batch, whose warp takes them one after the other
 constexpr int kPairChunk = 256;  // blocks a Galerkin chunk
 constexpr int kPairWarps = 4;    // warps a block of k_pairs
 constexpr double kDrop = 1e-12;  // pivot test, relative to the unknown's diagonal of E
@@ -95,7 +96,7 @@ __global__ void k_row_weights(int32_t nb, const double4* __restrict__ pos, const
         const double4 p = pos[i];
         w[i] = Vec4<T>::make(p, (uint32_t)__double_as_longlong(p.w));
         const int32_t r = order[i];
-        ws[i] = Vec4<T>::make(pos[r], (uint32_t)r);
+        ws[i] = Vec4<T>::make(pos[r], (uint32_t)r | ((uint32_t)__double_as_longlong(pos[r].w) >> 28 << 29));
     }
 }
 
@@ -487,8 +488,9 @@ void coarse_box(const double* xyz, int64_t n0, int64_t n1, double box[6]) {
 // 23x30x17 26.5 / 25.4 / 24.3.
 void coarse_cells(int dof, const double box[6], int64_t rows, int32_t k[3]) {
     const double more = dof == 1 ? 1.2 : 1.0;
+    if (rows < kMinRows) rows = 1;
     const double side = more * std::min(10.0, std::cbrt(3.0 * std::pow((double)std::max<int64_t>(rows, 1), 0.44)));
-    const double target = std::max(8.0, std::pow(side + 1.0, 3.0) * 1.0001);
+    const double target = rows == 1 ? 8.0 : std::max(8.0, std::pow(side + 1.0, 3.0) * 1.0001);
     double ext[3], longest = 0.0;
     for (int a = 0; a < 3; ++a) {
         ext[a] = std::max(0.0, box[3 + a] - box[a]);
@@ -520,7 +522,7 @@ Coarse::~Coarse() {
 }
 
 void Coarse::gather(std::vector<void*>& out) {
-    for (void** p : {(void**)&d_grids_, (void**)&d_inst_, (void**)&pos_, &w_, &ws_, &inv_, &part_, &rc_, &y_, (void**)&chunk_,
+    for (void** p : {(void**)&d_grids_, (void**)&node_inst_, (void**)&inst_tile_, (void**)&tile_, (void**)&dot_, (void**)&pos_, &w_, &ws_, &inv_, &part_, &rc_, &y_, (void**)&chunk_,
                      (void**)&cell_chunk_, (void**)&bpos_, (void**)&brow_, (void**)&bcol_, (void**)&schunk_ptr_,
                      (void**)&table_, (void**)&schunk_, (void**)&spart_, (void**)&A_, (void**)&diag_, (void**)&panel_w_,
                      (void**)&panel_v_, (void**)&piv_}) {
@@ -532,9 +534,11 @@ void Coarse::gather(std::vector<void*>& out) {
 
 void Coarse::plan(int dof, bool fp32, int32_t nb, int64_t blocks, const double* xyz, const int32_t* perm,
                   const uint8_t* fixmask, const int64_t* row_ptr, const int32_t* col, const int32_t* row_inst,
-                  const std::vector<double>& box, const std::vector<int64_t>& rows_of, cudaStream_t st) {
+                  const std::vector<double>& box, const std::vector<int64_t>& rows_of, cudaStream_t st, int rhs) {
     const int n_inst = (int)rows_of.size();
-    if (n_inst == 0 || *std::max_element(rows_of.begin(), rows_of.end()) < kMinRows || blocks >= INT_MAX) return;
+    if (n_inst == 0 || n_inst > 65535 || *std::max_element(rows_of.begin(), rows_of.end()) < kMinRows ||
+        blocks >= INT_MAX || nb >= (1 << 28))
+        return;
     dof_ = dof;
     fp32_ = fp32;
     grids_.assign(n_inst, CoarseGrid{});
@@ -568,7 +572,6 @@ void Coarse::plan(int dof, bool fp32, int32_t nb, int64_t blocks, const double* 
     }
     nodes_ = nodes;
     dense_ = dense;
-    d_inst_ = nullptr;
     pos_ = dalloc<double4>(nb);
     Temp cell(nb * sizeof(int32_t)), cell_sorted(nb * sizeof(int32_t)), rows(nb * sizeof(int32_t)),
         order(nb * sizeof(int32_t)), cell_ptr((ncells_ + 1) * sizeof(int32_t));
@@ -642,12 +645,25 @@ void Coarse::plan(int dof, bool fp32, int32_t nb, int64_t blocks, const double* 
     }
     nseg_ = (int32_t)seg_key.size();
     // chunks of rows and of blocks
-    std::vector<int2> chunk, schunk;
-    h_cell_chunk_.assign(ncells_ + 1, 0);
-    for (int32_t c = 0; c < ncells_; ++c) {
-        for (int32_t p = h_ptr[c]; p < h_ptr[c + 1]; p += kRowChunk)
-            chunk.push_back(make_int2(p, std::min(p + kRowChunk, h_ptr[c + 1])));
-        h_cell_chunk_[c + 1] = (int32_t)chunk.size();
+    std::vector<int4> chunk;
+    std::vector<int2> schunk, tile;
+    std::vector<int32_t> cell_chunk(ncells_ + 1, 0), node_inst, inst_tile(1, 0);
+    const int32_t step = rhs > 0 ? kBatchChunk : kRowChunk;
+    for (int q = 0; q < n_inst; ++q) {
+        const CoarseGrid& g = grids_[q];
+        const int32_t nc = g.k[0] * g.k[1] * g.k[2];
+        for (int32_t l = 0; l < nc; ++l) {
+            const int32_t c = g.cell0 + l, x = l % g.k[0], y = l / g.k[0] % g.k[1], z = l / (g.k[0] * g.k[1]);
+            const int32_t base = g.node0 + x + (g.k[0] + 1) * (y + (g.k[1] + 1) * z);
+            for (int32_t p = h_ptr[c]; p < h_ptr[c + 1]; p += step)
+                chunk.push_back(make_int4(p, std::min(p + step, h_ptr[c + 1]), base, q));
+            cell_chunk[c + 1] = (int32_t)chunk.size();
+        }
+        if (rhs > 0) {
+            node_inst.insert(node_inst.end(), g.m / dof, q);
+            for (int32_t e = 0; e < g.m; e += kCoarseTileRows) tile.push_back(make_int2(q, e));
+            inst_tile.push_back((int32_t)tile.size());
+        }
     }
     std::vector<int32_t> schunk_ptr(nseg_ + 1, 0);
     std::vector<int64_t> at(nseg_);
@@ -671,7 +687,7 @@ void Coarse::plan(int dof, bool fp32, int32_t nb, int64_t blocks, const double* 
     nschunks_ = (int32_t)schunk.size();
     CK(cudaMemcpyAsync(d_grids_, grids_.data(), grids_.size() * sizeof(CoarseGrid), cudaMemcpyHostToDevice, st));
     chunk_ = dupload(chunk.data(), chunk.size(), st);
-    cell_chunk_ = dupload(h_cell_chunk_.data(), h_cell_chunk_.size(), st);
+    cell_chunk_ = dupload(cell_chunk.data(), cell_chunk.size(), st);
     schunk_ = dupload(schunk.data(), schunk.size(), st);
     schunk_ptr_ = dupload(schunk_ptr.data(), schunk_ptr.size(), st);
     brow_ = dalloc<int32_t>(first);
@@ -692,11 +708,22 @@ void Coarse::plan(int dof, bool fp32, int32_t nb, int64_t blocks, const double* 
     panel_v_ = dalloc<double>(ldsum * kTile);
     piv_ = dalloc<double>((size_t)n_inst * kTile * kTile);
     inv_ = device_alloc(dense_ * tb);
-    part_ = device_alloc((size_t)std::max(1, nchunks_) * 8 * dof * tb);
-    rc_ = device_alloc(ldsum * tb);
-    y_ = device_alloc(nodes * (dof == 3 ? 4 : 1) * tb);
-    CK(cudaMemsetAsync(rc_, 0, ldsum * tb, st));
-    CK(cudaMemsetAsync(y_, 0, nodes * (dof == 3 ? 4 : 1) * tb, st));
+    // one system: rc by unknown, padded with zeros to ld; y 4 a node (dof 3). Batch: [node][R][3] both
+    const size_t cols = rhs > 0 ? rhs : 1;
+    const size_t nrc = rhs > 0 ? (size_t)nodes * dof * cols : (size_t)ldsum;
+    const size_t ny = rhs > 0 ? (size_t)nodes * dof * cols : (size_t)nodes * (dof == 3 ? 4 : 1);
+    part_ = device_alloc((size_t)std::max(1, nchunks_) * 8 * dof * cols * tb);
+    rc_ = device_alloc(nrc * tb);
+    y_ = device_alloc(ny * tb);
+    CK(cudaMemsetAsync(rc_, 0, nrc * tb, st));
+    CK(cudaMemsetAsync(y_, 0, ny * tb, st));
+    if (rhs > 0) {
+        ntiles_ = (int32_t)tile.size();
+        tile_ = dupload(tile.data(), tile.size(), st);
+        inst_tile_ = dupload(inst_tile.data(), inst_tile.size(), st);
+        node_inst_ = dupload(node_inst.data(), node_inst.size(), st);
+        dot_ = dalloc<double>((size_t)ntiles_ * (kCoarseTileRows / 4) * cols);
+    }
     CK(cudaStreamSynchronize(st));  // the host lists and the temporaries go
     dfree(d_at);
     nb_ = nb;
@@ -757,5 +784,29 @@ CoarseDev<T> Coarse::dev(int inst) const {
 }
 template CoarseDev<float> Coarse::dev<float>(int) const;
 template CoarseDev<double> Coarse::dev<double>(int) const;
+
+template <typename T>
+CoarseBatchDev<T> Coarse::batch() const {
+    CoarseBatchDev<T> c;
+    if (!active()) return c;
+    c.nodes = (int32_t)nodes_;
+    c.nchunks = nchunks_;
+    c.ntiles = ntiles_;
+    c.grids = d_grids_;
+    c.ws = static_cast<const T*>(ws_);
+    c.chunk = chunk_;
+    c.cell_chunk = cell_chunk_;
+    c.node_inst = node_inst_;
+    c.tile = tile_;
+    c.inst_tile = inst_tile_;
+    c.inv = static_cast<const T*>(inv_);
+    c.part = static_cast<T*>(part_);
+    c.rc = static_cast<T*>(rc_);
+    c.y = static_cast<T*>(y_);
+    c.dot = dot_;
+    return c;
+}
+template CoarseBatchDev<float> Coarse::batch<float>() const;
+template CoarseBatchDev<double> Coarse::batch<double>() const;
 
 }  // namespace maille

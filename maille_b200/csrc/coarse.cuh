@@ -49,13 +49,32 @@ struct CoarseDev {
     int32_t nchunks = 0;
     const T* w = nullptr;               // [4 nb] per row: fx, fy, fz in its cell, code (CoarseCode)
     const T* ws = nullptr;              // [4 nb] the same in cell order, code = the row
-    const int2* chunk = nullptr;        // [nchunks] ranges of the cell order, each inside one cell
+    const int4* chunk = nullptr;        // [nchunks] (first, end) in the cell order, inside one cell
     const int32_t* cell_chunk = nullptr;  // [cells + 1] first chunk of each cell
     const T* inv = nullptr;             // [m * ld] E^-1
     T* part = nullptr;                  // [nchunks * 8 * dof] restricted residual of each chunk
     T* rc = nullptr;                    // [ld] P^T r
     T* y = nullptr;                     // [(dof == 3 ? 4 : 1) * nn] E^-1 P^T r
 };
+
+// The same for a batch of instances with R load cases each: vectors are [node][R][3], r and p
+// [row][R][3], chunks and cells run over all instances.
+template <typename T>
+struct CoarseBatchDev {
+    int32_t nodes = 0;                    // coarse nodes of all instances; 0: no correction
+    int32_t nchunks = 0, ntiles = 0;
+    const CoarseGrid* grids = nullptr;
+    const T* ws = nullptr;                // [4 nb] in cell order: fx, fy, fz, row and fixed mask (kCoarseRow)
+    const int4* chunk = nullptr;          // [nchunks] (first, end, base coarse node, instance)
+    const int32_t* cell_chunk = nullptr;  // [cells + 1]
+    const int32_t* node_inst = nullptr;   // [nodes] instance of each coarse node
+    const int2* tile = nullptr;           // [ntiles] (instance, first unknown) of kCoarseTileRows rows
+    const int32_t* inst_tile = nullptr;   // [n_inst + 1] first tile of each instance
+    const T* inv = nullptr;
+    T *part = nullptr, *rc = nullptr, *y = nullptr;  // [nchunks 8][R][3], [nodes][R][3], [nodes][R][3]
+    double* dot = nullptr;                // [ntiles 4][R] shares of (P^T r) . y
+};
+constexpr int kCoarseTileRows = 16;
 
 // The correction of one system (one or several instances): plan and numeric state.
 class Coarse {
@@ -64,17 +83,18 @@ class Coarse {
     // Rows, pattern and grid of the system. xyz: [3 n_nodes] device coordinates; perm: [nb] row ->
     // node; fixmask: [nb] fixed components or null; row_ptr, col: the full pattern, dof x dof blocks.
     // row_inst: [nb] instance of each row or null (one instance). box: [6 instances] min and max
-    // corners; rows_of: rows per instance. Does nothing (active() stays false) when no
+    // corners; rows_of: rows per instance; rhs: load cases of a batch (its layouts), 0: one system. Does nothing (active() stays false) when no
     // instance is large enough. Synchronises the stream.
     void plan(int dof, bool fp32, int32_t nb, int64_t blocks, const double* xyz, const int32_t* perm,
               const uint8_t* fixmask, const int64_t* row_ptr, const int32_t* col, const int32_t* row_inst,
-              const std::vector<double>& box, const std::vector<int64_t>& rows_of, cudaStream_t st);
+              const std::vector<double>& box, const std::vector<int64_t>& rows_of, cudaStream_t st, int rhs = 0);
     // E and its inverse from the assembled values (dof x dof per block, CSR order); enqueued on st.
     void update(const double* vals, cudaStream_t st);
     bool active() const { return nb_ > 0; }
     CoarseDev<float> dev32(int inst = 0) const { return dev<float>(inst); }
     CoarseDev<double> dev64(int inst = 0) const { return dev<double>(inst); }
-    const std::vector<CoarseGrid>& grids() const { return grids_; }
+    template <typename T>
+    CoarseBatchDev<T> batch() const;
     // the device buffers, handed over to be freed together
     void gather(std::vector<void*>& out);
 
@@ -86,12 +106,14 @@ class Coarse {
     int32_t nb_ = 0, nchunks_ = 0, nseg_ = 0, nschunks_ = 0, steps_ = 0, ncells_ = 0;
     int64_t dense_ = 0, nodes_ = 0;
     std::vector<CoarseGrid> grids_;
-    std::vector<int32_t> h_cell_chunk_;
     CoarseGrid* d_grids_ = nullptr;
-    int32_t *d_inst_ = nullptr;
     double4* pos_ = nullptr;          // [nb] fractions and code, FP64 (Galerkin)
     void *w_ = nullptr, *ws_ = nullptr, *inv_ = nullptr, *part_ = nullptr, *rc_ = nullptr, *y_ = nullptr;
-    int2* chunk_ = nullptr;
+    int4* chunk_ = nullptr;
+    int32_t *node_inst_ = nullptr, *inst_tile_ = nullptr;
+    int2* tile_ = nullptr;
+    double* dot_ = nullptr;
+    int32_t ntiles_ = 0;
     int32_t* cell_chunk_ = nullptr;
     // Galerkin: blocks sorted by cell pair
     int32_t *bpos_ = nullptr, *brow_ = nullptr, *bcol_ = nullptr, *schunk_ptr_ = nullptr, *table_ = nullptr;
@@ -102,6 +124,8 @@ class Coarse {
 // Coarse node and fixed components of a row, packed: base node of its cell in the low 28 bits, fixed
 // mask above.
 constexpr uint32_t kCoarseBase = (1u << 28) - 1u;
+// Cell order: the row in the low 29 bits, fixed mask above.
+constexpr uint32_t kCoarseRow = (1u << 29) - 1u;
 
 // Host bounding box of the nodes [n0, n1) of xyz into box[6] (min x, y, z, max x, y, z).
 void coarse_box(const double* xyz, int64_t n0, int64_t n1, double box[6]);

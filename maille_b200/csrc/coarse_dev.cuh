@@ -76,7 +76,7 @@ template <typename T, int DOF>
 __device__ __noinline__ void coarse_restrict(const CoarseDev<T> c, const T* r, int32_t warp, int32_t nwarps) {
     const int lane = threadIdx.x & 31;
     for (int32_t k = warp; k < c.nchunks; k += nwarps) {
-        const int2 range = __ldg(c.chunk + k);
+        const int4 range = __ldg(c.chunk + k);
         T s[8 * DOF];
 #pragma unroll
         for (int q = 0; q < 8 * DOF; ++q) s[q] = T(0);
@@ -84,7 +84,7 @@ __device__ __noinline__ void coarse_restrict(const CoarseDev<T> c, const T* r, i
             T f[3], w[8], v[DOF];
             uint32_t row;
             coarse_row(c.ws, p, f, row);
-            coarse_load_r<DOF>(r, (int64_t)row, v);
+            coarse_load_r<DOF>(r, (int64_t)(row & kCoarseRow), v);
             coarse_weights(f, w);
 #pragma unroll
             for (int a = 0; a < 8; ++a)

@@ -95,3 +95,26 @@ def test_the_thermal_step_takes_the_correction(gpu, oracle_lib, monkeypatch, qua
         assert np.abs(out["temps"] - ref["temps"]).max() < 1e-9 * np.abs(ref["temps"]).max()
         iterations[knob] = int(out["iterations"].sum())
     assert iterations["1"] < iterations["0"] if cells > 5 else iterations["1"] == iterations["0"]
+
+
+@pytest.mark.parametrize("rhs,precision,tol,err", [(1, MAILLE_FP64, 1e-13, 1e-10), (3, MAILLE_FP64, 1e-13, 1e-10),
+                                                   (8, MAILLE_FP64, 1e-13, 1e-10), (8, MAILLE_MIXED, 1e-10, 1e-8),
+                                                   (2, MAILLE_MIXED, 1e-10, 1e-8)])
+@pytest.mark.parametrize("threads", ["128", "256"])
+def test_a_batch_takes_the_correction(gpu, monkeypatch, rhs, precision, tol, err, threads):
+    # instances of 12 to 1331 rows (one cell to 5 a side), every load-case layout, against the same batch
+    # with IC(0) alone
+    probs, loads = mg.batched_tet4(count=5, lo=2, hi=11, load_cases=rhs)
+    monkeypatch.setenv("MAILLE_BATCH_Q", {1: "2", 2: "1", 3: "2", 8: "4"}[rhs])
+    monkeypatch.setenv("MAILLE_BATCH_THREADS", threads)
+    out = {}
+    for knob in ("0", "1"):
+        monkeypatch.setenv("MAILLE_COARSE", knob)
+        with mb.BatchSolver(probs, loads, tol=tol, precision=precision) as b:
+            out[knob] = b.solve()
+            again = b.solve()
+        assert out[knob].info["status_code"] == 0
+        assert all(np.array_equal(x, y) for x, y in zip(out[knob].displacements, again.displacements))
+    for a, b in zip(out["0"].displacements, out["1"].displacements):
+        assert rel(b, a) < 2 * err
+    assert out["1"].iterations.max() < out["0"].iterations.max()
