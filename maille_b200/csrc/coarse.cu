@@ -6,8 +6,8 @@
 // Numeric set-up, once per factorisation:
 //  * k_pairs: one warp per chunk of blocks of one cell pair sums w_a(i) w_b(j) K_ij for the 64
 //    corner pairs (a, b), two pairs a lane, into the chunk's own slots;
-//  * k_dense: every entry of E sums the slots of the cell pairs that touch it, in order;
-//  * k_panel / k_trail: E^-1 by block symmetric sweeps (Beaton's sweep operator, 64 unknowns a
+//  * k_pair_sums, k_dense: every entry of E sums the slots of the cell pairs that touch it, in order;
+//  * k_panel, k_trail: E^-1 by block symmetric sweeps (Beaton's sweep operator, 64 unknowns a
 //    step, lower tiles only): m^3 flops, no pivoting (E is positive definite). An unknown whose
 //    pivot falls to 1e-12 of its own diagonal (a coarse node without support, or dependent on
 //    others) leaves the space: its row and column of the inverse are zero;
@@ -206,76 +206,163 @@ __global__ void __launch_bounds__(kPairWarps * 32) k_pairs(int32_t nchunks, cons
     }
 }
 
-// A (lower tiles) = E with ones on the padded diagonal, diag = its diagonal: one thread per pair of
-// coarse nodes h <= g of an instance. `span`: cells that a block of K reaches across at most.
+// The chunks of every cell pair, summed in order into its first one.
+template <int DOF>
+__global__ void k_pair_sums(int32_t nseg, const int32_t* __restrict__ schunk_ptr, double* __restrict__ part) {
+    constexpr int64_t N = 64 * DOF * DOF;
+    GRID_STRIDE(t, nseg * N) {
+        const int64_t seg = t / N, v = t - seg * N;
+        const int32_t k0 = schunk_ptr[seg], k1 = schunk_ptr[seg + 1];
+        if (k1 - k0 < 2) continue;
+        double s = part[k0 * N + v];
+        for (int32_t k = k0 + 1; k < k1; ++k) s += part[k * N + v];
+        part[k0 * N + v] = s;
+    }
+}
+
+// A (lower tiles, zero before) = E with ones on the padded diagonal, diag = its diagonal: one thread per
+// coarse node u, node v <= u within reach (`span`: cells that a block of K reaches across at most)
+// and entry of their block.
 template <int DOF>
 __global__ void k_dense(const CoarseGrid* __restrict__ grids, const int32_t* __restrict__ table,
                         const int32_t* __restrict__ schunk_ptr, const double* __restrict__ part, double* __restrict__ A,
                         double* __restrict__ diag, int64_t diag_stride) {
     constexpr int D2 = DOF * DOF;
     const CoarseGrid g = grids[blockIdx.y];
-    const int32_t nx = g.k[0] + 1, ny = g.k[1] + 1, nn = nx * ny * (g.k[2] + 1);
-    const int32_t nc = g.k[0] * g.k[1] * g.k[2], span = g.span + 1;
+    const int32_t nx = g.k[0] + 1, ny = g.k[1] + 1, nz = g.k[2] + 1, nn = nx * ny * nz;
+    const int32_t nc = g.k[0] * g.k[1] * g.k[2], reach = g.span + 1;
+    const int32_t wx = min(reach, g.k[0]), wy = min(reach, g.k[1]), wz = min(reach, g.k[2]);
+    const int32_t sx = 2 * wx + 1, sy = 2 * wy + 1, window = sx * sy * (2 * wz + 1);
     double* Ai = A + g.dense0;
     double* di = diag + blockIdx.y * diag_stride;
     const int32_t* tab = table + g.tab0;
-    GRID_STRIDE(t, (int64_t)nn * nn) {
-        const int32_t u = (int32_t)(t / nn), v = (int32_t)(t - (int64_t)u * nn);
-        if (v > u) continue;
+    GRID_STRIDE(t, (int64_t)nn * window * D2) {
+        const int32_t u = (int32_t)(t / (window * D2)), rest = (int32_t)(t - (int64_t)u * window * D2);
+        const int32_t q = rest / window, o = rest - q * window;
         const int32_t ux = u % nx, uy = (u / nx) % ny, uz = u / (nx * ny);
-        const int32_t vx = v % nx, vy = (v / nx) % ny, vz = v / (nx * ny);
-        double s[D2];
+        const int32_t vx = ux + o % sx - wx, vy = uy + o / sx % sy - wy, vz = uz + o / (sx * sy) - wz;
+        if (vx < 0 || vy < 0 || vz < 0 || vx >= nx || vy >= ny || vz >= nz) continue;
+        const int32_t v = vx + nx * (vy + ny * vz);
+        if (v > u) continue;
+        double s = 0.0;
+        for (int a = 0; a < 8; ++a) {
+            const int32_t cx = ux - (a & 1), cy = uy - ((a >> 1) & 1), cz = uz - (a >> 2);
+            if (cx < 0 || cy < 0 || cz < 0 || cx >= g.k[0] || cy >= g.k[1] || cz >= g.k[2]) continue;
+            const int32_t cu = cx + g.k[0] * (cy + g.k[1] * cz);
 #pragma unroll
-        for (int q = 0; q < D2; ++q) s[q] = 0.0;
-        if (abs(ux - vx) <= span && abs(uy - vy) <= span && abs(uz - vz) <= span)
-            for (int a = 0; a < 8; ++a) {
-                const int32_t cx = ux - (a & 1), cy = uy - ((a >> 1) & 1), cz = uz - (a >> 2);
-                if (cx < 0 || cy < 0 || cz < 0 || cx >= g.k[0] || cy >= g.k[1] || cz >= g.k[2]) continue;
-                const int32_t cu = cx + g.k[0] * (cy + g.k[1] * cz);
-                for (int b = 0; b < 8; ++b) {
-                    const int32_t ex = vx - (b & 1), ey = vy - ((b >> 1) & 1), ez = vz - (b >> 2);
-                    if (ex < 0 || ey < 0 || ez < 0 || ex >= g.k[0] || ey >= g.k[1] || ez >= g.k[2]) continue;
-                    const int32_t cv = ex + g.k[0] * (ey + g.k[1] * ez);
-                    const bool direct = cu >= cv;
-                    const int32_t seg = direct ? tab[(int64_t)cu * nc + cv] : tab[(int64_t)cv * nc + cu];
-                    if (seg < 0) continue;
-                    const int slot = direct ? a + 8 * b : b + 8 * a;
-                    for (int32_t k = schunk_ptr[seg]; k < schunk_ptr[seg + 1]; ++k)
-#pragma unroll
-                        for (int q = 0; q < D2; ++q) {
-                            const int from = direct ? q : (q % DOF) * DOF + q / DOF;
-                            s[q] += part[((int64_t)k * D2 + from) * 64 + slot];
-                        }
-                }
+            for (int b = 0; b < 8; ++b) {
+                const int32_t ex = vx - (b & 1), ey = vy - ((b >> 1) & 1), ez = vz - (b >> 2);
+                if (ex < 0 || ey < 0 || ez < 0 || ex >= g.k[0] || ey >= g.k[1] || ez >= g.k[2]) continue;
+                const int32_t cv = ex + g.k[0] * (ey + g.k[1] * ez);
+                const bool direct = cu >= cv;
+                const int32_t seg = direct ? tab[(int64_t)cu * nc + cv] : tab[(int64_t)cv * nc + cu];
+                if (seg < 0) continue;
+                const int slot = direct ? a + 8 * b : b + 8 * a;
+                const int from = direct ? q : (q % DOF) * DOF + q / DOF;
+                s += part[((int64_t)schunk_ptr[seg] * D2 + from) * 64 + slot];
             }
-#pragma unroll
-        for (int q = 0; q < D2; ++q) {
-            const int64_t r = (int64_t)DOF * u + q / DOF, c = (int64_t)DOF * v + q % DOF;
-            Ai[r * g.ld + c] = s[q];
-            if (r == c) di[r] = s[q];
         }
+        const int64_t r = (int64_t)DOF * u + q / DOF, c = (int64_t)DOF * v + q % DOF;
+        Ai[r * g.ld + c] = s;
+        if (r == c) di[r] = s;
     }
     // the padding of the last tiles: an identity
-    const int64_t pad = g.ld - g.m;
-    GRID_STRIDE(t, pad * g.ld) {
-        const int64_t r = g.m + t / g.ld, c = t % g.ld;
-        Ai[r * g.ld + c] = r == c ? 1.0 : 0.0;
-        if (r == c) di[r] = 1.0;
+    GRID_STRIDE(t, g.ld - g.m) {
+        Ai[(g.m + t) * (g.ld + 1)] = 1.0;
+        di[g.m + t] = 1.0;
     }
 }
 
-// Step s of the sweeps, panel: every block sweeps the pivot tile A_ss in registers (256 threads, 4 x 4
-// entries each; a step broadcasts the pivot row through shared memory), giving -A_ss^-1, then
-// block i forms W_i = A_is and V_i = W_i A_ss^-1 (transposed in the panels: unknown-major). Sweeping the
-// pivot in every block costs less than a launch between the two. Latency-bound: 64 dependent
-// pivots.
+// Sweeps the 64 x 64 tile held by 256 threads, 4 x 4 entries a[][] each (thread (ty, tx): rows 4 ty ..,
+// columns 4 tx ..): a = -tile^-1. Four pivots at a time: the thread on the diagonal sweeps its own 4 x 4
+// entries, its row of threads broadcasts its rows through shared memory, the block forms their
+// product with the 4 x 4 inverse, and every thread takes the rank-4 update. 16 such steps instead of
+// 64 pivots: one pivot at a time took 105 us a tile, with a division, a load of its limit and a
+// barrier on every pivot's path. An unknown whose pivot falls to kDrop of its diagonal of E is
+// dropped: a zero row and column.
+struct SweepMem {
+    double rows[4][kTile], u[kTile][4], P[16], limit[kTile];
+};
+__device__ __forceinline__ void sweep_tile(double a[4][4], SweepMem& m) {
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    for (int b = 0; b < kTile / 4; ++b) {
+        if (ty == b) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int p = 0; p < 4; ++p) m.rows[q][4 * tx + p] = a[q][p];
+            if (tx == b) {
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    const double d = a[t][t], inv = d > m.limit[4 * b + t] ? 1.0 / d : 0.0;
+                    double c[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) c[q] = a[q][t] * inv;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+#pragma unroll
+                        for (int p = 0; p < 4; ++p)
+                            if (q != t && p != t) a[q][p] -= c[q] * a[t][p];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if (q != t) a[q][t] = a[t][q] = c[q];
+                    a[t][t] = -inv;
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+#pragma unroll
+                    for (int p = 0; p < 4; ++p) m.P[4 * q + p] = a[q][p];
+            }
+        }
+        __syncthreads();
+        {  // u = (the pivot columns of every row) tile_bb^-1, one entry a thread
+            const int r = tid >> 2, p = tid & 3;
+            double s = 0.0;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) s -= m.rows[t][r] * m.P[4 * t + p];
+            m.u[r][p] = s;
+        }
+        __syncthreads();
+        if (tx == b) {
+            if (ty != b)
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+#pragma unroll
+                    for (int p = 0; p < 4; ++p) a[q][p] = m.u[4 * ty + q][p];
+        } else if (ty == b) {  // the pivot rows: the transposed columns
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int p = 0; p < 4; ++p) a[q][p] = m.u[4 * tx + p][q];
+        } else {
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                double w[4], u[4];
+#pragma unroll
+                for (int p = 0; p < 4; ++p) {
+                    w[p] = m.rows[t][4 * tx + p];
+                    u[p] = m.u[4 * ty + p][t];
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+#pragma unroll
+                    for (int p = 0; p < 4; ++p) a[q][p] -= u[q] * w[p];
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// Step s of the sweeps, panel: every block sweeps the pivot tile A_ss into -A_ss^-1 (each for itself: a
+// launch of its own would cost as much, and a block of k_trail that did it slowed that kernel by its
+// registers); block i then forms W_i = A_is and V_i = W_i A_ss^-1 (both transposed in the panels:
+// unknown-major), block s leaves the pivot in piv.
 constexpr int kPanelStride = kTile + 2;
 __global__ void __launch_bounds__(kT) k_panel(int s, const CoarseGrid* __restrict__ grids, const double* __restrict__ A,
                                               const double* __restrict__ diag, int64_t diag_stride,
                                               double* __restrict__ W, double* __restrict__ V, double* __restrict__ piv) {
     extern __shared__ __align__(16) double sm[];
-    __shared__ double rowbuf[2][kTile];
-    __shared__ double pivot[2];
+    __shared__ SweepMem mem;
     double *P = sm, *Wt = sm + kTile * kPanelStride;  // P[t][c]; Wt[t][r] = W_i[r][t]
     const CoarseGrid& g = grids[blockIdx.y];
     const int tiles = g.ld / kTile, i = blockIdx.x;
@@ -283,13 +370,14 @@ __global__ void __launch_bounds__(kT) k_panel(int s, const CoarseGrid* __restric
     const double* Ai = A + g.dense0;
     const int64_t ld = g.ld, o = (int64_t)s * kTile, oi = (int64_t)i * kTile;
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    if (tid < kTile) mem.limit[tid] = kDrop * diag[blockIdx.y * diag_stride + o + tid];
     double a[4][4];
 #pragma unroll
     for (int q = 0; q < 4; ++q)
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
             const int r = 4 * ty + q, c = 4 * tx + p;
-            a[q][p] = r >= c ? Ai[(o + r) * ld + o + c] : Ai[(o + c) * ld + o + r];
+            a[q][p] = Ai[(o + max(r, c)) * ld + o + min(r, c)];
         }
     if (i != s)
         for (int e = tid; e < kTile * kTile; e += kT) {
@@ -297,41 +385,8 @@ __global__ void __launch_bounds__(kT) k_panel(int s, const CoarseGrid* __restric
             if (i > s) Wt[l * kPanelStride + h] = Ai[(oi + h) * ld + o + l];
             else Wt[h * kPanelStride + l] = Ai[(o + h) * ld + oi + l];
         }
-    const double* d0 = diag + blockIdx.y * diag_stride + o;
-    for (int t = 0; t < kTile; ++t) {
-        const int buf = t & 1;
-        if (ty == (t >> 2)) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (q == (t & 3)) {
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) {
-                        rowbuf[buf][4 * tx + p] = a[q][p];
-                        if (4 * tx + p == t) {
-                            const double d = a[q][p];
-                            pivot[buf] = d > kDrop * d0[t] ? 1.0 / d : 0.0;  // 0: the unknown is dropped
-                        }
-                    }
-                }
-        }
-        __syncthreads();
-        const double inv = pivot[buf];
-        double rr[4], cc[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            rr[q] = rowbuf[buf][4 * ty + q] * inv;  // column t by symmetry
-            cc[q] = rowbuf[buf][4 * tx + q];
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-#pragma unroll
-            for (int p = 0; p < 4; ++p) {
-                const int r = 4 * ty + q, c = 4 * tx + p;
-                if (r == t) a[q][p] = c == t ? -inv : cc[p] * inv;
-                else if (c == t) a[q][p] = rr[q];
-                else a[q][p] -= rr[q] * cc[p];
-            }
-    }
+    __syncthreads();
+    sweep_tile(a, mem);
     if (i == s) {
         double* out = piv + (int64_t)blockIdx.y * kTile * kTile;
 #pragma unroll
@@ -345,15 +400,15 @@ __global__ void __launch_bounds__(kT) k_panel(int s, const CoarseGrid* __restric
 #pragma unroll
         for (int p = 0; p < 4; ++p) P[(4 * ty + q) * kPanelStride + 4 * tx + p] = a[q][p];
     __syncthreads();
-    // V_i = -W_i P (P = -A_ss^-1, symmetric): this thread's columns t = 4 ty .. of V, rows 4 tx ..
+    // this thread's columns t = 4 ty .. of V, rows 2 tx, 2 tx + 1, 32 + ..
     double v[4][4] = {};
+#pragma unroll 4
     for (int t = 0; t < kTile; ++t) {
-        double w[4], c[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            w[q] = Wt[t * kPanelStride + 4 * tx + q];
-            c[q] = P[t * kPanelStride + 4 * ty + q];
-        }
+        const double2 w0 = *reinterpret_cast<const double2*>(Wt + t * kPanelStride + 2 * tx);
+        const double2 w1 = *reinterpret_cast<const double2*>(Wt + t * kPanelStride + 32 + 2 * tx);
+        const double2 c0 = *reinterpret_cast<const double2*>(P + t * kPanelStride + 4 * ty);
+        const double2 c1 = *reinterpret_cast<const double2*>(P + t * kPanelStride + 4 * ty + 2);
+        const double w[4] = {w0.x, w0.y, w1.x, w1.y}, c[4] = {c0.x, c0.y, c1.x, c1.y};
 #pragma unroll
         for (int q = 0; q < 4; ++q)
 #pragma unroll
@@ -361,35 +416,37 @@ __global__ void __launch_bounds__(kT) k_panel(int s, const CoarseGrid* __restric
     }
     double *Wo = W + g.y0 * kTile + oi, *Vo = V + g.y0 * kTile + oi;
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int p = 0; p < 4; ++p) Vo[(int64_t)(4 * ty + q) * ld + 4 * tx + p] = v[q][p];
+    for (int q = 0; q < 4; ++q) {
+        *reinterpret_cast<double2*>(Vo + (int64_t)(4 * ty + q) * ld + 2 * tx) = make_double2(v[q][0], v[q][1]);
+        *reinterpret_cast<double2*>(Vo + (int64_t)(4 * ty + q) * ld + 32 + 2 * tx) = make_double2(v[q][2], v[q][3]);
+    }
     for (int e = tid; e < kTile * kTile; e += kT)
         Wo[(int64_t)(e / kTile) * ld + e % kTile] = Wt[(e / kTile) * kPanelStride + e % kTile];
 }
 
 // Step s, the rest: A_ij -= V_i W_j^T on the lower tiles, A_is = V_i, A_ss = -A_ss^-1. 64 x 64 x 64 a
-// block, 4 x 4 entries a thread from shared memory (columns 2 tx, 2 tx + 1, 32 + ..: 16-byte reads
-// without bank conflicts). Bound by the FP64 pipe once a step has more tiles than the device has
-// SMs.
-__global__ void __launch_bounds__(kT) k_trail(int s, const CoarseGrid* __restrict__ grids, double* __restrict__ A,
-                                              const double* __restrict__ W, const double* __restrict__ V,
-                                              const double* __restrict__ piv) {
+// block of 128 threads, 8 x 4 entries a thread from shared memory (columns 2 tx, 2 tx + 1, 32 + ..:
+// 16-byte reads without bank conflicts; 6 of them for 32 multiply-adds). Bound by the FP64 pipe once a
+// step has more tiles than the device has SMs.
+constexpr int kTrailT = 128;
+__global__ void __launch_bounds__(kTrailT, 3) k_trail(int s, const CoarseGrid* __restrict__ grids, double* __restrict__ A,
+                                                      const double* __restrict__ W, const double* __restrict__ V,
+                                                      const double* __restrict__ piv) {
     extern __shared__ __align__(16) double sm[];
     const CoarseGrid& g = grids[blockIdx.y];
-    const int tiles = g.ld / kTile;
-    if (s >= tiles || (int64_t)blockIdx.x >= (int64_t)tiles * (tiles + 1) / 2) return;
+    const int tiles = g.ld / kTile, at = blockIdx.x;
+    if (s >= tiles || at >= tiles * (tiles + 1) / 2) return;
     // tile (i, j), j <= i, of the linear index
-    int i = (int)((sqrt(8.0 * (double)blockIdx.x + 1.0) - 1.0) * 0.5);
-    while ((i + 1) * (i + 2) / 2 <= (int)blockIdx.x) ++i;
-    while (i * (i + 1) / 2 > (int)blockIdx.x) --i;
-    const int j = (int)blockIdx.x - i * (i + 1) / 2;
+    int i = (int)((sqrtf(8.0f * (float)at + 1.0f) - 1.0f) * 0.5f);
+    while ((i + 1) * (i + 2) / 2 <= at) ++i;
+    while (i * (i + 1) / 2 > at) --i;
+    const int j = at - i * (i + 1) / 2;
     double* Ai = A + g.dense0;
     const int64_t ld = g.ld, oi = (int64_t)i * kTile, oj = (int64_t)j * kTile;
     const double *Wp = W + g.y0 * kTile, *Vp = V + g.y0 * kTile;
     const int tid = threadIdx.x;
     if (i == s || j == s) {
-        for (int e = tid; e < kTile * kTile; e += kT) {
+        for (int e = tid; e < kTile * kTile; e += kTrailT) {
             const int r = e / kTile, c = e % kTile;
             double x;
             if (i == s && j == s) x = piv[(int64_t)blockIdx.y * kTile * kTile + e];
@@ -400,35 +457,44 @@ __global__ void __launch_bounds__(kT) k_trail(int s, const CoarseGrid* __restric
         return;
     }
     double *sv = sm, *sw = sm + kTile * kTile;
-    for (int e = tid; e < kTile * kTile / 2; e += kT) {
+#pragma unroll 4
+    for (int e = tid; e < kTile * kTile / 2; e += kTrailT) {
         const int t = e / (kTile / 2), q = 2 * (e % (kTile / 2));
         *reinterpret_cast<double2*>(sv + t * kTile + q) = *reinterpret_cast<const double2*>(Vp + t * ld + oi + q);
         *reinterpret_cast<double2*>(sw + t * kTile + q) = *reinterpret_cast<const double2*>(Wp + t * ld + oj + q);
     }
     const int tx = tid & 15, ty = tid >> 4;
-    double acc[4][4] = {};
+    double acc[8][4] = {};
     __syncthreads();
-#pragma unroll 4
+#pragma unroll 2
     for (int t = 0; t < kTile; ++t) {
-        const double2 a0 = *reinterpret_cast<const double2*>(sv + t * kTile + 4 * ty);
-        const double2 a1 = *reinterpret_cast<const double2*>(sv + t * kTile + 4 * ty + 2);
-        const double2 b0 = *reinterpret_cast<const double2*>(sw + t * kTile + 2 * tx);
-        const double2 b1 = *reinterpret_cast<const double2*>(sw + t * kTile + 32 + 2 * tx);
-        const double av[4] = {a0.x, a0.y, a1.x, a1.y}, bv[4] = {b0.x, b0.y, b1.x, b1.y};
+        double av[8], bv[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
+        for (int h = 0; h < 4; ++h) {
+            const double2 x = *reinterpret_cast<const double2*>(sv + t * kTile + 8 * ty + 2 * h);
+            av[2 * h] = x.x;
+            av[2 * h + 1] = x.y;
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const double2 x = *reinterpret_cast<const double2*>(sw + t * kTile + 32 * h + 2 * tx);
+            bv[2 * h] = x.x;
+            bv[2 * h + 1] = x.y;
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
 #pragma unroll
             for (int p = 0; p < 4; ++p) acc[q][p] += av[q] * bv[p];
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
+    for (int q = 0; q < 8; ++q)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            double2* at = reinterpret_cast<double2*>(Ai + (oi + 4 * ty + q) * ld + oj + 32 * h + 2 * tx);
-            double2 x = *at;
+            double2* to = reinterpret_cast<double2*>(Ai + (oi + 8 * ty + q) * ld + oj + 32 * h + 2 * tx);
+            double2 x = *to;
             x.x -= acc[q][2 * h];
             x.y -= acc[q][2 * h + 1];
-            *at = x;
+            *to = x;
         }
 }
 
@@ -732,16 +798,23 @@ void Coarse::plan(int dof, bool fp32, int32_t nb, int64_t blocks, const double* 
 void Coarse::update(const double* vals, cudaStream_t st) {
     if (!active()) return;
     const unsigned n_inst = (unsigned)grids_.size();
-    const int64_t stride = (int64_t)steps_ * kTile;
+    const int64_t stride = (int64_t)steps_ * kTile, d2 = (int64_t)dof_ * dof_;
     const unsigned pg = (unsigned)std::max(1, (nschunks_ + kPairWarps - 1) / kPairWarps);
-    int64_t most = 1;
-    for (const CoarseGrid& g : grids_) most = std::max<int64_t>(most, g.m / dof_);
-    const dim3 dg(grid_of(most * most), n_inst);
+    int64_t most = 1;  // (coarse node, node within reach, entry) of the largest instance
+    for (const CoarseGrid& g : grids_) {
+        int64_t window = 1;
+        for (int a = 0; a < 3; ++a) window *= 2 * std::min(g.span + 1, g.k[a]) + 1;
+        most = std::max<int64_t>(most, g.m / dof_ * window * d2);
+    }
+    const dim3 dg(grid_of(most), n_inst);
+    CK(cudaMemsetAsync(A_, 0, (size_t)dense_ * sizeof(double), st));
     if (dof_ == 3) {
         k_pairs<3><<<pg, kPairWarps * 32, 0, st>>>(nschunks_, schunk_, bpos_, brow_, bcol_, pos_, vals, spart_);
+        k_pair_sums<3><<<grid_of(nseg_ * 64 * d2), kT, 0, st>>>(nseg_, schunk_ptr_, spart_);
         k_dense<3><<<dg, kT, 0, st>>>(d_grids_, table_, schunk_ptr_, spart_, A_, diag_, stride);
     } else {
         k_pairs<1><<<pg, kPairWarps * 32, 0, st>>>(nschunks_, schunk_, bpos_, brow_, bcol_, pos_, vals, spart_);
+        k_pair_sums<1><<<grid_of(nseg_ * 64 * d2), kT, 0, st>>>(nseg_, schunk_ptr_, spart_);
         k_dense<1><<<dg, kT, 0, st>>>(d_grids_, table_, schunk_ptr_, spart_, A_, diag_, stride);
     }
     CK(cudaGetLastError());
@@ -751,13 +824,13 @@ void Coarse::update(const double* vals, cudaStream_t st) {
     CK(cudaFuncSetAttribute(k_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, psmem));
     for (int s = 0; s < steps_; ++s) {
         k_panel<<<dim3(steps_, n_inst), kT, psmem, st>>>(s, d_grids_, A_, diag_, stride, panel_w_, panel_v_, piv_);
-        k_trail<<<dim3(steps_ * (steps_ + 1) / 2, n_inst), kT, smem, st>>>(s, d_grids_, A_, panel_w_, panel_v_, piv_);
+        k_trail<<<dim3(steps_ * (steps_ + 1) / 2, n_inst), kTrailT, smem, st>>>(s, d_grids_, A_, panel_w_, panel_v_, piv_);
     }
     const dim3 mg(2 * steps_, 2 * steps_, n_inst);
     if (fp32_) k_mirror<float><<<mg, kT, 0, st>>>(d_grids_, A_, static_cast<float*>(inv_));
     else k_mirror<double><<<mg, kT, 0, st>>>(d_grids_, A_, static_cast<double*>(inv_));
     CK(cudaGetLastError());
-    counted(3 + 2 * steps_);
+    counted(4 + 2 * steps_);
 }
 
 template <typename T>

@@ -142,14 +142,9 @@ __device__ __noinline__ double coarse_apply(const CoarseDev<T> c, int32_t warp, 
     double loc = 0.0;
     for (int32_t e = warp; e < c.m; e += nwarps) {
         const T* row = c.inv + (int64_t)e * c.ld;
-        T s0 = T(0), s1 = T(0);  // ld is a multiple of 64, zero beyond m in the matrix and in rc
-        int32_t q = lane * V;
-        for (; q + 32 * V < c.ld; q += 64 * V) {
-            s0 = coarse_dot16(row + q, c.rc + q, s0);
-            s1 = coarse_dot16(row + q + 32 * V, c.rc + q + 32 * V, s1);
-        }
-        if (q < c.ld) s0 = coarse_dot16(row + q, c.rc + q, s0);
-        T s = s0 + s1;
+        T s = T(0);  // ld is a multiple of 64, zero beyond m in the matrix and in rc
+#pragma unroll 8
+        for (int32_t q = lane * V; q < c.ld; q += 32 * V) s = coarse_dot16(row + q, c.rc + q, s);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (lane == 0) {
