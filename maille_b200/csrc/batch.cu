@@ -104,6 +104,7 @@ struct MailleGpuBatch {
     bool any_imposed = false;
     Symbolic sym;
     std::vector<int32_t> row_inst;
+    SideStream side;  // the coarse correction's set-up runs beside the factorisation
     Coarse coarse;  // the preconditioner's coarse correction, a grid per instance
     // device: inputs (packed numbering)
     double *coords = nullptr, *young = nullptr, *poisson = nullptr, *imposed = nullptr, *f0 = nullptr,
@@ -179,6 +180,7 @@ struct MailleGpuBatch {
                          t[0] * 1e-6, t[1] * 1e-6, t[2] * 1e-6, t[3] * 1e-6, t[4] * 1e-6, t[5] * 1e-6,
                          t[7] * 1e-6, t[6], grid);
         }
+        side.finish();
         release_config();
         void* bufs[] = {coords, young, poisson, imposed, f0, f, conn, fixed, perm, inv, col, lrow, inc,
                         belem, bnodes, elem_slot, fixmask, row_ptr, diag, tpos, lslot, lptr, inc_ptr,
@@ -278,14 +280,19 @@ bool check_batch(const MailleBatchProblem* p, Error& err) {
     return true;
 }
 
-int32_t factorize(MailleGpuBatch* b, Error& err, int32_t* dfail) {
+// `meanwhile` enqueues what may run beside the first attempt on another stream.
+template <typename F>
+int32_t factorize(MailleGpuBatch* b, Error& err, int32_t* dfail, F meanwhile) {
     const Pattern pt = b->pattern();
+    bool first = true;
     for (double shift : kShifts) {
         CK(cudaMemsetAsync(dfail, 0, sizeof(int32_t), b->st));
         for (int l = 0; l < b->sym.levels; ++l)
             launch_factor_level(pt, b->sym.level_ptr[l], b->sym.level_ptr[l + 1], b->K, b->F, shift, dfail,
                                 b->st);
         CK(cudaGetLastError());
+        if (first) meanwhile();
+        first = false;
         int32_t failed = 0;
         CK(cudaMemcpyAsync(&failed, dfail, sizeof(int32_t), cudaMemcpyDeviceToHost, b->st));
         CK(cudaStreamSynchronize(b->st));
@@ -308,9 +315,12 @@ int32_t numeric(MailleGpuBatch* b, Error& err) {
     CK(cudaGetLastError());
     CK(cudaEventRecord(b->ev[6], b->st));
     int32_t* dfail = dalloc<int32_t>(1);
-    const int32_t status = factorize(b, err, dfail);
+    cudaStream_t side = b->coarse.active() ? b->side.fork(b->st) : nullptr;
+    const int32_t status = factorize(b, err, dfail, [&] {
+        if (side) b->coarse.update(b->K, side);
+    });
+    b->side.join(b->st);
     dfree(dfail);
-    if (status == MAILLE_OK) b->coarse.update(b->K, b->st);
     CK(cudaEventRecord(b->ev[7], b->st));
     return status;
 }

@@ -70,6 +70,43 @@ T* dupload(const T* src, size_t n, cudaStream_t st) {
 
 inline void dfree(void* p) { device_free(p); }
 
+// A second stream beside a main one, for work that the main stream's next steps do not need: fork()
+// makes it wait for everything enqueued on the main stream, join() makes the main stream wait for it.
+// Its work may use the main stream's buffers between the two; the destructor waits for it.
+struct SideStream {
+    cudaStream_t st = nullptr;
+    cudaEvent_t from = nullptr, to = nullptr;
+    bool forked = false;
+    cudaStream_t fork(cudaStream_t main) {
+        if (!st) {
+            CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+            CK(cudaEventCreateWithFlags(&from, cudaEventDisableTiming));
+            CK(cudaEventCreateWithFlags(&to, cudaEventDisableTiming));
+        }
+        CK(cudaEventRecord(from, main));
+        CK(cudaStreamWaitEvent(st, from, 0));
+        forked = true;
+        return st;
+    }
+    void join(cudaStream_t main) {
+        if (!forked) return;
+        forked = false;
+        CK(cudaEventRecord(to, st));
+        CK(cudaStreamWaitEvent(main, to, 0));
+    }
+    void finish() {
+        if (st) {
+            cudaStreamSynchronize(st);
+            cudaStreamDestroy(st);
+        }
+        if (from) cudaEventDestroy(from);
+        if (to) cudaEventDestroy(to);
+        st = nullptr;
+        from = to = nullptr;
+    }
+    ~SideStream() { finish(); }
+};
+
 constexpr double kDefaultTol = 1e-12;      // iterative.rs:9
 constexpr int32_t kDefaultMaxIter = 10000;  // iterative.rs:11
 constexpr double kShifts[6] = {0.0, 1e-3, 1e-2, 1e-1, 1.0, 10.0};  // iterative.rs:14

@@ -134,6 +134,7 @@ struct MailleGpuHandle {
     double* ke = nullptr;
     double *K = nullptr, *F = nullptr;
     SellBuf sk;      // K, sliced, for the SpMV
+    SideStream side;  // the coarse correction's set-up runs beside the factorisation
     Coarse coarse;   // the preconditioner's coarse correction (multicolour orderings)
     PsellBuf pl, pu;  // strictly lower / upper blocks of the factor, packed, for the sweeps
     double *Ks64 = nullptr, *Ls64 = nullptr, *Us64 = nullptr, *D64 = nullptr;

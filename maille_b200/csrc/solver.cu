@@ -43,6 +43,7 @@ thread_local std::string g_last_error;
 
 MailleGpuHandle::~MailleGpuHandle() {
     cudaSetDevice(device);
+    side.finish();
     if (st) cudaStreamSynchronize(st);
     if (timing) {
         unsigned long long t[8] = {0};
@@ -261,14 +262,19 @@ void build_rhs(MailleGpuHandle* h) {
     launch_build_rhs(h->sym.nb, h->perm, h->fixmask, h->f_cur, coupling, h->b64, h->st);
 }
 
-int32_t factorize(MailleGpuHandle* h, Error& err) {
+// `meanwhile` enqueues what may run beside the first attempt on another stream.
+template <typename F>
+int32_t factorize(MailleGpuHandle* h, Error& err, F meanwhile) {
     const Pattern pt = h->pattern();
+    bool first = true;
     for (double shift : kShifts) {
         CK(cudaMemsetAsync(h->dfail, 0, sizeof(int32_t), h->st));
         for (int l = 0; l < h->sym.levels; ++l)
             launch_factor_level(pt, h->sym.level_ptr[l], h->sym.level_ptr[l + 1], h->K, h->F, shift,
                                 h->dfail, h->st);
         CK(cudaGetLastError());
+        if (first) meanwhile();
+        first = false;
         int32_t failed = 0;
         CK(cudaMemcpyAsync(&failed, h->dfail, sizeof(int32_t), cudaMemcpyDeviceToHost, h->st));
         CK(cudaStreamSynchronize(h->st));
@@ -299,7 +305,14 @@ int32_t assemble_factor(MailleGpuHandle* h, Error& err) {
     launch_sell_fill<double>(h->sk.h.steps(), h->sk.src, h->K, h->Ks64, st);
     CK(cudaGetLastError());
     CK(cudaEventRecord(h->ev[2], st));
-    if (factorize(h, err) != MAILLE_OK) return err.status;
+    // the coarse correction needs K only: its chain of small launches runs beside the factorisation's
+    // latency-bound levels
+    cudaStream_t side = h->coarse.active() ? h->side.fork(st) : nullptr;
+    const int32_t status = factorize(h, err, [&] {
+        if (side) h->coarse.update(h->K, side);
+    });
+    h->side.join(st);
+    if (status != MAILLE_OK) return err.status;
     if (is_mixed(h)) {
         launch_sell_fill<float>(h->sk.h.steps(), h->sk.src, h->K, h->Ks32, st);
         launch_sell_fill<float>(h->pl.h.steps(), h->pl.src, h->F, h->Ls32, st);
@@ -310,7 +323,6 @@ int32_t assemble_factor(MailleGpuHandle* h, Error& err) {
         launch_sell_fill<double>(h->pu.h.steps(), h->pu.src, h->F, h->Us64, st);
         launch_diag_fill<double>(s.nb, h->diag, h->F, h->D64, st);
     }
-    h->coarse.update(h->K, st);
     CK(cudaGetLastError());
     CK(cudaEventRecord(h->ev[3], st));
     return MAILLE_OK;

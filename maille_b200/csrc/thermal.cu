@@ -1269,6 +1269,7 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
     cudaEvent_t ev[7] = {};
     DevBufs mem;
     Coarse coarse;
+    SideStream side;  // declared after the buffers its work uses: it is waited for before they go
     Slices sk, sl, su;
     sk.kind = SELL_FULL;
     sl.kind = SELL_LOWER;
@@ -1414,6 +1415,8 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
         CK(cudaEventRecord(ev[6], st));
         // IC(0) with the shift ladder (Pcg::new, iterative.rs:201-207)
         int32_t* dfail = mem.take(dalloc<int32_t>(1));
+        // the coarse correction needs A only: its set-up runs beside the factorisation
+        cudaStream_t beside = coarse.active() ? side.fork(st) : nullptr;
         double shift_used = -1.0;
         for (double shift : kShifts) {
             CK(cudaMemsetAsync(dfail, 0, sizeof(int32_t), st));
@@ -1425,6 +1428,8 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
                     pt.row_ptr, pt.col, pt.diag, pt.tpos, r0, r1, A, F, shift, dfail);
             }
             CK(cudaGetLastError());
+            if (beside) coarse.update(A, beside);
+            beside = nullptr;  // with the first attempt only
             int32_t h_fail = 0;
             CK(cudaMemcpyAsync(&h_fail, dfail, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));
@@ -1434,8 +1439,7 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
             }
         }
         if (shift_used < 0.0) return th_fail(MAILLE_SINGULAR, "Singular: IC(0) failed for every diagonal shift");
-        // the coarse correction, as in the elastic solve (solver.cu)
-        coarse.update(A, st);
+        side.join(st);
         // iteration operands
         auto slots = [&](const Slices& s) { return (int64_t)s.h.steps() * kStepSlots; };
         double* Av = mem.take(dalloc<double>((size_t)slots(sk)));
