@@ -76,6 +76,9 @@ struct CoarseBatchDev {
 };
 constexpr int kCoarseTileRows = 16;
 
+// Mixed forms with the correction: reliable update when the FP32 residual fell by this factor.
+constexpr double kCoarseDelta = 0.01;
+
 // The correction of one system (one or several instances): plan and numeric state.
 class Coarse {
   public:

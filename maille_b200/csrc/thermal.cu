@@ -1589,7 +1589,7 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
                 HeatPcg<float> a{nb, sk.dev(), sl.dev(), su.dev(), bwd_slice, Av32, Lv32, Uv32, D32, b, x32, r32,
                                  p32, ap32, yrec32, zrec32, partials, timeout, epoch0, tol, max_iter,
                                  d_status + (s - 1), d_iters + (s - 1), d_rel + (s - 1), timing,
-                                 Av, x, r64, kHeatDelta, coarse.dev32()};
+                                 Av, x, r64, coarse.active() ? kCoarseDelta : kHeatDelta, coarse.dev32()};
                 void* args[] = {&a};
                 CK(cudaLaunchCooperativeKernel(pcg_fn, dim3(grid), dim3(kT), args, csmem, st));
             }
