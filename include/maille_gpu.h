@@ -53,8 +53,8 @@ typedef enum {
  * with its Galerkin matrix inverted densely): the same stopping test, statuses and results, in
  * 5 to 12 times fewer iterations. RCM keeps IC(0) alone, for the reference's iteration counts. */
 typedef enum {
-    MAILLE_ORDER_AUTO = 0,           /* the path's measured best: MULTICOLOR_ITERATED for the
-                                        elastic solves, MULTICOLOR_BFS for the thermal step */
+    MAILLE_ORDER_AUTO = 0,           /* the path's measured best: greedy colouring visited by node
+                                        index, then one pass of iterated greedy (no searches) */
     MAILLE_ORDER_MULTICOLOR = 1,     /* greedy colouring of the node graph visited in RCM order:
                                         one level per colour, a few dozen levels */
     MAILLE_ORDER_RCM = 2,            /* reverse Cuthill-McKee on the node graph (the reference's
@@ -109,9 +109,7 @@ typedef struct {
     int64_t block_rows;         /* free nodes in the 3x3-block system */
     int64_t blocks;             /* 3x3 blocks of the full symmetric pattern */
     int32_t levels;             /* levels of the IC(0) sweeps */
-    double ms_setup;            /* host analysis on a thread that runs while the device takes the
-                                   inputs (create): node incidence and boundary lists, and with
-                                   MAILLE_HOST_ORDERING=1 the ordering too */
+    double ms_setup;            /* 0: the analysis runs on the device (ms_ordering, ms_symbolic) */
     double ms_upload;           /* host -> device copies of the inputs (create) */
     double ms_assembly;         /* scatter-reduce assembly of the element matrices (create,
                                    refactor) */
@@ -122,10 +120,9 @@ typedef struct {
     /* the rest of create, in order on the device stream (each 0 after solve-only calls): */
     double ms_element;          /* element integration (Ke of every element) */
     double ms_ordering;         /* wall time from the element integration to a known ordering:
-                                   the device node incidence, the device ordering (node graph,
-                                   RCM, greedy colouring) and the join of the host thread */
-    double ms_symbolic;         /* device pattern and scatter map (radix sorts), the host plan of
-                                   the sliced layouts and their slot fills */
+                                   node incidence, node graph, ordering */
+    double ms_symbolic;         /* block pattern, boundary lists, the host plan of the sliced
+                                   layouts and their slot fills, the coarse correction's plan */
     double ms_buffers;          /* numeric buffers and the remaining index uploads */
 } MailleElasticResult;
 
@@ -214,8 +211,8 @@ int32_t maille_gpu_spmv_device(MailleGpuHandle* h, int32_t precision, int32_t co
 int64_t maille_gpu_kernel_launches(void);
 
 /* Raise (1) or clear (0) the cancel flag; checked before the PCG's first launch and between its
- * launches. Safe to call
- * from another thread while a solve runs (the Observer / Flow::Stop role, model.rs:1203-1218). */
+ * launches. Safe to call from another thread while a solve runs (the Observer / Flow::Stop role,
+ * model.rs:1203-1218). */
 void maille_gpu_cancel(MailleGpuHandle* h, int32_t flag);
 
 /* CUDA stream (cudaStream_t) the handle launches on, for event timing by the caller. */

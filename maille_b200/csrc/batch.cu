@@ -2,8 +2,8 @@
 // include/maille_gpu.h).
 //
 // create: the instances are packed into one mesh (node ids offset by the instance's first node),
-//   analysed once (setup.cpp: the union graph has one component per instance, so the RCM visit,
-//   the colouring and hence the levels of every instance are those it would get alone), uploaded,
+//   analysed once on the device (the union graph has one component per instance, so the colouring
+//   by node index and hence the levels of every instance are those it would get alone),
 //   integrated, assembled and factorised with the same kernels as a single model. Rows of one
 //   instance couple only to rows of the same instance: the packed matrix is block diagonal.
 // solve: right-hand sides of all load cases, then ONE persistent kernel (batch_kernels.cu) that
@@ -29,10 +29,12 @@
 
 #include <cuda_runtime.h>
 
+#include "analysis.cuh"
 #include "batch.cuh"
 #include "common.hpp"
 #include "cuda_host.hpp"
 #include "kernels.cuh"
+#include "ordering.cuh"
 #include "sparse.cuh"
 
 using namespace maille;
@@ -48,12 +50,14 @@ struct BLayout {
     BSellHost h;
     int32_t *rowid = nullptr, *col = nullptr, *src = nullptr, *inst = nullptr;
     int64_t* off = nullptr;
-    void upload(cudaStream_t st) {
+    void upload(SellKind kind, const Pattern& pt, cudaStream_t st) {
         rowid = dupload(h.rowid.data(), h.rowid.size(), st);
-        col = dupload(h.col.data(), h.col.size(), st);
-        src = dupload(h.src.data(), h.src.size(), st);
         inst = dupload(h.inst.data(), h.inst.size(), st);
         off = dupload(h.off.data(), h.off.size(), st);
+        col = dalloc<int32_t>((size_t)h.steps() * h.slots());
+        src = dalloc<int32_t>((size_t)h.steps() * h.slots());
+        fill_bsell(kind, h.rows, h.sub, h.nslices(), h.steps(), rowid, off, pt.row_ptr, pt.col, pt.diag, pt.nb, col, src,
+                   st);
     }
     void release() {
         for (void* p : {(void*)rowid, (void*)col, (void*)src, (void*)inst, (void*)off}) dfree(p);
@@ -113,12 +117,10 @@ struct MailleGpuBatch {
     int32_t* conn = nullptr;
     uint8_t* fixed = nullptr;
     // device: symbolic
-    int32_t *perm = nullptr, *inv = nullptr, *col = nullptr, *lrow = nullptr, *inc = nullptr,
-            *belem = nullptr, *bnodes = nullptr, *elem_slot = nullptr;
+    int32_t *perm = nullptr, *inv = nullptr, *col = nullptr, *inc = nullptr;
+    BoundaryDev bd;
     uint8_t* fixmask = nullptr;
-    int64_t *row_ptr = nullptr, *diag = nullptr, *tpos = nullptr, *lslot = nullptr, *lptr = nullptr,
-            *inc_ptr = nullptr;
-    uint32_t* contrib = nullptr;
+    int64_t *row_ptr = nullptr, *diag = nullptr, *tpos = nullptr, *inc_ptr = nullptr;
     // device: numeric (CSR), coupling scratch
     double *ke = nullptr, *K = nullptr, *F = nullptr, *y_full = nullptr, *ye = nullptr;
     double shift = 0.0;
@@ -182,12 +184,13 @@ struct MailleGpuBatch {
         }
         side.finish();
         release_config();
-        void* bufs[] = {coords, young, poisson, imposed, f0, f, conn, fixed, perm, inv, col, lrow, inc,
-                        belem, bnodes, elem_slot, fixmask, row_ptr, diag, tpos, lslot, lptr, inc_ptr,
-                        contrib, ke, K, F, y_full, ye, x, r, z, p, ap, b, x64, r64, u_out, tickets,
-                        flags, timing};
-        for (void* q : bufs) dfree(q);
-        for (void* q : state_bufs) dfree(q);
+        if (st) cudaStreamSynchronize(st);
+        std::vector<void*> all{coords, young, poisson, imposed, f0, f, conn, fixed, perm, inv, col, inc,
+                               bd.belem, bd.bnodes, bd.elem_slot, fixmask, row_ptr, diag, tpos, inc_ptr,
+                               ke, K, F, y_full, ye, x, r, z, p, ap, b, x64, r64, u_out, tickets, flags, timing};
+        all.insert(all.end(), state_bufs.begin(), state_bufs.end());
+        coarse.gather(all);
+        device_free_all(all);
         pinned_slot_free(h_cancel);
         for (auto& e : ev)
             if (e) cudaEventDestroy(e);
@@ -307,11 +310,9 @@ int32_t factorize(MailleGpuBatch* b, Error& err, int32_t* dfail, F meanwhile) {
 
 // element integration + assembly + IC(0) on the packed mesh (CSR K and F)
 int32_t numeric(MailleGpuBatch* b, Error& err) {
-    const Symbolic& s = b->sym;
     ElemIn in{b->n_elems, b->coords, b->conn, b->young, b->poisson};
     launch_elem_stiffness(b->npe, in, b->ke, b->st);
-    launch_assemble(b->pattern(), (int64_t)s.lslot.size(), b->lslot, b->lrow, b->lptr, b->contrib, b->ke, b->K,
-                    b->st);
+    launch_assemble(b->npe, b->pattern(), AssembleIn{b->perm, b->inc_ptr, b->inc, b->conn, b->inv}, b->ke, b->K, b->st);
     CK(cudaGetLastError());
     CK(cudaEventRecord(b->ev[6], b->st));
     int32_t* dfail = dalloc<int32_t>(1);
@@ -361,7 +362,9 @@ bool apply_config(MailleGpuBatch* b, const BatchConfig& c, Error& err) {
         build_bsell(b->sym, SELL_UPPER, rows, c.SUB, b->row_inst, b->lu.h);
         tk.join();
         tl.join();
-        for (BLayout* l : {&b->lk, &b->ll, &b->lu}) l->upload(st);
+        b->lk.upload(SELL_FULL, b->pattern(), st);
+        b->ll.upload(SELL_LOWER, b->pattern(), st);
+        b->lu.upload(SELL_UPPER, b->pattern(), st);
         const size_t ek = (size_t)b->lk.h.steps() * 9 * shp.slots(), el = (size_t)b->ll.h.steps() * 9 * shp.slots(),
                      eu = (size_t)b->lu.h.steps() * 9 * shp.slots();
         if (b->mixed()) {
@@ -502,9 +505,9 @@ void enqueue_rhs(MailleGpuBatch* b) {
     const int64_t n3 = 3 * b->n_nodes;
     if (b->any_imposed) {
         CK(cudaMemsetAsync(b->y_full, 0, n3 * sizeof(double), b->st));
-        launch_elem_apply(b->npe, (int64_t)s.belem.size(), b->belem, b->conn, b->ke, b->imposed, b->ye, b->st);
-        launch_node_gather(b->npe, (int64_t)s.bnodes.size(), b->bnodes, b->inc_ptr, b->inc, b->elem_slot, b->ye,
-                           b->y_full, b->st);
+        launch_elem_apply(b->npe, b->bd.nbelem, b->bd.belem, b->conn, b->ke, b->imposed, b->ye, b->st);
+        launch_node_gather(b->npe, b->bd.nbnodes, b->bd.bnodes, b->inc_ptr, b->inc, b->bd.elem_slot, b->ye, b->y_full,
+                           b->st);
         coupling = b->y_full;
     }
     launch_batch_rhs(s.nb, b->R, b->n_rhs, n3, b->perm, b->fixmask, b->f_cur, coupling, b->b, b->st);
@@ -622,31 +625,13 @@ int32_t create_batch(const MailleBatchProblem* p, MailleGpuBatch** out) {
     b->h_f0.assign((size_t)n3 * b->n_rhs, 0.0);
     if (p->f) std::memcpy(b->h_f0.data(), p->f, b->h_f0.size() * sizeof(double));
 
-    // the packed mesh: node ids offset by the instance's first node
-    const double t0 = now_ms();
-    std::vector<int64_t> conn((size_t)b->n_elems * b->npe);
+    if (b->n_nodes >= (int64_t(1) << 30) || b->n_elems * node_pairs(b->npe) >= (int64_t(1) << 31))
+        return fail({MAILLE_INVALID_INPUT, "mesh too large for 32-bit element-pair indices"});
     for (int32_t k = 0; k < b->n_inst; ++k)
-        for (int64_t e = b->elem_off[k] * b->npe; e < b->elem_off[k + 1] * b->npe; ++e)
-            conn[e] = p->conn[e] + b->node_off[k];
-    if (!analyse(b->n_nodes, b->npe, b->n_elems, conn.data(), b->h_fixed.data(), MAILLE_ORDER_MULTICOLOR, b->sym,
-                 err))
-        return fail(err);
-    const Symbolic& s = b->sym;
-    if (s.levels >= kMaxLevels) return fail({MAILLE_INVALID_INPUT, "too many IC(0) levels"});
-    b->row_inst.resize(s.nb);
-    {
-        std::vector<int32_t> node_inst(b->n_nodes);
-        for (int32_t k = 0; k < b->n_inst; ++k)
-            for (int64_t v = b->node_off[k]; v < b->node_off[k + 1]; ++v) node_inst[v] = k;
-        std::vector<int64_t> rows(b->n_inst, 0);
-        for (int32_t r = 0; r < s.nb; ++r) {
-            b->row_inst[r] = node_inst[s.perm[r]];
-            rows[b->row_inst[r]]++;
-        }
-        for (int32_t k = 0; k < b->n_inst; ++k)
-            if (rows[k] == 0) return fail({MAILLE_INVALID_INPUT, "instance " + std::to_string(k) + ": every DOF is fixed"});
-    }
-    const double t1 = now_ms();
+        if (std::all_of(b->h_fixed.begin() + 3 * b->node_off[k], b->h_fixed.begin() + 3 * b->node_off[k + 1],
+                        [](uint8_t f) { return f != 0; }))
+            return fail({MAILLE_INVALID_INPUT, "instance " + std::to_string(k) + ": every DOF is fixed"});
+    const double t0 = now_ms();
     try {
         int ndev = 0;
         CK(cudaGetDeviceCount(&ndev));
@@ -657,8 +642,11 @@ int32_t create_batch(const MailleBatchProblem* p, MailleGpuBatch** out) {
         for (auto& e : b->ev) CK(cudaEventCreate(&e));
         cudaStream_t st = b->st;
         CK(cudaEventRecord(b->ev[4], st));
-        std::vector<int32_t> conn32(conn.size());
-        for (size_t k = 0; k < conn.size(); ++k) conn32[k] = (int32_t)conn[k];
+        // the packed mesh: node ids offset by the instance's first node
+        std::vector<int32_t> conn32((size_t)b->n_elems * b->npe);
+        for (int32_t k = 0; k < b->n_inst; ++k)
+            for (int64_t e = b->elem_off[k] * b->npe; e < b->elem_off[k + 1] * b->npe; ++e)
+                conn32[e] = (int32_t)(p->conn[e] + b->node_off[k]);
         b->coords = dupload(p->coords, n3, st);
         b->conn = dupload(conn32.data(), conn32.size(), st);
         b->young = dupload(p->young, b->n_elems, st);
@@ -668,35 +656,52 @@ int32_t create_batch(const MailleBatchProblem* p, MailleGpuBatch** out) {
         b->f0 = dupload(b->h_f0.data(), b->h_f0.size(), st);
         b->f = dalloc<double>(b->h_f0.size());
         b->f_cur = b->f0;
-        b->perm = dupload(s.perm.data(), s.perm.size(), st);
-        b->inv = dupload(s.inv.data(), s.inv.size(), st);
-        b->fixmask = dupload(s.fixmask.data(), s.fixmask.size(), st);
-        b->row_ptr = dupload(s.row_ptr.data(), s.row_ptr.size(), st);
-        b->col = dupload(s.col.data(), s.col.size(), st);
-        b->diag = dupload(s.diag.data(), s.diag.size(), st);
-        b->tpos = dupload(s.tpos.data(), s.tpos.size(), st);
-        std::vector<int32_t> lrow(s.lslot.size());
+        // the analysis of the packed mesh: the union graph has one component per instance
+        const int64_t nconn = b->n_elems * b->npe;
+        b->inc_ptr = dalloc<int64_t>(b->n_nodes + 1);
+        b->inc = dalloc<int32_t>(nconn);
+        gpu_incidence(b->conn, nconn, b->n_nodes, st, b->inc_ptr, b->inc);
+        Symbolic& s = b->sym;
         {
-            size_t q = 0;
-            for (int32_t r = 0; r < s.nb; ++r)
-                for (int64_t pp = s.row_ptr[r]; pp <= s.diag[r]; ++pp) lrow[q++] = r;
+            Scratch tmp(st);
+            GraphDev graph;
+            int32_t *kept_of = tmp.take<int32_t>(b->n_nodes), *kept = tmp.take<int32_t>(b->n_nodes);
+            const int32_t nk = gpu_keep(3, b->n_nodes, b->fixed, st, kept_of, kept);
+            int32_t *order = tmp.take<int32_t>(nk), *rank = tmp.take<int32_t>(nk);
+            gpu_graph(b->npe, b->n_elems, b->conn, b->inc_ptr, b->inc, kept_of, kept, nk, st, graph);
+            gpu_ordering(graph, kOrderIndex, st, order, s.level_ptr);
+            s.levels = (int32_t)s.level_ptr.size() - 1;
+            s.nb = nk;
+            s.free_dofs = std::count(b->h_fixed.begin(), b->h_fixed.end(), (uint8_t)0);
+            if (s.levels >= kMaxLevels) return fail({MAILLE_INVALID_INPUT, "too many IC(0) levels"});
+            b->perm = dalloc<int32_t>(nk);
+            b->inv = dalloc<int32_t>(b->n_nodes);
+            b->fixmask = dalloc<uint8_t>(nk);
+            gpu_rows(3, nk, b->n_nodes, order, kept, kept_of, b->fixed, st, b->perm, b->inv, rank, b->fixmask);
+            PatternDev pt;
+            gpu_pattern(graph, order, rank, st, pt, s.row_ptr, s.diag);
+            b->row_ptr = pt.row_ptr;
+            b->col = pt.col;
+            b->diag = pt.diag;
+            b->tpos = pt.tpos;
+            s.blocks = pt.blocks;
+            s.perm.resize(nk);
+            CK(cudaMemcpyAsync(s.perm.data(), b->perm, nk * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+            gpu_boundary(b->npe, b->n_elems, b->conn, b->n_nodes, b->fixed, b->inc_ptr, st, b->bd);
         }
-        b->lslot = dupload(s.lslot.data(), s.lslot.size(), st);
-        b->lrow = dupload(lrow.data(), lrow.size(), st);
-        b->lptr = dupload(s.lptr.data(), s.lptr.size(), st);
-        b->contrib = dupload(s.contrib.data(), s.contrib.size(), st);
-        b->inc_ptr = dupload(s.inc_ptr.data(), s.inc_ptr.size(), st);
-        b->inc = dupload(s.inc.data(), s.inc.size(), st);
-        b->belem = dupload(s.belem.data(), s.belem.size(), st);
-        b->bnodes = dupload(s.bnodes.data(), s.bnodes.size(), st);
-        std::vector<int32_t> slot(b->n_elems, -1);
-        for (size_t k = 0; k < s.belem.size(); ++k) slot[s.belem[k]] = (int32_t)k;
-        b->elem_slot = dupload(slot.data(), slot.size(), st);
+        b->row_inst.resize(s.nb);
+        {
+            std::vector<int32_t> node_inst(b->n_nodes);
+            for (int32_t k = 0; k < b->n_inst; ++k)
+                std::fill(node_inst.begin() + b->node_off[k], node_inst.begin() + b->node_off[k + 1], k);
+            for (int32_t r = 0; r < s.nb; ++r) b->row_inst[r] = node_inst[s.perm[r]];
+        }
+        const double t1 = now_ms();
         b->ke = dalloc<double>((size_t)b->n_elems * node_pairs(b->npe) * 9);
         b->K = dalloc<double>((size_t)s.blocks * 9);
         b->F = dalloc<double>((size_t)s.blocks * 9);
         b->y_full = dalloc<double>(n3);
-        b->ye = dalloc<double>(std::max<size_t>(1, s.belem.size()) * 3 * b->npe);
+        b->ye = dalloc<double>(std::max<int64_t>(1, b->bd.nbelem) * 3 * b->npe);
         const size_t nv = b->vec_len();
         const size_t tsz = b->mixed() ? sizeof(float) : sizeof(double);
         for (void** q : {&b->x, &b->r, &b->z, &b->p, &b->ap}) {
@@ -771,10 +776,10 @@ int32_t create_batch(const MailleBatchProblem* p, MailleGpuBatch** out) {
         if (numeric(b.get(), err) != MAILLE_OK) return fail(err);
         CK(cudaStreamSynchronize(st));
         b->h_ctrl.assign(8, 0);
+        b->sym.ms = t1 - t0;
     } catch (const CudaFailure& e) {
         return fail({MAILLE_CUDA_ERROR, e.what});
     }
-    b->sym.ms = t1 - t0;
     *out = b.release();
     return MAILLE_OK;
 }

@@ -115,7 +115,6 @@ struct MailleGpuHandle {
     int32_t max_iter = kDefaultMaxIter;
     double delta = 0.3;  // reliable update when the FP32 residual fell by this factor
     std::vector<uint8_t> h_fixed;
-    std::vector<double> h_f, h_f0;
     bool any_imposed = false;
     // device: inputs (caller numbering)
     double *coords = nullptr, *young = nullptr, *poisson = nullptr, *imposed = nullptr, *f = nullptr,
@@ -124,12 +123,12 @@ struct MailleGpuHandle {
     int32_t* conn = nullptr;
     uint8_t* fixed = nullptr;
     // device: symbolic
-    int32_t *perm = nullptr, *inv = nullptr, *col = nullptr, *lrow = nullptr;
+    int32_t *perm = nullptr, *inv = nullptr, *col = nullptr;
     uint8_t* fixmask = nullptr;
-    int64_t *row_ptr = nullptr, *diag = nullptr, *tpos = nullptr, *lslot = nullptr, *lptr = nullptr;
-    uint32_t* contrib = nullptr;
+    int64_t *row_ptr = nullptr, *diag = nullptr, *tpos = nullptr;
     int64_t* inc_ptr = nullptr;
-    int32_t *inc = nullptr, *belem = nullptr, *bnodes = nullptr, *elem_slot = nullptr;
+    int32_t* inc = nullptr;
+    BoundaryDev bd;  // elements and nodes of the reactions
     // device: numeric (CSR K and factor F; sliced copies for the iterations)
     double* ke = nullptr;
     double *K = nullptr, *F = nullptr;
@@ -153,7 +152,7 @@ struct MailleGpuHandle {
     double* dsum = nullptr;        // [4] misc sums
     double* h_sum = nullptr;       // pinned [4]
     unsigned int* dticket = nullptr;
-    int32_t* dfail = nullptr;
+    int32_t* dfail = nullptr;  // [2]
     int spmv_grid = 1;
     int persist_grid = 0;             // co-resident grid of the persistent PCG kernel
     int persist_chunk = 64;           // iterations per persistent launch
@@ -165,6 +164,7 @@ struct MailleGpuHandle {
     Pattern pattern() const {
         return Pattern{sym.nb, row_ptr, col, diag, tpos, fixmask};
     }
+    AssembleIn assembly() const { return AssembleIn{perm, inc_ptr, inc, conn, inv}; }
     ~MailleGpuHandle();
 };
 

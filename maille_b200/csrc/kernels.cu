@@ -6,6 +6,7 @@
 #include <atomic>
 #include <cmath>
 
+#include "cuda_host.hpp"
 #include "kernels.cuh"
 #include "reduce.cuh"
 #include "tet.cuh"
@@ -114,48 +115,88 @@ __global__ void __launch_bounds__(kThreads) k_elem_stiffness(ElemIn in, double* 
 
 // ---- deterministic assembly -----------------------------------------------------------------
 
-// One thread per lower slot (I, J), J <= I: sums its element-pair blocks in the order of the
-// precomputed map (element order), applies the identity rows/columns of fixed DOFs, and writes
-// the block and its transpose.
-__global__ void k_assemble(Pattern pt, int64_t nl, const int64_t* __restrict__ lslot,
-                           const int32_t* __restrict__ lrow, const int64_t* __restrict__ lptr,
-                           const uint32_t* __restrict__ contrib, const double* __restrict__ ke,
-                           double* __restrict__ K) {
-    const int64_t l = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (l >= nl) return;
-    const int64_t pos = lslot[l];
-    const int32_t I = lrow[l], J = pt.col[pos];
-    double s[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int64_t k = lptr[l]; k < lptr[l + 1]; ++k) {
-        const uint32_t c = contrib[k];
-        const double* B = ke + (int64_t)(c & 0x7fffffffu) * 9;
-        if (c & 0x80000000u) {
+// K rows from the element matrices: one warp per row walks the elements incident to its node in element
+// order; the npe blocks of an element's row find their columns by binary search among the row's
+// (in shared memory) and are added to the row's sums there, 32 entries at a time. Every entry is thus
+// summed in element order, the same in K_IJ and K_JI, with no map from element pairs to slots
+// (whose sort took longer than the assembly: 38.4 M pairs on Tet10 40^3). A row of more than kAsmCols
+// blocks is taken in windows. Bound by the gather of the element blocks, each read twice.
+constexpr int kAsmCols = 72;
+template <int NPE>
+__global__ void __launch_bounds__(kThreads) k_assemble(Pattern pt, AssembleIn in, const double* __restrict__ ke,
+                                                       double* __restrict__ K) {
+    constexpr int NP = NPE * (NPE + 1) / 2;
+    __shared__ double sums[kWarps][kAsmCols * 9];
+    __shared__ int32_t cols[kWarps][kAsmCols];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int64_t I = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (I >= pt.nb) return;
+    double* sum = sums[wp];
+    int32_t* col = cols[wp];
+    const int32_t v = in.perm[I];
+    const int64_t q0 = in.inc_ptr[v], q1 = in.inc_ptr[v + 1], rb = pt.row_ptr[I];
+    const int n = (int)(pt.row_ptr[I + 1] - rb);
+    const uint8_t mi = pt.fixmask[I];
+    for (int c0 = 0; c0 < n; c0 += kAsmCols) {
+        const int nc = min(kAsmCols, n - c0);
+        for (int t = lane; t < nc; t += 32) col[t] = pt.col[rb + c0 + t];
+        for (int t = lane; t < nc * 9; t += 32) sum[t] = 0.0;
+        __syncwarp();
+        // G elements at a time: lane g NPE + b looks node b of element g up, all their entries are
+        // requested, then added element by element
+        constexpr int G = 32 / NPE, V = (NPE * 9 + 31) / 32;
+        const int g = lane / NPE, b = lane % NPE;
+        for (int64_t q = q0; q < q1; q += G) {
+            int32_t pos = 0;
+            int slot = -1;
+            if (g < G && q + g < q1) {
+                pos = in.inc[q + g];
+                const int32_t J = in.inv[in.conn[(int64_t)(pos / NPE) * NPE + b]];
+                int lo = 0, hi = J < 0 ? 0 : nc;
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    if (col[mid] < J) lo = mid + 1; else hi = mid;
+                }
+                if (J >= 0 && lo < nc && col[lo] == J) slot = lo;
+            }
+            double x[G][V];
+            int at[G][V];
 #pragma unroll
-            for (int r = 0; r < 3; ++r)
+            for (int k = 0; k < G; ++k) {
+                const int32_t p = __shfl_sync(0xffffffffu, pos, k * NPE);
+                const int64_t e = p / NPE;
+                const int a = p - (int)(e * NPE);
 #pragma unroll
-                for (int q = 0; q < 3; ++q) s[3 * r + q] += B[3 * q + r];
-        } else {
+                for (int h = 0; h < V; ++h) {
+                    const int t = 32 * h + lane, n1 = t / 9, w = t - 9 * n1;
+                    at[k][h] = __shfl_sync(0xffffffffu, slot, k * NPE + (n1 < NPE ? n1 : 0));
+                    if (t >= NPE * 9) at[k][h] = -1;
+                    if (at[k][h] >= 0) {
+                        const int lo = min(a, n1), hi = max(a, n1);
+                        const int pair = lo * NPE - lo * (lo - 1) / 2 + (hi - lo);
+                        // the block of (lo, hi) is stored with lo's components as rows
+                        x[k][h] = __ldg(ke + (e * NP + pair) * 9 + (a <= n1 ? w : (w % 3) * 3 + w / 3));
+                        at[k][h] = at[k][h] * 9 + w;
+                    }
+                }
+            }
 #pragma unroll
-            for (int q = 0; q < 9; ++q) s[q] += B[q];
+            for (int k = 0; k < G; ++k) {
+#pragma unroll
+                for (int h = 0; h < V; ++h)
+                    if (at[k][h] >= 0) sum[at[k][h]] += x[k][h];
+                __syncwarp();
+            }
         }
-    }
-    const uint8_t mi = pt.fixmask[I], mj = pt.fixmask[J];
-    if (mi | mj) {
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-#pragma unroll
-            for (int q = 0; q < 3; ++q)
-                if (((mi >> r) & 1) || ((mj >> q) & 1)) s[3 * r + q] = (I == J && r == q) ? 1.0 : 0.0;
-    }
-    double* out = K + 9 * pos;
-#pragma unroll
-    for (int q = 0; q < 9; ++q) out[q] = s[q];
-    if (I != J) {
-        double* tr = K + 9 * pt.tpos[pos];
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-#pragma unroll
-            for (int q = 0; q < 3; ++q) tr[3 * q + r] = s[3 * r + q];
+        for (int t = lane; t < nc * 9; t += 32) {
+            const int c = t / 9, w = t - 9 * c, r = w / 3, k = w - 3 * r;
+            const int32_t J = col[c];
+            const uint8_t mj = pt.fixmask[J];
+            double x = sum[t];
+            if (((mi >> r) & 1) || ((mj >> k) & 1)) x = J == (int32_t)I && r == k ? 1.0 : 0.0;
+            K[9 * (rb + c0) + t] = x;
+        }
+        __syncwarp();
     }
 }
 
@@ -486,6 +527,42 @@ __global__ void k_reactions(const int32_t* __restrict__ nodes, int64_t nnodes,
     react[g] = fixed[g] ? y[g] - (f ? f[g] : 0.0) : 0.0;
 }
 
+// a fixed DOF of a node that no element touches: K u = 0 there
+__global__ void k_orphan_reactions(int64_t n_nodes, const int64_t* __restrict__ inc_ptr, const uint8_t* __restrict__ fixed,
+                                   const double* __restrict__ f, double* __restrict__ react) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= 3 * n_nodes) return;
+    const int64_t v = t / 3;
+    if (inc_ptr[v] == inc_ptr[v + 1] && fixed[t]) react[t] = -f[t];
+}
+
+// *bad = 1 when an entry is not finite
+__global__ void k_finite(int64_t n, const double* __restrict__ a, int32_t* __restrict__ bad) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        if (!isfinite(a[i])) *bad = 1;
+}
+
+// The checks of a model's values (materials may be null): flags[0] = 1 when one fails; flags[1] = 1 when a fixed
+// DOF has a non-zero imposed value.
+__global__ void k_check_model(ModelCheck m, int32_t* __restrict__ flags) {
+    const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    bool bad = false, imposed = false;
+    for (int64_t i = t0; i < 3 * m.n_nodes; i += step) {
+        bad = bad || !isfinite(m.coords[i]) || (m.f && !isfinite(m.f[i]));
+        if (m.imposed && m.fixed[i]) {
+            bad = bad || !isfinite(m.imposed[i]);
+            imposed = imposed || m.imposed[i] != 0.0;
+        }
+    }
+    for (int64_t e = t0; e < m.n_elems; e += step) {
+        const double E = m.young[e], nu = m.poisson[e];
+        bad = bad || !isfinite(E) || !isfinite(nu) || E <= 0.0 || nu <= -1.0 || nu >= 0.5;
+    }
+    for (int64_t k = t0; k < m.n_conn; k += step) bad = bad || m.conn[k] < 0 || m.conn[k] >= m.n_nodes;
+    if (bad) flags[0] = 1;
+    if (imposed) flags[1] = 1;
+}
+
 // sigma = D B u_e at every Gauss point and its von Mises value (solid_stresses,
 // element.rs:270-302; Stress::von_mises, results.rs:24-32). One thread per (element, point).
 template <int NPE>
@@ -681,12 +758,11 @@ void launch_elem_stiffness(int npe, const ElemIn& in, double* ke_up, cudaStream_
         k_elem_stiffness<10><<<(unsigned)((in.ne + Tet<10>::G - 1) / Tet<10>::G), kThreads, 0, st>>>(in, ke_up);
 }
 
-void launch_assemble(const Pattern& pt, int64_t nl, const int64_t* lslot, const int32_t* lrow,
-                     const int64_t* lptr, const uint32_t* contrib, const double* ke_up, double* K,
-                     cudaStream_t st) {
+void launch_assemble(int npe, const Pattern& pt, const AssembleIn& in, const double* ke, double* K, cudaStream_t st) {
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-    k_assemble<<<blocks_for(nl, kThreads, INT32_MAX), kThreads, 0, st>>>(pt, nl, lslot, lrow, lptr,
-                                                                       contrib, ke_up, K);
+    const unsigned grid = blocks_for(pt.nb, kWarps, INT32_MAX);
+    if (npe == 4) k_assemble<4><<<grid, kThreads, 0, st>>>(pt, in, ke, K);
+    else k_assemble<10><<<grid, kThreads, 0, st>>>(pt, in, ke, K);
 }
 
 void launch_factor_level(const Pattern& pt, int32_t r0, int32_t r1, const double* K, double* F,
@@ -729,6 +805,22 @@ void launch_reactions(int64_t n_nodes, const int32_t* nodes, int64_t nnodes, con
     if (nnodes <= 0) return;
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
     k_reactions<<<blocks_for(3 * nnodes, kThreads, INT32_MAX), kThreads, 0, st>>>(nodes, nnodes, fixed, y, f, react);
+}
+
+void launch_orphan_reactions(int64_t n_nodes, const int64_t* inc_ptr, const uint8_t* fixed, const double* f,
+                             double* react, cudaStream_t st) {
+    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+    k_orphan_reactions<<<blocks_for(3 * n_nodes, kThreads, INT32_MAX), kThreads, 0, st>>>(n_nodes, inc_ptr, fixed, f, react);
+}
+
+void launch_finite(int64_t n, const double* a, int32_t* bad, cudaStream_t st) {
+    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+    k_finite<<<blocks_for(n, kThreads, 8 * device_sms()), kThreads, 0, st>>>(n, a, bad);
+}
+
+void launch_check_model(const ModelCheck& m, int32_t* flags, cudaStream_t st) {
+    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+    k_check_model<<<blocks_for(3 * m.n_nodes, kThreads, 8 * device_sms()), kThreads, 0, st>>>(m, flags);
 }
 
 void launch_stresses(int npe, const ElemIn& in, const double* u, double* gauss, double* vm,

@@ -43,11 +43,28 @@ struct Pattern {
     const uint8_t* fixmask;
 };
 
+// What the assembly reads beside the pattern: row -> node, the incidence of the nodes, node -> row.
+struct AssembleIn {
+    const int32_t* perm;
+    const int64_t* inc_ptr;
+    const int32_t *inc, *conn, *inv;
+};
+
+// A model's values as the caller gave them (device copies; imposed and f may be null): launch_check_model.
+struct ModelCheck {
+    int64_t n_nodes, n_elems, n_conn;
+    const double *coords, *young, *poisson, *imposed, *f;
+    const int64_t* conn;
+    const uint8_t* fixed;
+};
+
 // ---- launchers (defined in kernels.cu) -------------------------------------------------------
 void launch_elem_stiffness(int npe, const ElemIn& in, double* ke_up, cudaStream_t st);
-void launch_assemble(const Pattern& pt, int64_t nl, const int64_t* lslot, const int32_t* lrow,
-                     const int64_t* lptr,
-                     const uint32_t* contrib, const double* ke_up, double* K, cudaStream_t st);
+// K (all rows of the pattern) from the element matrices ke_up
+void launch_assemble(int npe, const Pattern& pt, const AssembleIn& in, const double* ke_up, double* K, cudaStream_t st);
+// *bad = 1 when an entry of a is not finite; the checks of a model (flags: [2], zeroed by the caller)
+void launch_finite(int64_t n, const double* a, int32_t* bad, cudaStream_t st);
+void launch_check_model(const ModelCheck& m, int32_t* flags, cudaStream_t st);
 void launch_factor_level(const Pattern& pt, int32_t r0, int32_t r1, const double* K, double* F,
                         double shift, int32_t* fail, cudaStream_t st);
 // b (padded solver numbering, 4 per node) = F_f - K_fc u_c, 0 at fixed DOFs
@@ -64,6 +81,9 @@ void launch_node_gather(int npe, int64_t nnodes, const int32_t* nodes, const int
 void launch_reactions(int64_t n_nodes, const int32_t* nodes, int64_t nnodes,
                       const uint8_t* fixed, const double* y, const double* f, double* react,
                       cudaStream_t st);
+// reactions -f at the fixed DOFs of nodes that no element touches
+void launch_orphan_reactions(int64_t n_nodes, const int64_t* inc_ptr, const uint8_t* fixed, const double* f,
+                             double* react, cudaStream_t st);
 void launch_stresses(int npe, const ElemIn& in, const double* u, double* gauss, double* vm,
                      cudaStream_t st);
 // smoothed nodal stresses [n * 6] and their von Mises values [n] from the Gauss stresses

@@ -557,7 +557,7 @@ int32_t ls_create(const MailleLargeStrainProblem* p, MailleGpuLargeStrain** out)
     ep.rel_tol = p->rel_tol;
     ep.max_iter = p->max_iter;
     ep.precision = p->precision;
-    ep.ordering = MAILLE_ORDER_MULTICOLOR;
+    ep.ordering = MAILLE_ORDER_AUTO;
     ep.device = p->device;
     auto s = std::make_unique<MailleGpuLargeStrain>();
     int32_t status = maille::handle_create(&ep, &s->h, nullptr);

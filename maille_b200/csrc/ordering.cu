@@ -5,8 +5,7 @@
 // (setup.cpp) runs the same algorithms sequentially on nodes; here each one is restated in a
 // form whose result does not depend on the order the GPU's threads run in, so the device and the
 // host produce the same permutation:
-//  * graph: every element emits the (row, column) keys of its kept node pairs; a radix sort and a
-//    unique pass give every node's neighbours by ascending index (the host sorts its lists too);
+//  * graph: every node's neighbours by ascending index (analysis.cu; the host sorts its lists too);
 //  * breadth-first search, level by level in one cooperative launch: a node of the next level
 //    takes as parent its neighbour of the current level that came first (the largest key of an
 //    atomicMax over (search id, complement of the parent's position)), which is the node that
@@ -44,6 +43,7 @@ constexpr int kW = kT / 32;
 constexpr int32_t kVisited = INT_MAX;          // mark of a node an ordering search has placed
 constexpr unsigned int kSpin = 1u << 22;       // polls of one neighbour value before a wait gives up
 constexpr int kMaxColourWords = 32;            // colours below 32 x 32 = 1024
+constexpr int32_t kMaxRowLevels = 65536;       // levels of the RCM ordering
 
 inline unsigned grid_of(int64_t n) {
     const int64_t g = (n + kT - 1) / kT;
@@ -62,33 +62,6 @@ __device__ __forceinline__ int64_t lower_bound_dev(const K* a, int64_t n, K key)
         if (a[mid] < key) lo = mid + 1; else hi = mid;
     }
     return lo;
-}
-
-// (I << 32) | J for every ordered pair of distinct kept nodes of an element; ~0 otherwise
-__global__ void k_graph_keys(int npe, int64_t ne, const int32_t* __restrict__ conn,
-                             const int32_t* __restrict__ kept_of, uint64_t* __restrict__ keys) {
-    const int64_t per = (int64_t)npe * (npe - 1);
-    GRID_STRIDE(t, ne * per) {
-        const int64_t e = t / per;
-        const int rem = (int)(t - e * per);
-        const int a = rem / (npe - 1), bi = rem % (npe - 1), b = bi < a ? bi : bi + 1;
-        const int32_t I = kept_of[conn[e * npe + a]], J = kept_of[conn[e * npe + b]];
-        keys[t] = (I < 0 || J < 0 || I == J) ? ~0ull : (((uint64_t)(uint32_t)I << 32) | (uint64_t)(uint32_t)J);
-    }
-}
-
-// row pointers and degrees of the unique sorted keys (m valid keys, all below nk << 32)
-__global__ void k_graph_csr(const uint64_t* __restrict__ keys, int64_t m, int32_t nk, int64_t* __restrict__ off,
-                            int32_t* __restrict__ deg) {
-    GRID_STRIDE(k, (int64_t)nk + 1) {
-        const int64_t o = lower_bound_dev<uint64_t>(keys, m, (uint64_t)k << 32);
-        off[k] = o;
-        if (k < nk) deg[k] = (int32_t)(lower_bound_dev<uint64_t>(keys, m, (uint64_t)(k + 1) << 32) - o);
-    }
-}
-
-__global__ void k_graph_adj(const uint64_t* __restrict__ keys, int64_t m, int32_t* __restrict__ adj) {
-    GRID_STRIDE(p, m) adj[p] = (int32_t)(keys[p] & 0xFFFFFFFFull);
 }
 
 __device__ __forceinline__ void warp_min_atomic(unsigned long long b, unsigned long long* best) {
@@ -427,21 +400,21 @@ __global__ void k_reverse(int32_t nk, const int32_t* __restrict__ queue, int32_t
     }
 }
 
-__global__ void k_order_keys(int32_t nk, const int32_t* __restrict__ value, const int32_t* __restrict__ rpos,
-                             uint64_t* __restrict__ keys, int32_t* __restrict__ ids) {
+// sort keys (value << pbits) | position of every node; from the last value to the first when top >= 0
+__global__ void k_row_keys(int32_t nk, const int32_t* __restrict__ value, const int32_t* __restrict__ rpos, int pbits,
+                           int32_t top, uint64_t* __restrict__ keys, int32_t* __restrict__ ids) {
     GRID_STRIDE(v, (int64_t)nk) {
-        keys[v] = ((uint64_t)(uint32_t)value[v] << 32) | (uint64_t)(uint32_t)rpos[v];
+        const uint64_t c = (uint64_t)(uint32_t)(top >= 0 ? top - value[v] : value[v]);
+        keys[v] = (c << pbits) | (uint64_t)(uint32_t)rpos[v];
         ids[v] = (int32_t)v;
     }
 }
-
-// visit keys of an iterated-greedy pass: classes from the last to the first, RCM position inside
-__global__ void k_class_keys(int32_t nk, int32_t top, const int32_t* __restrict__ value,
-                             const int32_t* __restrict__ rpos, uint64_t* __restrict__ keys, int32_t* __restrict__ ids) {
-    GRID_STRIDE(v, (int64_t)nk) {
-        keys[v] = ((uint64_t)(uint32_t)(top - value[v]) << 32) | (uint64_t)(uint32_t)rpos[v];
-        ids[v] = (int32_t)v;
-    }
+__global__ void k_level_ptr(int32_t nk, const uint64_t* __restrict__ keys, int pbits, int32_t most,
+                            int32_t* __restrict__ ptr) {
+    GRID_STRIDE(l, (int64_t)most + 1) ptr[l] = (int32_t)lower_bound_dev<uint64_t>(keys, nk, (uint64_t)l << pbits);
+}
+__global__ void k_copy_i32(int64_t n, const int32_t* __restrict__ a, int32_t* __restrict__ b) {
+    GRID_STRIDE(i, n) b[i] = a[i];
 }
 
 // rpos of a visit order given as an array of nodes
@@ -503,80 +476,34 @@ int coop_grid(const void* fn, int threads) {
 
 }  // namespace
 
-void gpu_ordering(int npe, int64_t n_elems, const int32_t* conn, const int32_t* kept_of, int32_t nk,
-                  int ordering, cudaStream_t st, std::vector<int32_t>& order, std::vector<int32_t>& level) {
-    if (nk <= 0) throw CudaFailure{"no kept node to order"};
-    // MAILLE_SETUP_TIMING: wall time of each step (stream synchronised)
-    const bool timing = std::getenv("MAILLE_SETUP_TIMING") != nullptr;
-    double t_mark = now_ms();
-    auto tmark = [&](const char* name, int extra = -1) {
-        if (!timing) return;
-        cudaStreamSynchronize(st);
-        const double t = now_ms();
-        std::fprintf(stderr, "maille ordering %-16s %8.2f ms %d\n", name, t - t_mark, extra);
-        t_mark = t;
-    };
-    // the kept-node graph, neighbours by ascending index
-    const int64_t nkeys = n_elems * npe * (npe - 1);
-    if (nkeys >= INT_MAX || nkeys <= 0) throw CudaFailure{"mesh size outside the device ordering's range"};
-    Temp temp;
-    Buf<int64_t> off((size_t)nk + 1);
-    Buf<int32_t> deg(nk);
-    int64_t m = 0;
-    int32_t* adj = nullptr;
-    {
-        Buf<uint64_t> ka(nkeys), kb(nkeys), uk(nkeys);
-        Buf<int> nsel(1);
-        counted();
-        k_graph_keys<<<grid_of(nkeys), kT, 0, st>>>(npe, n_elems, conn, kept_of, ka.p);
-        CK(cudaGetLastError());
-        cub::DoubleBuffer<uint64_t> db(ka.p, kb.p);
-        size_t bytes = 0;
-        CK(cub::DeviceRadixSort::SortKeys(nullptr, bytes, db, (int)nkeys, 0, 64, st));
-        temp.reserve(bytes);
-        CK(cub::DeviceRadixSort::SortKeys(temp.p, bytes, db, (int)nkeys, 0, 64, st));
-        bytes = 0;
-        CK(cub::DeviceSelect::Unique(nullptr, bytes, db.Current(), uk.p, nsel.p, (int)nkeys, st));
-        temp.reserve(bytes);
-        CK(cub::DeviceSelect::Unique(temp.p, bytes, db.Current(), uk.p, nsel.p, (int)nkeys, st));
-        counted(2);
-        int n = 0;
-        CK(cudaMemcpyAsync(&n, nsel.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        uint64_t last = 0;
-        if (n > 0) CK(cudaMemcpy(&last, uk.p + (n - 1), sizeof(uint64_t), cudaMemcpyDeviceToHost));
-        m = (n > 0 && last == ~0ull) ? n - 1 : n;
-        adj = dalloc<int32_t>((size_t)std::max<int64_t>(1, m));
-        counted(2);
-        k_graph_csr<<<grid_of((int64_t)nk + 1), kT, 0, st>>>(uk.p, m, nk, off.p, deg.p);
-        k_graph_adj<<<grid_of(std::max<int64_t>(1, m)), kT, 0, st>>>(uk.p, m, adj);
-        CK(cudaGetLastError());
-        CK(cudaStreamSynchronize(st));  // the key buffers are freed below
-    }
-    struct AdjFree {
-        int32_t* p;
-        ~AdjFree() { dfree(p); }
-    } adj_free{adj};
-    tmark("graph", (int)m);
+namespace {
 
-    Buf<int32_t> mark(nk), queue(nk), cnt(nk), out(4);
-    Buf<unsigned long long> par(nk), best(1);
+// The visit order of the searches: reverse Cuthill-McKee, or reverse breadth-first (MULTICOLOR_BFS).
+template <typename Mark>
+void search_order(const GraphDev& g, int ordering, cudaStream_t st, int32_t* visit, int32_t* rpos, Mark&& tmark) {
+    const int32_t nk = g.nk;
+    const int64_t* off = g.off;
+    const int32_t *adj = g.adj, *deg = g.deg;
+    Scratch tmp(st);
+    int32_t *mark = tmp.take<int32_t>(nk), *queue = tmp.take<int32_t>(nk), *cnt = tmp.take<int32_t>(nk),
+            *out = tmp.take<int32_t>(4);
+    unsigned long long *par = tmp.take<unsigned long long>(nk), *best = tmp.take<unsigned long long>(1);
     counted();
-    k_fill_i32<<<grid_of(nk), kT, 0, st>>>(nk, 0, mark.p);
-    CK(cudaMemsetAsync(par.p, 0, (size_t)nk * sizeof(unsigned long long), st));
+    k_fill_i32<<<grid_of(nk), kT, 0, st>>>(nk, 0, mark);
+    CK(cudaMemsetAsync(par, 0, (size_t)nk * sizeof(unsigned long long), st));
     const int bfs_grid = coop_grid((const void*)k_bfs, kT);
-    Buf<int32_t> bsum(bfs_grid);
+    int32_t* bsum = tmp.take<int32_t>(bfs_grid);
     int32_t next_id = 1;
     auto bfs = [&](int32_t start, int32_t qbase, bool ordering_search, bool by_degree, int32_t& levels,
                    int32_t& qend, int32_t& last_begin) {
-        BfsArgs a{nk, off.p, adj, deg.p, mark.p, par.p, queue.p, cnt.p, bsum.p, next_id,
-                  ordering_search ? kVisited : next_id, start, qbase, by_degree ? 1 : 0, out.p};
+        BfsArgs a{nk, off, adj, deg, mark, par, queue, cnt, bsum, next_id,
+                  ordering_search ? kVisited : next_id, start, qbase, by_degree ? 1 : 0, out};
         ++next_id;
         void* args[] = {&a};
         counted();
         CK(cudaLaunchCooperativeKernel((const void*)k_bfs, dim3(bfs_grid), dim3(kT), args, 0, st));
         int32_t h[3];
-        CK(cudaMemcpyAsync(h, out.p, 3 * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(h, out, 3 * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         levels = h[0];
         qend = h[1];
@@ -585,10 +512,10 @@ void gpu_ordering(int npe, int64_t n_elems, const int32_t* conn, const int32_t* 
     };
     auto argmin = [&](auto launch) -> int64_t {
         static const unsigned long long none = ~0ull;
-        CK(cudaMemcpyAsync(best.p, &none, sizeof(none), cudaMemcpyHostToDevice, st));
+        CK(cudaMemcpyAsync(best, &none, sizeof(none), cudaMemcpyHostToDevice, st));
         launch();
         unsigned long long h = 0;
-        CK(cudaMemcpyAsync(&h, best.p, sizeof(h), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(&h, best, sizeof(h), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         return h == none ? -1 : (int64_t)(h & 0xFFFFFFFFull);
     };
@@ -598,7 +525,7 @@ void gpu_ordering(int npe, int64_t n_elems, const int32_t* conn, const int32_t* 
     while (ordered < nk) {
         const int64_t seed = argmin([&] {
             counted();
-            k_seed<<<grid_of(nk), kT, 0, st>>>(nk, deg.p, mark.p, best.p);
+            k_seed<<<grid_of(nk), kT, 0, st>>>(nk, deg, mark, best);
         });
         if (seed < 0) throw CudaFailure{"device ordering: no seed while nodes remain"};
         int32_t start = (int32_t)seed, levels = 0, qend = 0, lastb = 0;
@@ -609,11 +536,11 @@ void gpu_ordering(int npe, int64_t n_elems, const int32_t* conn, const int32_t* 
                 const int32_t lb = lastb, le = qend;
                 const int64_t fpos = argmin([&] {
                     counted();
-                    k_far<<<grid_of(le - lb), kT, 0, st>>>(lb, le, queue.p, deg.p, best.p);
+                    k_far<<<grid_of(le - lb), kT, 0, st>>>(lb, le, queue, deg, best);
                 });
                 if (fpos < 0) throw CudaFailure{"device ordering: empty last level"};
                 int32_t far = 0;
-                CK(cudaMemcpy(&far, queue.p + fpos, sizeof(int32_t), cudaMemcpyDeviceToHost));
+                CK(cudaMemcpy(&far, queue + fpos, sizeof(int32_t), cudaMemcpyDeviceToHost));
                 int32_t fd = 0;
                 bfs(far, ordered, false, false, fd, qend, lastb);
                 if (fd <= depth) break;
@@ -625,74 +552,107 @@ void gpu_ordering(int npe, int64_t n_elems, const int32_t* conn, const int32_t* 
         if (qend <= ordered) throw CudaFailure{"device ordering: a search placed no node"};
         ordered = qend;
     }
-    // visit order = the reversed search order; colours (multicolour) or dependency levels (RCM)
-    Buf<int32_t> visit(nk), rpos(nk), value(nk), fail(1);
-    counted(2);
-    k_reverse<<<grid_of(nk), kT, 0, st>>>(nk, queue.p, visit.p, rpos.p);
-    k_fill_i32<<<grid_of(nk), kT, 0, st>>>(nk, -1, value.p);
-    CK(cudaMemsetAsync(fail.p, 0, sizeof(int32_t), st));
+    counted();
+    k_reverse<<<grid_of(nk), kT, 0, st>>>(nk, queue, visit, rpos);
+    CK(cudaGetLastError());
+}
+
+}  // namespace
+
+void gpu_ordering(const GraphDev& g, int ordering, cudaStream_t st, int32_t* order, std::vector<int32_t>& level_ptr) {
+    const int32_t nk = g.nk;
+    const int64_t* off = g.off;
+    const int32_t* adj = g.adj;
+    // MAILLE_SETUP_TIMING: wall time of each step (stream synchronised)
+    const bool timing = std::getenv("MAILLE_SETUP_TIMING") != nullptr;
+    double t_mark = now_ms();
+    auto tmark = [&](const char* name, int extra = -1) {
+        if (!timing) return;
+        cudaStreamSynchronize(st);
+        const double t = now_ms();
+        std::fprintf(stderr, "maille ordering %-16s %8.2f ms %d\n", name, t - t_mark, extra);
+        t_mark = t;
+    };
+    Scratch tmp(st);
+    int32_t *visit = tmp.take<int32_t>(nk), *rpos = tmp.take<int32_t>(nk), *value = tmp.take<int32_t>(nk),
+            *fail = tmp.take<int32_t>(1);
+    counted();
+    k_fill_i32<<<grid_of(nk), kT, 0, st>>>(nk, -1, value);
+    CK(cudaMemsetAsync(fail, 0, sizeof(int32_t), st));
+    if (ordering == kOrderIndex) {
+        counted(2);
+        k_iota<<<grid_of(nk), kT, 0, st>>>(nk, visit);
+        k_iota<<<grid_of(nk), kT, 0, st>>>(nk, rpos);
+    } else {
+        search_order(g, ordering, st, visit, rpos, tmark);
+    }
     // every co-resident warp: a warp's node spends most of its time in dependent loads and polls,
     // so the colouring is paced by the nodes in flight (Tet10 40^3: 19 ms with one block of 8 warps
     // per SM, 6.7 ms with 64 warps per SM; without the pause between polls the full grid took 88 ms)
     const int greedy_grid = coop_grid((const void*)k_greedy, kT);
-    Buf<int32_t> claim(1);
+    int32_t* claim = tmp.take<int32_t>(1);
     auto colour = [&](const int32_t* vis, const int32_t* rp, int mode) {
         int32_t nk_ = nk;
-        const int64_t* o = off.p;
+        const int64_t* o = off;
         const int32_t* ad = adj;
-        int32_t* va = value.p;
-        int32_t* fl = fail.p;
-        int32_t* nx = claim.p;
-        CK(cudaMemsetAsync(claim.p, 0, sizeof(int32_t), st));
+        int32_t* va = value;
+        int32_t* fl = fail;
+        int32_t* nx = claim;
+        CK(cudaMemsetAsync(claim, 0, sizeof(int32_t), st));
         unsigned int p0 = kGreedyPause0, pc = kGreedyPauseCap;
         void* args[] = {&nk_, &o, &ad, &vis, &rp, &va, &mode, &fl, &nx, &p0, &pc};
         counted();
         CK(cudaLaunchCooperativeKernel((const void*)k_greedy, dim3(greedy_grid), dim3(kT), args, 0, st));
     };
-    colour(visit.p, rpos.p, ordering == MAILLE_ORDER_RCM ? 1 : 0);
+    colour(visit, rpos, ordering == MAILLE_ORDER_RCM ? 1 : 0);
     tmark("greedy", greedy_grid);
-    Buf<uint64_t> k0(nk), k1(nk);
-    Buf<int32_t> i0(nk), i1(nk);
-    if (ordering == MAILLE_ORDER_MULTICOLOR_ITERATED) {
-        // iterated greedy: recolour visiting the classes from the last to the first (RCM order
-        // inside a class), twice; the node dependencies now span at most the class count
-        Buf<int32_t> rpos2(nk);
-        for (int pass = 0; pass < 2; ++pass) {
-            std::vector<int32_t> hv(nk);
-            CK(cudaMemcpyAsync(hv.data(), value.p, (size_t)nk * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-            CK(cudaStreamSynchronize(st));
-            const int32_t top = *std::max_element(hv.begin(), hv.end());
-            counted();
-            k_class_keys<<<grid_of(nk), kT, 0, st>>>(nk, top, value.p, rpos.p, k0.p, i0.p);
-            size_t b2 = 0;
-            CK(cub::DeviceRadixSort::SortPairs(nullptr, b2, k0.p, k1.p, i0.p, i1.p, nk, 0, 64, st));
-            temp.reserve(b2);
-            CK(cub::DeviceRadixSort::SortPairs(temp.p, b2, k0.p, k1.p, i0.p, i1.p, nk, 0, 64, st));
-            counted(3);
-            k_inverse<<<grid_of(nk), kT, 0, st>>>(nk, i1.p, rpos2.p);
-            k_fill_i32<<<grid_of(nk), kT, 0, st>>>(nk, -1, value.p);
-            colour(i1.p, rpos2.p, 0);
-        }
-    }
-    int32_t h_fail = 0;
-    CK(cudaMemcpyAsync(&h_fail, fail.p, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    // rows by (colour or level, RCM visit position)
-    counted();
-    k_order_keys<<<grid_of(nk), kT, 0, st>>>(nk, value.p, rpos.p, k0.p, i0.p);
+    uint64_t *k0 = tmp.take<uint64_t>(nk), *k1 = tmp.take<uint64_t>(nk);
+    int32_t *i0 = tmp.take<int32_t>(nk), *i1 = tmp.take<int32_t>(nk), *rpos2 = tmp.take<int32_t>(nk);
+    int pbits = 1;
+    while ((int64_t(1) << pbits) < (int64_t)nk) ++pbits;  // positions
+    const int vbits = ordering == MAILLE_ORDER_RCM ? 31 : 10;  // levels; colours below 1024
     size_t bytes = 0;
-    CK(cub::DeviceRadixSort::SortPairs(nullptr, bytes, k0.p, k1.p, i0.p, i1.p, nk, 0, 64, st));
-    temp.reserve(bytes);
-    CK(cub::DeviceRadixSort::SortPairs(temp.p, bytes, k0.p, k1.p, i0.p, i1.p, nk, 0, 64, st));
-    counted();
-    order.resize(nk);
-    level.resize(nk);
-    CK(cudaMemcpyAsync(order.data(), i1.p, (size_t)nk * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(level.data(), value.p, (size_t)nk * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    CK(cub::DeviceRadixSort::SortPairs(nullptr, bytes, k0, k1, i0, i1, nk, 0, 64, st));
+    unsigned char* sort_mem = tmp.take<unsigned char>(bytes);
+    // sorts by (value, position) into i1
+    auto sort_rows = [&] {
+        CK(cub::DeviceRadixSort::SortPairs(sort_mem, bytes, k0, k1, i0, i1, nk, 0, pbits + vbits, st));
+        counted(3);
+    };
+    // iterated greedy: recolour visiting the classes from the last to the first (the first visit's
+    // position inside a class); the node dependencies then span at most the class count
+    const int passes = ordering == MAILLE_ORDER_MULTICOLOR_ITERATED ? 2 : ordering == kOrderIndex ? 1 : 0;
+    for (int pass = 0; pass < passes; ++pass) {
+        counted(4);
+        k_row_keys<<<grid_of(nk), kT, 0, st>>>(nk, value, rpos, pbits, 32 * kMaxColourWords - 1, k0, i0);
+        sort_rows();
+        k_inverse<<<grid_of(nk), kT, 0, st>>>(nk, i1, rpos2);
+        k_copy_i32<<<grid_of(nk), kT, 0, st>>>(nk, i1, visit);
+        k_fill_i32<<<grid_of(nk), kT, 0, st>>>(nk, -1, value);
+        colour(visit, rpos2, 0);
+    }
+    tmark("iterated greedy", passes);
+    // rows by (colour or level, visit position)
+    counted(3);
+    k_row_keys<<<grid_of(nk), kT, 0, st>>>(nk, value, rpos, pbits, -1, k0, i0);
+    sort_rows();
+    k_copy_i32<<<grid_of(nk), kT, 0, st>>>(nk, i1, order);
+    const int32_t most = ordering == MAILLE_ORDER_RCM ? kMaxRowLevels : 32 * kMaxColourWords;
+    int32_t* ptr = tmp.take<int32_t>(most + 1);
+    k_level_ptr<<<grid_of(most + 1), kT, 0, st>>>(nk, k1, pbits, most, ptr);
+    CK(cudaGetLastError());
+    int32_t h_fail = 0;
+    level_ptr.assign(most + 1, 0);
+    CK(cudaMemcpyAsync(&h_fail, fail, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(level_ptr.data(), ptr, level_ptr.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    tmark("sort and copies", bfs_grid);
+    // drop the levels after the last row; a level beyond `most` leaves the last entry below nk
+    size_t n = level_ptr.size();
+    while (n >= 2 && level_ptr[n - 2] == nk) --n;
+    level_ptr.resize(n);
+    tmark("sort and levels", (int)n - 1);
     if (h_fail) throw CudaFailure{"device ordering: a colouring wait ran out or a node needs 1024 colours or more"};
 }
-
 
 void gpu_narrow(const int64_t* in, int64_t n, int32_t* out, cudaStream_t st) {
     if (n <= 0) return;

@@ -1,12 +1,10 @@
-// setup.cpp -- host-side symbolic analysis: kept nodes, node graph, ordering (RCM or multicolour),
-// level sets, the full 3x3-block CSR pattern and the deterministic element-to-slot scatter map.
+// setup.cpp -- host side of the symbolic analysis: the layout plans of the SpMV and the sweeps, face
+// pressure loads, and the sequential form of the ordering (kept nodes, node graph, RCM or colouring,
+// level sets), which the device's (ordering.cu) is checked against (MAILLE_HOST_ORDERING=1).
 //
 // Reference counterparts: FreeSystem::new numbers the free DOFs, builds the DOF graph
-// (Graph::from_elements, iterative.rs:38-76), orders it by reverse_cuthill_mckee (solve.rs:200-245)
-// and allocates the lower-triangular CSR profile (Csr::zeros, iterative.rs:91-114); each element
-// matrix entry is then added by a binary search (Csr::add, iterative.rs:121-128). Here the same
-// work is done once per mesh topology on nodes instead of scalar DOFs, and the binary searches
-// are replaced by a precomputed scatter map that the GPU reduces in a fixed order.
+// (Graph::from_elements, iterative.rs:38-76) and orders it by reverse_cuthill_mckee
+// (solve.rs:200-245); here on nodes instead of scalar DOFs.
 
 #include <algorithm>
 #include <chrono>
@@ -270,31 +268,10 @@ std::vector<int32_t> iterated_greedy(const NodeGraph& g, const std::vector<int32
     return colour;
 }
 
-// elements touching a fixed DOF, and the nodes with a fixed DOF they contain
-void boundary(Symbolic& s, int64_t n_nodes, int npe, int64_t n_elems, const int64_t* conn,
-              const uint8_t* fixed) {
-    if (!fixed) return;
-    std::vector<uint8_t> bn(n_nodes, 0);
-    for (int64_t e = 0; e < n_elems; ++e) {
-        bool any = false;
-        for (int a = 0; a < npe && !any; ++a) {
-            const int64_t v = conn[e * npe + a];
-            any = fixed[3 * v] || fixed[3 * v + 1] || fixed[3 * v + 2];
-        }
-        if (any) {
-            s.belem.push_back((int32_t)e);
-            for (int a = 0; a < npe; ++a) bn[conn[e * npe + a]] = 1;
-        }
-    }
-    for (int64_t v = 0; v < n_nodes; ++v)
-        if (bn[v]) s.bnodes.push_back((int32_t)v);
-}
-
-}  // namespace
-
+// The input checks, the node incidence, the kept nodes (a node with a free DOF: kept in caller order,
+// kept_of[v] its kept index or -1) and the free DOF count.
 bool analyse_topology(int64_t n_nodes, int npe, int64_t n_elems, const int64_t* conn, const uint8_t* fixed,
-                      Symbolic& s, std::vector<int32_t>& kept, std::vector<int32_t>& kept_of, Error& err,
-                      bool boundary_lists, bool incidence) {
+                      Symbolic& s, std::vector<int32_t>& kept, std::vector<int32_t>& kept_of, Error& err) {
     if (npe != 4 && npe != 10) {
         err = {MAILLE_INVALID_INPUT, "nodes_per_elem must be 4 or 10"};
         return false;
@@ -318,16 +295,13 @@ bool analyse_topology(int64_t n_nodes, int npe, int64_t n_elems, const int64_t* 
     s.n_elems = n_elems;
     s.npe = npe;
     const int32_t N = (int32_t)n_nodes;
-    // node -> (element, local) incidence, sorted by element (the run starts always: the solve
-    // looks up the nodes no element touches there)
+    // node -> (element, local) incidence, sorted by element
     s.inc_ptr.assign(N + 1, 0);
     for (int64_t k = 0; k < n_elems * npe; ++k) s.inc_ptr[conn[k] + 1]++;
     for (int32_t v = 0; v < N; ++v) s.inc_ptr[v + 1] += s.inc_ptr[v];
-    if (incidence) {
-        s.inc.resize(n_elems * npe);
-        std::vector<int64_t> cur(s.inc_ptr.begin(), s.inc_ptr.end() - 1);
-        for (int64_t k = 0; k < n_elems * npe; ++k) s.inc[cur[conn[k]]++] = (int32_t)k;
-    }
+    s.inc.resize(n_elems * npe);
+    std::vector<int64_t> cur(s.inc_ptr.begin(), s.inc_ptr.end() - 1);
+    for (int64_t k = 0; k < n_elems * npe; ++k) s.inc[cur[conn[k]]++] = (int32_t)k;
     // kept nodes (at least one free DOF) in original order
     kept_of.assign(N, -1);
     kept.clear();
@@ -343,10 +317,11 @@ bool analyse_topology(int64_t n_nodes, int npe, int64_t n_elems, const int64_t* 
         err = {MAILLE_INVALID_INPUT, "every DOF is fixed"};
         return false;
     }
-    if (boundary_lists) boundary(s, n_nodes, npe, n_elems, conn, fixed);
     return true;
 }
 
+// The ordering fields of s (nb, perm, inv, fixmask, levels, level_ptr): order[new row] = kept index with
+// rows grouped by level, level[kept index].
 void apply_ordering(const std::vector<int32_t>& kept, const std::vector<int32_t>& order,
                     const std::vector<int32_t>& level, const uint8_t* fixed, Symbolic& s) {
     const int32_t nk = (int32_t)kept.size();
@@ -371,8 +346,11 @@ void apply_ordering(const std::vector<int32_t>& kept, const std::vector<int32_t>
     }
 }
 
+}  // namespace
+
+
 bool analyse(int64_t n_nodes, int npe, int64_t n_elems, const int64_t* conn,
-             const uint8_t* fixed, int ordering, Symbolic& s, Error& err, bool pattern, bool boundary_lists) {
+             const uint8_t* fixed, int ordering, Symbolic& s, Error& err) {
     const double t0 = now_ms();
     const bool stage_timing = std::getenv("MAILLE_SETUP_TIMING") != nullptr;
     double t_stage = now_ms();
@@ -383,8 +361,7 @@ bool analyse(int64_t n_nodes, int npe, int64_t n_elems, const int64_t* conn,
         t_stage = t;
     };
     std::vector<int32_t> kept_of, kept;
-    if (!analyse_topology(n_nodes, npe, n_elems, conn, fixed, s, kept, kept_of, err, boundary_lists && !pattern))
-        return false;
+    if (!analyse_topology(n_nodes, npe, n_elems, conn, fixed, s, kept, kept_of, err)) return false;
     stage("topology");
     const int32_t nk = (int32_t)kept.size();
     NodeGraph g;
@@ -429,11 +406,18 @@ bool analyse(int64_t n_nodes, int npe, int64_t n_elems, const int64_t* conn,
 
     stage("graph");
     // ordering over kept nodes: order[new] = kept index
-    std::vector<int32_t> order = ordering == MAILLE_ORDER_MULTICOLOR_BFS ? reverse_bfs(g) : rcm(g);
+    std::vector<int32_t> order;
+    if (ordering == kOrderIndex) {
+        order.resize(kept.size());
+        std::iota(order.begin(), order.end(), 0);
+    } else {
+        order = ordering == MAILLE_ORDER_MULTICOLOR_BFS ? reverse_bfs(g) : rcm(g);
+    }
     std::vector<int32_t> level;
     if (ordering != MAILLE_ORDER_RCM) {
         level = greedy_colour(g, order);
         if (ordering == MAILLE_ORDER_MULTICOLOR_ITERATED) level = iterated_greedy(g, order, level, kIteratedPasses);
+        if (ordering == kOrderIndex) level = iterated_greedy(g, order, level, 1);
         // rows by colour, visit order inside a colour (a stable counting sort). A row's lower
         // neighbours are exactly its neighbours of smaller colours, and greedy colouring gives a
         // node colour c only when its earlier-visited neighbours hold every colour below c, so the
@@ -465,99 +449,6 @@ bool analyse(int64_t n_nodes, int npe, int64_t n_elems, const int64_t* conn,
     stage("ordering");
     apply_ordering(kept, order, level, fixed, s);
     stage("levels");
-    if (!pattern) {
-        s.ms = now_ms() - t0;
-        return true;
-    }
-    // full block pattern in new numbering (neighbours + the diagonal), columns ascending
-    s.row_ptr.assign(nk + 1, 0);
-    for (int32_t r = 0; r < nk; ++r) {
-        const int32_t k = kept_of[s.perm[r]];
-        s.row_ptr[r + 1] = s.row_ptr[r] + (g.off[k + 1] - g.off[k]) + 1;
-    }
-    s.blocks = s.row_ptr[nk];
-    if (s.blocks >= (int64_t(1) << 31)) {
-        err = {MAILLE_INVALID_INPUT, "pattern too large for 32-bit block positions"};
-        return false;
-    }
-    s.col.resize(s.blocks);
-    s.diag.resize(nk);
-    parallel_for(nk, [&](int64_t r0, int64_t r1) {
-        for (int64_t r = r0; r < r1; ++r) {
-            const int32_t k = kept_of[s.perm[r]];
-            int64_t p = s.row_ptr[r];
-            s.col[p++] = (int32_t)r;
-            for (int64_t q = g.off[k]; q < g.off[k + 1]; ++q) s.col[p++] = s.inv[kept[g.adj[q]]];
-            std::sort(s.col.begin() + s.row_ptr[r], s.col.begin() + s.row_ptr[r + 1]);
-            s.diag[r] = std::lower_bound(s.col.begin() + s.row_ptr[r],
-                                         s.col.begin() + s.row_ptr[r + 1], (int32_t)r) -
-                        s.col.begin();
-        }
-    });
-    g = NodeGraph{};
-    auto find = [&](int32_t i, int32_t j) -> int64_t {
-        auto b = s.col.begin() + s.row_ptr[i], e = s.col.begin() + s.row_ptr[i + 1];
-        auto it = std::lower_bound(b, e, j);
-        return (it != e && *it == j) ? (int64_t)(it - s.col.begin()) : -1;
-    };
-    stage("pattern");
-    s.tpos.resize(s.blocks);
-    parallel_for(nk, [&](int64_t r0, int64_t r1) {
-        for (int64_t r = r0; r < r1; ++r)
-            for (int64_t p = s.row_ptr[r]; p < s.row_ptr[r + 1]; ++p)
-                s.tpos[p] = find(s.col[p], (int32_t)r);
-    });
-
-    stage("transpose");
-    // lower slots (row by row, columns ascending) and the scatter map: for lower slot (I, J) the
-    // element node pairs that couple I and J, in element order. Built row by row from the
-    // node's incident elements (ascending), with a per-thread column -> slot map.
-    const int64_t nl0 = 0;
-    (void)nl0;
-    std::vector<int64_t> lfirst(nk + 1, 0);
-    for (int32_t r = 0; r < nk; ++r) lfirst[r + 1] = lfirst[r] + (s.diag[r] - s.row_ptr[r] + 1);
-    const int64_t nl = lfirst[nk];
-    s.lslot.resize(nl);
-    for (int32_t r = 0; r < nk; ++r)
-        for (int64_t p = s.row_ptr[r]; p <= s.diag[r]; ++p) s.lslot[lfirst[r] + (p - s.row_ptr[r])] = p;
-    const int np = node_pairs(npe);
-    auto pair_index = [npe](int a, int b) { return a * npe - a * (a - 1) / 2 + (b - a); };
-    // visit(r, fn): fn(local slot, contribution) for every contribution of row r, element order
-    auto visit_row = [&](int32_t r, std::vector<int32_t>& slotmap, auto&& fn) {
-        for (int64_t p = s.row_ptr[r]; p <= s.diag[r]; ++p) slotmap[s.col[p]] = (int32_t)(p - s.row_ptr[r]);
-        const int32_t v = s.perm[r];
-        for (int64_t q = s.inc_ptr[v]; q < s.inc_ptr[v + 1]; ++q) {
-            const int64_t e = s.inc[q] / npe;
-            const int a = (int)(s.inc[q] - e * npe);
-            for (int b = 0; b < npe; ++b) {
-                const int32_t J = s.inv[conn[e * npe + b]];
-                if (J < 0 || J > r) continue;
-                const uint32_t k = (uint32_t)(e * np + (a <= b ? pair_index(a, b) : pair_index(b, a)));
-                fn(slotmap[J], k | (a <= b ? 0u : 0x80000000u));
-            }
-        }
-    };
-    s.lptr.assign(nl + 1, 0);
-    parallel_for(nk, [&](int64_t r0, int64_t r1) {
-        std::vector<int32_t> slotmap(nk, -1);
-        for (int64_t r = r0; r < r1; ++r)
-            visit_row((int32_t)r, slotmap, [&](int32_t ls, uint32_t) { s.lptr[lfirst[r] + ls + 1]++; });
-    });
-    for (int64_t l = 0; l < nl; ++l) s.lptr[l + 1] += s.lptr[l];
-    s.contrib.resize(s.lptr[nl]);
-    parallel_for(nk, [&](int64_t r0, int64_t r1) {
-        std::vector<int32_t> slotmap(nk, -1);
-        std::vector<int64_t> cur;
-        for (int64_t r = r0; r < r1; ++r) {
-            cur.assign(s.lptr.begin() + lfirst[r], s.lptr.begin() + lfirst[r + 1]);
-            visit_row((int32_t)r, slotmap, [&](int32_t ls, uint32_t c) { s.contrib[cur[ls]++] = c; });
-        }
-    });
-    s.nl = nl;
-
-    stage("scatter map");
-    if (boundary_lists) boundary(s, n_nodes, npe, n_elems, conn, fixed);
-    stage("boundary");
     s.ms = now_ms() - t0;
     return true;
 }
@@ -650,7 +541,7 @@ void build_bsell(const Symbolic& s, SellKind kind, int rows, int sub, const std:
     out = BSellHost{};
     out.rows = rows;
     out.sub = sub;
-    const int slots = out.slots(), per_step = 4 * sub;
+    const int per_step = 4 * sub;
     auto start = [&](int32_t i) { return kind == SELL_UPPER ? s.diag[i] + 1 : s.row_ptr[i]; };
     auto end = [&](int32_t i) { return kind == SELL_LOWER ? s.diag[i] : s.row_ptr[i + 1]; };
     auto emit = [&](std::vector<int32_t>& rs) {
@@ -666,19 +557,7 @@ void build_bsell(const Symbolic& s, SellKind kind, int rows, int sub, const std:
             const int64_t g0 = out.off.back();
             out.off.push_back(g0 + steps);
             out.inst.push_back(group[rs[c0]]);
-            out.col.resize((size_t)(g0 + steps) * slots, s.nb);
-            out.src.resize((size_t)(g0 + steps) * slots, -1);
             for (int r = 0; r < rows; ++r) out.rowid.push_back(c0 + r < c1 ? rs[c0 + r] : -1);
-            for (size_t k = c0; k < c1; ++k) {
-                const int32_t i = rs[k];
-                const int r = (int)(k - c0);
-                for (int64_t p = start(i), b = 0; p < end(i); ++p, ++b) {
-                    const int64_t t = b / per_step, rem = b % per_step;
-                    const size_t slot = (size_t)(g0 + t) * slots + 4 * (r * sub + rem / 4) + rem % 4;
-                    out.col[slot] = s.col[p];
-                    out.src[slot] = (int32_t)p;
-                }
-            }
         }
     };
     // rows bucketed by group, keeping row order inside a group

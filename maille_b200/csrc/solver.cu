@@ -54,9 +54,8 @@ MailleGpuHandle::~MailleGpuHandle() {
                      t[0] * 1e-6, t[1] * 1e-6, t[2] * 1e-6, t[3] * 1e-6, t[4] * 1e-6, t[5] * 1e-6,
                      t[6], persist_grid);
     }
-    void* bufs[] = {coords, young, poisson, imposed, f, f0, conn, fixed, perm, inv, col, lrow, fixmask,
-                    row_ptr, diag, tpos, lslot, lptr, contrib, inc_ptr, inc, belem, bnodes,
-                    elem_slot, ke, K, F, Ks64, Ls64, Us64, D64, Ks32, Ls32, Us32, D32, b64, x64,
+    void* bufs[] = {coords, young, poisson, imposed, f, f0, conn, fixed, perm, inv, col, fixmask,
+                    row_ptr, diag, tpos, inc_ptr, inc, bd.belem, bd.bnodes, bd.elem_slot, ke, K, F, Ks64, Ls64, Us64, D64, Ks32, Ls32, Us32, D32, b64, x64,
                     r64, z64, p64, ap64, x32, r32, z32, p32, ap32, u_full, y_full, ye, gauss, vm,
                     react, lambda_full, grad, node_stress, node_vm, scal, partials, timing, claim, dsum, dticket, dfail};
     // one device synchronisation for all of them (a free per buffer waited for the device each time)
@@ -204,7 +203,8 @@ int32_t fail(const Error& e) {
     return e.status;
 }
 
-bool check_problem(const MailleElasticProblem* p, Error& err) {
+// The problem's pointers and options.
+bool check_arguments(const MailleElasticProblem* p, Error& err) {
     if (!p) {
         err = {MAILLE_INVALID_INPUT, "null problem"};
         return false;
@@ -221,6 +221,24 @@ bool check_problem(const MailleElasticProblem* p, Error& err) {
         err = {MAILLE_INVALID_INPUT, "unknown ordering"};
         return false;
     }
+    if (p->nodes_per_elem != 4 && p->nodes_per_elem != 10) {
+        err = {MAILLE_INVALID_INPUT, "nodes_per_elem must be 4 or 10"};
+        return false;
+    }
+    if (p->n_nodes <= 0 || p->n_elems <= 0) {
+        err = {MAILLE_INVALID_INPUT, "empty mesh"};
+        return false;
+    }
+    if (p->n_nodes >= (int64_t(1) << 30) || p->n_elems * node_pairs(p->nodes_per_elem) >= (int64_t(1) << 31)) {
+        err = {MAILLE_INVALID_INPUT, "mesh too large for 32-bit node and element-pair indices"};
+        return false;
+    }
+    return true;
+}
+
+// The problem's values, entry by entry, for the message of the first bad one: the device checks them all
+// at once (launch_check_model) and this runs when it found one, or when there is no device.
+bool check_values(const MailleElasticProblem* p, Error& err) {
     for (int64_t k = 0; k < 3 * p->n_nodes; ++k)
         if (!std::isfinite(p->coords[k])) {
             err = {MAILLE_INVALID_INPUT, "non-finite coordinate at node " + std::to_string(k / 3)};
@@ -244,6 +262,13 @@ bool check_problem(const MailleElasticProblem* p, Error& err) {
                 err = {MAILLE_INVALID_INPUT, "non-finite imposed value at DOF " + std::to_string(k)};
                 return false;
             }
+    const int64_t nc = p->n_elems * p->nodes_per_elem;
+    for (int64_t k = 0; k < nc; ++k)
+        if (p->conn[k] < 0 || p->conn[k] >= p->n_nodes) {
+            err = {MAILLE_INVALID_INPUT, "element " + std::to_string(k / p->nodes_per_elem) + " refers to unknown node " +
+                                             std::to_string(p->conn[k])};
+            return false;
+        }
     return true;
 }
 
@@ -253,10 +278,9 @@ void build_rhs(MailleGpuHandle* h) {
     if (h->any_imposed) {
         // u_c: imposed values at fixed DOFs, 0 elsewhere; coupling = K u_c on boundary nodes
         CK(cudaMemsetAsync(h->y_full, 0, 3 * h->n_nodes * sizeof(double), h->st));
-        launch_elem_apply(h->npe, (int64_t)h->sym.belem.size(), h->belem, h->conn, h->ke,
-                          h->imposed, h->ye, h->st);
-        launch_node_gather(h->npe, (int64_t)h->sym.bnodes.size(), h->bnodes, h->inc_ptr, h->inc,
-                           h->elem_slot, h->ye, h->y_full, h->st);
+        launch_elem_apply(h->npe, h->bd.nbelem, h->bd.belem, h->conn, h->ke, h->imposed, h->ye, h->st);
+        launch_node_gather(h->npe, h->bd.nbnodes, h->bd.bnodes, h->inc_ptr, h->inc, h->bd.elem_slot, h->ye, h->y_full,
+                           h->st);
         coupling = h->y_full;
     }
     launch_build_rhs(h->sym.nb, h->perm, h->fixmask, h->f_cur, coupling, h->b64, h->st);
@@ -300,8 +324,7 @@ int32_t numeric_phase(MailleGpuHandle* h, Error& err) {
 int32_t assemble_factor(MailleGpuHandle* h, Error& err) {
     const Symbolic& s = h->sym;
     cudaStream_t st = h->st;
-    launch_assemble(h->pattern(), s.nl, h->lslot, h->lrow, h->lptr, h->contrib,
-                    h->ke, h->K, st);
+    launch_assemble(h->npe, h->pattern(), h->assembly(), h->ke, h->K, st);
     launch_sell_fill<double>(h->sk.h.steps(), h->sk.src, h->K, h->Ks64, st);
     CK(cudaGetLastError());
     CK(cudaEventRecord(h->ev[2], st));
@@ -338,7 +361,18 @@ int32_t create_impl(const MailleElasticProblem* p, MailleGpuHandle** out, Maille
     Error err{MAILLE_OK, ""};
     if (!out) return fail({MAILLE_INVALID_INPUT, "null handle pointer"});
     *out = nullptr;
-    if (!check_problem(p, err)) return fail(err);
+    if (!check_arguments(p, err)) return fail(err);
+    {
+        int ndev = 0;
+        const bool none = cudaGetDeviceCount(&ndev) != cudaSuccess;
+        if (none) cudaGetLastError();
+        if (none || p->device < 0 || p->device >= ndev) {
+            if (!check_values(p, err)) return fail(err);
+            if (p->fixed && std::all_of(p->fixed, p->fixed + 3 * p->n_nodes, [](uint8_t f) { return f != 0; }))
+                return fail({MAILLE_INVALID_INPUT, "every DOF is fixed"});
+            return fail({MAILLE_CUDA_ERROR, "no CUDA device " + std::to_string(p->device)});
+        }
+    }
     auto h = std::make_unique<MailleGpuHandle>();
     h->device = p->device;
     h->npe = p->nodes_per_elem;
@@ -350,70 +384,29 @@ int32_t create_impl(const MailleElasticProblem* p, MailleGpuHandle** out, Maille
     if (const char* e = std::getenv("MAILLE_RELIABLE_DELTA")) h->delta = std::atof(e);
     const int64_t n3 = 3 * p->n_nodes;
     h->h_fixed.assign(n3, 0);
+    int64_t nfixed = 0;
     if (p->fixed)
-        for (int64_t k = 0; k < n3; ++k) h->h_fixed[k] = p->fixed[k] ? 1 : 0;
-    // the element kernels index with the connectivity: check it before any device work (a
-    // min / max pass; the offending entry is looked for only when there is one)
-    if (p->nodes_per_elem != 4 && p->nodes_per_elem != 10)
-        return fail({MAILLE_INVALID_INPUT, "nodes_per_elem must be 4 or 10"});
-    {
-        const int64_t nc = p->n_elems * p->nodes_per_elem;
-        int64_t lo = INT64_MAX, hi = INT64_MIN;
-        for (int64_t k = 0; k < nc; ++k) {
-            lo = std::min(lo, p->conn[k]);
-            hi = std::max(hi, p->conn[k]);
+        for (int64_t k = 0; k < n3; ++k) {
+            h->h_fixed[k] = p->fixed[k] ? 1 : 0;
+            nfixed += h->h_fixed[k];
         }
-        if (nc > 0 && (lo < 0 || hi >= p->n_nodes))
-            for (int64_t k = 0; k < nc; ++k)
-                if (p->conn[k] < 0 || p->conn[k] >= p->n_nodes)
-                    return fail({MAILLE_INVALID_INPUT, "element " + std::to_string(k / p->nodes_per_elem) +
-                                                           " refers to unknown node " + std::to_string(p->conn[k])});
-    }
-    if (std::all_of(h->h_fixed.begin(), h->h_fixed.end(), [](uint8_t f) { return f != 0; }))
+    if (nfixed == n3) {
+        if (!check_values(p, err)) return fail(err);
         return fail({MAILLE_INVALID_INPUT, "every DOF is fixed"});
-    if (p->n_nodes >= (int64_t(1) << 30) || p->n_elems * node_pairs(p->nodes_per_elem) >= (int64_t(1) << 31))
-        return fail({MAILLE_INVALID_INPUT, "mesh too large for 32-bit node and element-pair indices"});
-    // The ordering and the node incidence run on the device (ordering.cu) once the inputs are
-    // there; the host keeps the part that does not depend on them (kept nodes, boundary lists, the
-    // host copies of the loads and the imposed-value flag) on a thread of its own meanwhile.
-    // MAILLE_HOST_ORDERING=1 orders on that host thread instead (the same permutation: the same
-    // algorithms on the same graph). The pattern and scatter map follow on the device
-    // (analysis.cu).
+    }
+    // The analysis runs on the device: kept nodes, their graph, the ordering and levels (ordering.cu), the
+    // pattern and the boundary lists (analysis.cu). MAILLE_HOST_ORDERING=1 orders on the host instead (the
+    // same permutation: the same algorithms on the same graph).
     const bool host_ordering = env_int("MAILLE_HOST_ORDERING", 0) != 0;
-    // AUTO: MULTICOLOR_ITERATED (Tet10 40^3 mixed: 15 levels against 18, 1.6 % more iterations,
-    // the step 4 % shorter than MULTICOLOR)
-    const int ordering = p->ordering == MAILLE_ORDER_AUTO ? MAILLE_ORDER_MULTICOLOR_ITERATED : p->ordering;
-    std::vector<int32_t> kept, kept_of;
+    const int ordering = p->ordering == MAILLE_ORDER_AUTO ? kOrderIndex : p->ordering;
     std::vector<double> box(6, 0.0);  // of the nodes, for the coarse grid
-    const double t_setup0 = now_ms();
-    double t_setup1 = t_setup0;
-    bool analysed = false;
-    std::thread analysis([&] {
-        if (host_ordering)
-            analysed = analyse(p->n_nodes, p->nodes_per_elem, p->n_elems, p->conn, h->h_fixed.data(), ordering,
-                               h->sym, err, /*pattern=*/false);
-        else
-            analysed = analyse_topology(p->n_nodes, p->nodes_per_elem, p->n_elems, p->conn, h->h_fixed.data(),
-                                        h->sym, kept, kept_of, err, /*boundary_lists=*/true,
-                                        /*incidence=*/false);
-        if (p->imposed)
-            for (int64_t k = 0; k < n3; ++k)
-                if (h->h_fixed[k] && p->imposed[k] != 0.0) {
-                    h->any_imposed = true;
-                    break;
-                }
-        h->h_f.assign(n3, 0.0);
-        if (p->f) std::memcpy(h->h_f.data(), p->f, n3 * sizeof(double));
-        h->h_f0 = h->h_f;
-        coarse_box(p->coords, 0, p->n_nodes, box.data());
-        t_setup1 = now_ms();
-    });
+    std::thread boxer([&] { coarse_box(p->coords, 0, p->n_nodes, box.data()); });
     struct Joiner {
         std::thread& t;
         ~Joiner() {
             if (t.joinable()) t.join();
         }
-    } joiner{analysis};
+    } joiner{boxer};
     // MAILLE_SETUP_TIMING: wall time of the device-side set-up steps (stream synchronised)
     const bool stage_timing = std::getenv("MAILLE_SETUP_TIMING") != nullptr;
     double t_mark = now_ms();
@@ -425,10 +418,6 @@ int32_t create_impl(const MailleElasticProblem* p, MailleGpuHandle** out, Maille
         t_mark = t;
     };
     try {
-        int ndev = 0;
-        CK(cudaGetDeviceCount(&ndev));
-        if (p->device < 0 || p->device >= ndev)
-            return fail({MAILLE_CUDA_ERROR, "no CUDA device " + std::to_string(p->device)});
         CK(cudaSetDevice(p->device));
         CK(cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking));
         for (auto& e : h->ev) CK(cudaEventCreate(&e));
@@ -452,71 +441,74 @@ int32_t create_impl(const MailleElasticProblem* p, MailleGpuHandle** out, Maille
         h->poisson = dupload(p->poisson, p->n_elems, st);
         h->fixed = dupload(h->h_fixed.data(), n3, st);
         h->imposed = dupload(p->imposed, n3, st);
+        h->f0 = dupload(p->f, n3, st);
+        h->dfail = dalloc<int32_t>(2);
+        CK(cudaMemsetAsync(h->dfail, 0, 2 * sizeof(int32_t), st));
+        launch_check_model(ModelCheck{p->n_nodes, p->n_elems, nconn, h->coords, h->young, h->poisson,
+                                      p->imposed ? h->imposed : nullptr, p->f ? h->f0 : nullptr,
+                                      static_cast<const int64_t*>(conn64.p), h->fixed},
+                           h->dfail, st);
         if (p->imposed)
             gpu_zero_free(n3, h->fixed, h->imposed, st);
         else
             CK(cudaMemsetAsync(h->imposed, 0, n3 * sizeof(double), st));
-        h->f0 = dupload(p->f, n3, st);
         if (!p->f) CK(cudaMemsetAsync(h->f0, 0, n3 * sizeof(double), st));
+        int32_t flags[2] = {0, 0};
+        CK(cudaMemcpyAsync(flags, h->dfail, sizeof(flags), cudaMemcpyDeviceToHost, st));
+        CK(cudaEventRecord(h->ev[8], st));  // inputs copied
+        CK(cudaStreamSynchronize(st));
+        if (flags[0] && !check_values(p, err)) return fail(err);  // before a kernel indexes with the connectivity
+        h->any_imposed = flags[1] != 0;
         h->f = dalloc<double>(n3);
         h->f_cur = h->f0;
         h->inc_ptr = dalloc<int64_t>(p->n_nodes + 1);
         h->inc = dalloc<int32_t>(nconn);
         h->ke = dalloc<double>((size_t)p->n_elems * np * 9);
-        CK(cudaEventRecord(h->ev[8], st));  // inputs copied
         {
             ElemIn in{h->n_elems, h->coords, h->conn, h->young, h->poisson};
             launch_elem_stiffness(h->npe, in, h->ke, st);
         }
         CK(cudaEventRecord(h->ev[9], st));  // element matrices integrated
         const double t_wait0 = now_ms();
+        tmark("element");
         gpu_incidence(h->conn, nconn, p->n_nodes, st, h->inc_ptr, h->inc);
-        if (host_ordering) {
-            analysis.join();
-            if (!analysed) return fail(err);
-        } else {
-            // kept nodes: at least one free DOF (the same rule as analyse_topology)
-            std::vector<int32_t> h_kept_of(p->n_nodes, -1), h_kept;
-            for (int64_t v = 0; v < p->n_nodes; ++v)
-                if (!(h->h_fixed[3 * v] && h->h_fixed[3 * v + 1] && h->h_fixed[3 * v + 2])) {
-                    h_kept_of[v] = (int32_t)h_kept.size();
-                    h_kept.push_back((int32_t)v);
-                }
-            int32_t* d_kept_of = dupload(h_kept_of.data(), h_kept_of.size(), st);
-            std::vector<int32_t> order, level;
-            try {
-                gpu_ordering(h->npe, h->n_elems, h->conn, d_kept_of, (int32_t)h_kept.size(), ordering, st, order,
-                             level);
-            } catch (...) {
-                dfree(d_kept_of);
-                throw;
-            }
-            dfree(d_kept_of);
-            analysis.join();
-            if (!analysed) return fail(err);
-            apply_ordering(h_kept, order, level, h->h_fixed.data(), h->sym);
-        }
-        const double t_wait1 = now_ms();
-        CK(cudaEventRecord(h->ev[10], st));  // symbolic: the ordering is known
-        if (h->sym.levels >= kMaxLevels) return fail({MAILLE_INVALID_INPUT, "too many IC(0) levels"});
-        // symbolic
-        h->perm = dupload(s.perm.data(), s.perm.size(), st);
-        h->inv = dupload(s.inv.data(), s.inv.size(), st);
-        h->fixmask = dupload(s.fixmask.data(), s.fixmask.size(), st);
-        tmark("inputs");
+        double t_wait1 = t_wait0;
         {
+            Scratch tmp(st);
+            GraphDev graph;
+            int32_t *kept_of = tmp.take<int32_t>(p->n_nodes), *kept = tmp.take<int32_t>(p->n_nodes);
+            const int32_t nk = gpu_keep(3, p->n_nodes, h->fixed, st, kept_of, kept);
+            int32_t *order = tmp.take<int32_t>(nk), *rank = tmp.take<int32_t>(nk);
+            gpu_graph(h->npe, h->n_elems, h->conn, h->inc_ptr, h->inc, kept_of, kept, nk, st, graph);
+            tmark("graph");
+            h->perm = dalloc<int32_t>(nk);
+            h->inv = dalloc<int32_t>(p->n_nodes);
+            h->fixmask = dalloc<uint8_t>(nk);
+            if (host_ordering) {
+                if (!analyse(p->n_nodes, p->nodes_per_elem, p->n_elems, p->conn, h->h_fixed.data(), ordering, h->sym, err))
+                    return fail(err);
+                CK(cudaMemcpyAsync(h->perm, s.perm.data(), nk * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+                gpu_ranks(nk, h->perm, kept_of, st, order, rank);
+            } else {
+                gpu_ordering(graph, ordering, st, order, h->sym.level_ptr);
+            }
+            gpu_rows(3, nk, p->n_nodes, order, kept, kept_of, h->fixed, st, h->perm, h->inv, rank, h->fixmask);
+            h->sym.nb = nk;
+            h->sym.levels = (int32_t)h->sym.level_ptr.size() - 1;
+            h->sym.free_dofs = n3 - nfixed;
+            t_wait1 = now_ms();
+            CK(cudaEventRecord(h->ev[10], st));  // symbolic: the ordering is known
+            if (h->sym.levels >= kMaxLevels) return fail({MAILLE_INVALID_INPUT, "too many IC(0) levels"});
+            tmark("ordering");
             PatternDev pt;
-            gpu_pattern(h->npe, h->n_elems, h->conn, h->inv, s.nb, st, pt, h->sym.row_ptr, h->sym.diag);
+            gpu_pattern(graph, order, rank, st, pt, h->sym.row_ptr, h->sym.diag);
             h->row_ptr = pt.row_ptr;
             h->col = pt.col;
             h->diag = pt.diag;
             h->tpos = pt.tpos;
-            h->lslot = pt.lslot;
-            h->lrow = pt.lrow;
-            h->lptr = pt.lptr;
-            h->contrib = pt.contrib;
             h->sym.blocks = pt.blocks;
-            h->sym.nl = pt.nl;
+            gpu_boundary(h->npe, h->n_elems, h->conn, p->n_nodes, h->fixed, h->inc_ptr, st, h->bd);
+            tmp.release();
             tmark("pattern");
             // layout plans from the row lengths (host, side by side), slot fills on the device
             const int lk = env_int("MAILLE_LPR_K", 0);
@@ -534,6 +526,7 @@ int32_t create_impl(const MailleElasticProblem* p, MailleGpuHandle** out, Maille
         }
         // the coarse correction, with the multicolour orderings (RCM stands for the reference's own
         // iteration counts). MAILLE_COARSE=0: IC(0) alone (a measurement knob)
+        boxer.join();
         if (ordering != MAILLE_ORDER_RCM && env_int("MAILLE_COARSE", 1) != 0)
             h->coarse.plan(3, is_mixed(h.get()), s.nb, s.blocks, h->coords, h->perm, h->fixmask, h->row_ptr, h->col,
                            nullptr, box, {(int64_t)s.nb}, st);
@@ -543,11 +536,6 @@ int32_t create_impl(const MailleElasticProblem* p, MailleGpuHandle** out, Maille
         if (h->coarse.active() && !std::getenv("MAILLE_RELIABLE_DELTA")) h->delta = kCoarseDelta;
         tmark("coarse plan");
         CK(cudaEventRecord(h->ev[11], st));  // pattern and layouts on the device
-        h->belem = dupload(s.belem.data(), s.belem.size(), st);
-        h->bnodes = dupload(s.bnodes.data(), s.bnodes.size(), st);
-        std::vector<int32_t> slot(p->n_elems, -1);
-        for (size_t k = 0; k < s.belem.size(); ++k) slot[s.belem[k]] = (int32_t)k;
-        h->elem_slot = dupload(slot.data(), slot.size(), st);
         // numeric buffers
         const int64_t n4 = 4 * ((int64_t)s.nb + 1);  // + the dummy node that padding points at
         h->K = dalloc<double>((size_t)s.blocks * 9);
@@ -584,7 +572,7 @@ int32_t create_impl(const MailleElasticProblem* p, MailleGpuHandle** out, Maille
         h->u_full = dalloc<double>(n3);
         h->y_full = dalloc<double>(n3);
         h->react = dalloc<double>(n3);
-        h->ye = dalloc<double>(std::max<size_t>(1, s.belem.size()) * 3 * h->npe);
+        h->ye = dalloc<double>(std::max<int64_t>(1, h->bd.nbelem) * 3 * h->npe);
         h->scal = dalloc<PcgScalars>(1);
         CK(cudaMemsetAsync(h->scal, 0, sizeof(PcgScalars), st));
         h->h_scal = static_cast<PcgScalars*>(pinned_slot_alloc(sizeof(PcgScalars)));
@@ -592,7 +580,6 @@ int32_t create_impl(const MailleElasticProblem* p, MailleGpuHandle** out, Maille
         h->dsum = dalloc<double>(4);
         h->dticket = dalloc<unsigned int>(1);
         CK(cudaMemsetAsync(h->dticket, 0, sizeof(unsigned int), st));
-        h->dfail = dalloc<int32_t>(1);
         h->spmv_grid = grid_for_slices(h->sk.h.nslices());
         h->claim = dalloc<int32_t>(4);
         CK(cudaMemsetAsync(h->claim, 0, 4 * sizeof(int32_t), st));
@@ -622,7 +609,7 @@ int32_t create_impl(const MailleElasticProblem* p, MailleGpuHandle** out, Maille
         tmark("numeric");
         CK(cudaStreamSynchronize(st));
         if (res) {
-            res->ms_setup = t_setup1 - t_setup0;
+            res->ms_setup = 0.0;
             res->ms_upload = elapsed(h->ev[0], h->ev[8]);
             res->ms_element = elapsed(h->ev[8], h->ev[9]);
             res->ms_ordering = t_wait1 - t_wait0;
@@ -649,6 +636,16 @@ const char* status_message(int32_t status, int32_t iters, double rel) {
     return m.c_str();
 }
 
+// Whether the n device entries of a are all finite (waits for the stream).
+bool all_finite(MailleGpuHandle* h, const double* a, int64_t n) {
+    CK(cudaMemsetAsync(h->dfail, 0, sizeof(int32_t), h->st));
+    launch_finite(n, a, h->dfail, h->st);
+    int32_t bad = 0;
+    CK(cudaMemcpyAsync(&bad, h->dfail, sizeof(bad), cudaMemcpyDeviceToHost, h->st));
+    CK(cudaStreamSynchronize(h->st));
+    return bad == 0;
+}
+
 int32_t solve_impl(MailleGpuHandle* h, const double* f, MailleElasticResult* res) {
     NvtxRange nvtx("maille solve: PCG, reactions, stresses");
     if (!h) return fail({MAILLE_INVALID_INPUT, "null handle"});
@@ -658,13 +655,10 @@ int32_t solve_impl(MailleGpuHandle* h, const double* f, MailleElasticResult* res
         const Symbolic& s = h->sym;
         const int64_t n3 = 3 * h->n_nodes;
         if (f) {
-            for (int64_t k = 0; k < n3; ++k)
-                if (!std::isfinite(f[k])) return fail({MAILLE_INVALID_INPUT, "non-finite load"});
-            std::memcpy(h->h_f.data(), f, n3 * sizeof(double));
             CK(cudaMemcpyAsync(h->f, f, n3 * sizeof(double), cudaMemcpyHostToDevice, st));
+            if (!all_finite(h, h->f, n3)) return fail({MAILLE_INVALID_INPUT, "non-finite load"});
             h->f_cur = h->f;
         } else {
-            h->h_f = h->h_f0;
             h->f_cur = h->f0;
         }
         CK(cudaEventRecord(h->ev[4], st));
@@ -691,15 +685,14 @@ int32_t solve_impl(MailleGpuHandle* h, const double* f, MailleElasticResult* res
         // u in caller numbering, reactions, stresses
         launch_gather_u(h->n_nodes, h->inv, h->fixed, h->imposed, h->x64, h->u_full, st);
         CK(cudaMemsetAsync(h->react, 0, n3 * sizeof(double), st));
-        if (!s.belem.empty()) {
+        if (h->bd.nbelem) {
             CK(cudaMemsetAsync(h->y_full, 0, n3 * sizeof(double), st));
-            launch_elem_apply(h->npe, (int64_t)s.belem.size(), h->belem, h->conn, h->ke, h->u_full,
-                              h->ye, st);
-            launch_node_gather(h->npe, (int64_t)s.bnodes.size(), h->bnodes, h->inc_ptr, h->inc,
-                               h->elem_slot, h->ye, h->y_full, st);
-            launch_reactions(h->n_nodes, h->bnodes, (int64_t)s.bnodes.size(), h->fixed, h->y_full,
-                             h->f_cur, h->react, st);
+            launch_elem_apply(h->npe, h->bd.nbelem, h->bd.belem, h->conn, h->ke, h->u_full, h->ye, st);
+            launch_node_gather(h->npe, h->bd.nbnodes, h->bd.bnodes, h->inc_ptr, h->inc, h->bd.elem_slot, h->ye, h->y_full,
+                               st);
+            launch_reactions(h->n_nodes, h->bd.bnodes, h->bd.nbnodes, h->fixed, h->y_full, h->f_cur, h->react, st);
         }
+        if (h->bd.orphans) launch_orphan_reactions(h->n_nodes, h->inc_ptr, h->fixed, h->f_cur, h->react, st);
         const int ng = gauss_points(h->npe);
         if (!h->gauss) {
             h->gauss = dalloc<double>((size_t)h->n_elems * ng * 9);
@@ -726,13 +719,6 @@ int32_t solve_impl(MailleGpuHandle* h, const double* f, MailleElasticResult* res
             res->ms_solve = elapsed(h->ev[4], h->ev[5]);
             res->ms_post = elapsed(h->ev[5], h->ev[6]);
             res->ms_download = elapsed(h->ev[6], h->ev[7]);
-            // a fixed DOF that no element touches: K u = 0 there (product skips it)
-            if (res->reactions && s.belem.size() < (size_t)h->n_elems) {
-                for (int64_t v = 0; v < h->n_nodes; ++v)
-                    if (s.inc_ptr[v] == s.inc_ptr[v + 1])
-                        for (int c = 0; c < 3; ++c)
-                            if (h->h_fixed[3 * v + c]) res->reactions[3 * v + c] = -h->h_f[3 * v + c];
-            }
         }
         h->solved = true;
     } catch (const CudaFailure& e) {
@@ -754,7 +740,6 @@ int32_t solve_device_impl(MailleGpuHandle* h, const double* f_dev, double* u_dev
             CK(cudaMemcpyAsync(h->f, f_dev, n3 * sizeof(double), cudaMemcpyDeviceToDevice, st));
             h->f_cur = h->f;
         } else {
-            h->h_f = h->h_f0;
             h->f_cur = h->f0;
         }
         build_rhs(h);
@@ -783,10 +768,9 @@ int32_t backward_impl(MailleGpuHandle* h, const double* dJdu, double* dJdE, doub
         CK(cudaSetDevice(h->device));
         cudaStream_t st = h->st;
         const int64_t n3 = 3 * h->n_nodes;
-        for (int64_t k = 0; k < n3; ++k)
-            if (!std::isfinite(dJdu[k])) return fail({MAILLE_INVALID_INPUT, "non-finite dJ/du"});
         // adjoint right-hand side g at free DOFs; lambda = 0 at fixed DOFs (no coupling term)
         CK(cudaMemcpyAsync(h->y_full, dJdu, n3 * sizeof(double), cudaMemcpyHostToDevice, st));
+        if (!all_finite(h, h->y_full, n3)) return fail({MAILLE_INVALID_INPUT, "non-finite dJ/du"});
         launch_build_rhs(h->sym.nb, h->perm, h->fixmask, h->y_full, nullptr, h->b64, st);
         if (!h->lambda_full) {
             h->lambda_full = dalloc<double>(n3);

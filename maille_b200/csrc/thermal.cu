@@ -311,27 +311,71 @@ __global__ void __launch_bounds__(kT) k_heat_elem(HeatElemIn in, double* __restr
 
 // ---- assembly and factorisation --------------------------------------------------------------
 
-// One thread per lower slot (I, J), J <= I: the left and right entries summed over the slot's
-// element pairs in element order (the scatter map of gpu_pattern), written at the slot and at
-// its transposed position.
-__global__ void k_heat_assemble(int64_t nl, int64_t ne, int np, const int64_t* __restrict__ lslot,
-                                const int64_t* __restrict__ lptr, const uint32_t* __restrict__ contrib,
-                                const int64_t* __restrict__ tpos, const double* __restrict__ left,
-                                const double* __restrict__ right, double* __restrict__ A,
-                                double* __restrict__ R) {
-    for (int64_t l = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; l < nl; l += (int64_t)gridDim.x * blockDim.x) {
-        double sa = 0.0, sr = 0.0;
-        for (int64_t k = lptr[l]; k < lptr[l + 1]; ++k) {
-            const uint32_t c = contrib[k] & 0x7fffffffu;
-            const int64_t e = c / (uint32_t)np, pair = c - e * np;
-            sa += left[pair * ne + e];
-            sr += right[pair * ne + e];
+// The left and right matrices on the free-node pattern: one warp per row walks the elements incident to
+// its node in element order (k_assemble of kernels.cu on scalars): lane b finds the column of the
+// element's node b and adds the pair's two entries to the row's sums in shared memory.
+constexpr int kHeatCols = 128;
+template <int NPE>
+__global__ void __launch_bounds__(kT) k_heat_assemble(int32_t nb, int64_t ne, const int32_t* __restrict__ perm,
+                                                      const int64_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc,
+                                                      const int32_t* __restrict__ conn, const int32_t* __restrict__ inv,
+                                                      const int64_t* __restrict__ row_ptr, const int32_t* __restrict__ col,
+                                                      const double* __restrict__ left, const double* __restrict__ right,
+                                                      double* __restrict__ A, double* __restrict__ R) {
+    __shared__ double2 sums[kT / 32][kHeatCols];
+    __shared__ int32_t cols[kT / 32][kHeatCols];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int64_t I = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (I >= nb) return;
+    double2* sum = sums[wp];
+    int32_t* rc = cols[wp];
+    const int32_t v = perm[I];
+    const int64_t q0 = inc_ptr[v], q1 = inc_ptr[v + 1], rb = row_ptr[I];
+    const int n = (int)(row_ptr[I + 1] - rb);
+    for (int c0 = 0; c0 < n; c0 += kHeatCols) {
+        const int nc = min(kHeatCols, n - c0);
+        for (int t = lane; t < nc; t += 32) {
+            rc[t] = col[rb + c0 + t];
+            sum[t] = make_double2(0.0, 0.0);
         }
-        const int64_t pos = lslot[l], tp = tpos[pos];
-        A[pos] = sa;
-        R[pos] = sr;
-        A[tp] = sa;
-        R[tp] = sr;
+        __syncwarp();
+        auto load = [&](int64_t q, int32_t& pos, int32_t& J, double& l, double& r) {
+            pos = inc[q];
+            J = -1;
+            if (lane < NPE) {
+                const int64_t e = pos / NPE;
+                const int a = pos - (int)(e * NPE), lo = min(a, lane), hi = max(a, lane);
+                const int64_t pair = lo * NPE - lo * (lo - 1) / 2 + (hi - lo);
+                J = inv[conn[e * NPE + lane]];
+                l = left[pair * ne + e];
+                r = right[pair * ne + e];
+            }
+        };
+        int32_t pos = 0, J = -1;
+        double l = 0.0, r = 0.0;
+        if (q0 < q1) load(q0, pos, J, l, r);
+        for (int64_t q = q0; q < q1; ++q) {
+            const int32_t j = J;
+            const double lv = l, rv = r;
+            if (q + 1 < q1) load(q + 1, pos, J, l, r);
+            if (j >= 0) {
+                int lo = 0, hi = nc;
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    if (rc[mid] < j) lo = mid + 1; else hi = mid;
+                }
+                if (lo < nc && rc[lo] == j) {
+                    sum[lo].x += lv;
+                    sum[lo].y += rv;
+                }
+            }
+            __syncwarp();
+        }
+        for (int t = lane; t < nc; t += 32) {
+            A[rb + c0 + t] = sum[t].x;
+            R[rb + c0 + t] = sum[t].y;
+        }
+        __syncwarp();
     }
 }
 
@@ -1135,6 +1179,7 @@ struct Slices {
     }
 };
 
+// Device buffers of a step, freed together (the step's stream is idle by then).
 struct DevBufs {
     std::vector<void*> all;
     template <typename T>
@@ -1142,9 +1187,7 @@ struct DevBufs {
         all.push_back((void*)p);
         return p;
     }
-    ~DevBufs() {
-        for (void* p : all) dfree(p);
-    }
+    ~DevBufs() { device_free_all(all); }
 };
 
 bool finite_all(const double* v, int64_t n) {
@@ -1230,40 +1273,23 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || p->device < 0 || p->device >= ndev)
         return th_fail(MAILLE_CUDA_ERROR, "no CUDA device " + std::to_string(p->device));
 
-    // host: ordering of the free nodes (one DOF per node: a node is kept when free) on a thread
-    // of its own while the device takes the inputs and integrates the element matrices
-    std::vector<uint8_t> fixed3(3 * n);
-    for (int64_t v = 0; v < n; ++v) fixed3[3 * v] = fixed3[3 * v + 1] = fixed3[3 * v + 2] = p->fixed[v] ? 1 : 0;
     Symbolic sym;
     Error err{MAILLE_OK, ""};
-    bool analysed = false;
     const double t_setup0 = now_ms();
-    double t_setup1 = t_setup0;
-    // AUTO: MULTICOLOR_BFS (on Tet10 40^3: 17 levels against 18 and 12 % fewer iterations than
-    // MULTICOLOR, the step 21 % shorter). The ordering runs on the device (ordering.cu) once the
-    // connectivity is there, the node incidence on this thread meanwhile; MAILLE_HOST_ORDERING=1
-    // orders on the thread instead (the same permutation).
-    const int ordering = p->ordering == MAILLE_ORDER_AUTO ? MAILLE_ORDER_MULTICOLOR_BFS : p->ordering;
+    // AUTO: kOrderIndex, as the elastic solves (against MULTICOLOR_BFS with the coarse correction: Tet4
+    // 23x30x17 22.6 against 24.1 ms, Tet10 40^3 152 against 148, 14 levels against 18, 40 iterations
+    // against 38)
+    const int ordering = p->ordering == MAILLE_ORDER_AUTO ? kOrderIndex : p->ordering;
     const char* host_env = std::getenv("MAILLE_HOST_ORDERING");
     const bool host_ordering = host_env && std::atoi(host_env) != 0;
-    std::vector<int32_t> kept, kept_of;
     std::vector<double> box(6, 0.0);  // of the nodes, for the coarse grid
-    std::thread analysis([&] {
-        if (host_ordering)
-            analysed = analyse(n, npe, ne, p->conn, fixed3.data(), ordering, sym, err, /*pattern=*/false,
-                               /*boundary_lists=*/false);
-        else
-            analysed = analyse_topology(n, npe, ne, p->conn, fixed3.data(), sym, kept, kept_of, err,
-                                        /*boundary_lists=*/false, /*incidence=*/false);
-        coarse_box(p->coords, 0, n, box.data());
-        t_setup1 = now_ms();
-    });
+    std::thread boxer([&] { coarse_box(p->coords, 0, n, box.data()); });
     struct Joiner {
         std::thread& t;
         ~Joiner() {
             if (t.joinable()) t.join();
         }
-    } joiner{analysis};
+    } joiner{boxer};
 
     cudaStream_t st = nullptr;
     cudaEvent_t ev[7] = {};
@@ -1349,38 +1375,37 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
         }
         CK(cudaEventRecord(ev[2], st));
         gpu_incidence(conn, ne * npe, n, st, inc_ptr, inc);
+        Scratch tmp(st);
+        GraphDev graph;
+        int32_t *kept_of = tmp.take<int32_t>(n), *kept = tmp.take<int32_t>(n);
+        const int32_t nb = gpu_keep(1, n, fixed, st, kept_of, kept);
+        if (nb == 0) return th_fail(MAILLE_INVALID_INPUT, "every DOF is fixed");
+        int32_t *order = tmp.take<int32_t>(nb), *rank = tmp.take<int32_t>(nb);
+        gpu_graph(npe, ne, conn, inc_ptr, inc, kept_of, kept, nb, st, graph);
+        int32_t *perm = mem.take(dalloc<int32_t>(nb)), *inv = mem.take(dalloc<int32_t>(n));
         if (host_ordering) {
-            analysis.join();
-            if (!analysed) return th_fail(err.status, err.message);
+            std::vector<uint8_t> fixed3(3 * n);
+            for (int64_t v = 0; v < n; ++v) fixed3[3 * v] = fixed3[3 * v + 1] = fixed3[3 * v + 2] = p->fixed[v] ? 1 : 0;
+            if (!analyse(n, npe, ne, p->conn, fixed3.data(), ordering, sym, err)) return th_fail(err.status, err.message);
+            CK(cudaMemcpyAsync(perm, sym.perm.data(), nb * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+            gpu_ranks(nb, perm, kept_of, st, order, rank);
         } else {
-            std::vector<int32_t> h_kept_of(n, -1), h_kept;
-            for (int64_t v = 0; v < n; ++v)
-                if (!p->fixed[v]) {
-                    h_kept_of[v] = (int32_t)h_kept.size();
-                    h_kept.push_back((int32_t)v);
-                }
-            int32_t* d_kept_of = mem.take(dupload(h_kept_of.data(), h_kept_of.size(), st));
-            std::vector<int32_t> order, level;
-            gpu_ordering(npe, ne, conn, d_kept_of, (int32_t)h_kept.size(), ordering, st, order, level);
-            analysis.join();
-            if (!analysed) return th_fail(err.status, err.message);
-            apply_ordering(h_kept, order, level, fixed3.data(), sym);
+            gpu_ordering(graph, ordering, st, order, sym.level_ptr);
         }
+        gpu_rows(1, nb, n, order, kept, kept_of, fixed, st, perm, inv, rank, nullptr);
+        sym.nb = nb;
+        sym.levels = (int32_t)sym.level_ptr.size() - 1;
+        const double t_setup1 = now_ms();
         if (sym.levels >= kMaxLevels) return th_fail(MAILLE_INVALID_INPUT, "too many IC(0) levels");
-        const int32_t nb = sym.nb;
-        int32_t* perm = mem.take(dupload(sym.perm.data(), sym.perm.size(), st));
-        int32_t* inv = mem.take(dupload(sym.inv.data(), sym.inv.size(), st));
         std::vector<int32_t> fixed_nodes;
         for (int64_t v = 0; v < n; ++v)
             if (p->fixed[v]) fixed_nodes.push_back((int32_t)v);
         int32_t* fnodes = mem.take(dupload(fixed_nodes.data(), fixed_nodes.size(), st));
         PatternDev pt;
-        gpu_pattern(npe, ne, conn, inv, nb, st, pt, sym.row_ptr, sym.diag);
-        for (void* q : {(void*)pt.row_ptr, (void*)pt.col, (void*)pt.diag, (void*)pt.tpos, (void*)pt.lslot,
-                        (void*)pt.lrow, (void*)pt.lptr, (void*)pt.contrib})
-            mem.take(q);
+        gpu_pattern(graph, order, rank, st, pt, sym.row_ptr, sym.diag);
+        for (void* q : {(void*)pt.row_ptr, (void*)pt.col, (void*)pt.diag, (void*)pt.tpos}) mem.take(q);
         sym.blocks = pt.blocks;
-        sym.nl = pt.nl;
+        tmp.release();
         {
             // lanes per row: MAILLE_THERMAL_LPR_A (the SpMV layouts; 0 picks from the mean row
             // length), MAILLE_THERMAL_LPR_LU (the triangles; 2 measured best on Tet10 40^3 against
@@ -1399,6 +1424,7 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
         sk.upload(pt, nb, st);
         sl.upload(pt, nb, st);
         su.upload(pt, nb, st);
+        boxer.join();
         if (const char* e = std::getenv("MAILLE_COARSE");
             ordering != MAILLE_ORDER_RCM && !(e && std::atoi(e) == 0) && coarse_pays(p, box, nb))
             coarse.plan(1, p->precision == MAILLE_MIXED, nb, pt.blocks, coords, perm, nullptr, pt.row_ptr, pt.col, nullptr,
@@ -1409,8 +1435,15 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
         double* F = mem.take(dalloc<double>((size_t)pt.blocks));
         CK(cudaEventRecord(ev[3], st));
         counted();
-        k_heat_assemble<<<grid_of(pt.nl), kT, 0, st>>>(pt.nl, ne, np, pt.lslot, pt.lptr, pt.contrib, pt.tpos, left,
-                                                       right, A, R);
+        {
+            const unsigned rows_grid = (unsigned)(((int64_t)nb * 32 + kT - 1) / kT);
+            if (npe == 4)
+                k_heat_assemble<4><<<rows_grid, kT, 0, st>>>(nb, ne, perm, inc_ptr, inc, conn, inv, pt.row_ptr, pt.col, left,
+                                                             right, A, R);
+            else
+                k_heat_assemble<10><<<rows_grid, kT, 0, st>>>(nb, ne, perm, inc_ptr, inc, conn, inv, pt.row_ptr, pt.col,
+                                                              left, right, A, R);
+        }
         CK(cudaGetLastError());
         CK(cudaEventRecord(ev[6], st));
         // IC(0) with the shift ladder (Pcg::new, iterative.rs:201-207)
