@@ -12,13 +12,11 @@
 //
 // Sweeps are dataflow instead of one barrier per level: warps take slices in level order on a
 // fixed round-robin schedule; before gathering a neighbour's value a lane waits until that row
-// has been written in the current sweep (epoch): while any record of the warp is stale, one lane
-// polls the one likely written last and the warp then re-reads its stale records together (a
-// poll by every lane is up to 128 scattered L2 requests per warp, and the waiting warps' polls
-// delayed the working warps' own instructions). A slice only depends on slices of earlier
-// levels, which come earlier in every warp's schedule, and all warps are co-resident
-// (cooperative launch), so every wait ends; each wait is also bounded and reports a timeout
-// status instead of spinning forever. How a lane knows a row is ready depends on the precision:
+// has been written in the current sweep (epoch), re-reading its stale records. A slice only depends on
+// slices of earlier levels, which come earlier in every warp's schedule, and all warps are
+// co-resident (cooperative launch), so every wait ends; each wait is also bounded and reports a
+// timeout status instead of spinning forever. How a lane knows a row is ready depends on the
+// precision:
 //  * FP32: the sweep vector holds one 16-byte record per node, (z0, z1, z2, tag), written and
 //    read as single 128-bit accesses; the tag is the epoch of the sweep that wrote the record.
 //    A gather that sees the current tag has the row's values in the same access (the
@@ -254,38 +252,19 @@ __device__ __forceinline__ Rec64 pad_record<double>() {
     return Rec64{0.0, 0.0, 0.0, __longlong_as_double(-1ll)};
 }
 
-// Waits until the 4 records q (read from z at columns cc) carry `epoch`; called by the whole warp.
-// While any lane has a record that is not current, one lane polls the warp's pending record that
-// is usually written last (rows are numbered by level: the largest column in a forward sweep, the
-// smallest in a backward one), then every lane re-reads its pending records together (one L2
-// round trip), and so on; at most `limit` polls in all; false when the limit ran out. Polling with one lane instead of every lane's
-// records matters: a warp-wide poll of 128 scattered records is 128 L2 requests, and the waiting
-// warps' polls queued ahead of the working warps' own loads and shuffles (Tet4 20^3 FP64: the
-// sweeps' per-level time fell from 9 us to 4 us; Tet10 40^3: the mixed step 11 % shorter).
+// Waits until this lane's 4 records q (read from z at columns cc) carry `epoch`, re-reading the stale
+// ones, at most `limit` times; false when the limit ran out. Every lane polls its own: with the coarse
+// correction's few iterations the waits are worth the most direct path. (One lane polling the
+// warp's latest record and the warp re-reading its records afterwards was an extra L2 round trip a
+// level; an iteration took, against this form, Tet4 6^3 80 / 61 us, 20^3 97 / 75, 26^3 98 / 79, Tet10
+// 12^3 156 / 122 FP64 and 117 / 96 mixed, 28^3 320 / 305 FP64 and 219 / 209 mixed, 40^3 mixed 391 / 385.)
 template <typename T>
 __device__ __forceinline__ bool await_records(const T* z, const int32_t cc[4], unsigned int epoch,
-                                              typename RecOf<T>::type q[4], unsigned int limit, bool fwd) {
+                                              typename RecOf<T>::type q[4], unsigned int limit) {
     bool pending = false;
 #pragma unroll
     for (int j = 0; j < 4; ++j) pending = pending || !ready(q[j], epoch);
-    unsigned int k = 0;
-    while (__any_sync(0xffffffffu, pending) && k < limit) {
-        // the pending column to poll: largest (forward) or smallest (backward), as an unsigned
-        // maximum of c or of ~c
-        uint32_t key = 0u;
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (!ready(q[j], epoch)) key = max(key, fwd ? (uint32_t)cc[j] + 1u : ~(uint32_t)cc[j]);
-        key = __reduce_max_sync(0xffffffffu, key);
-        const int32_t mc = fwd ? (int32_t)(key - 1u) : (int32_t)~key;
-        if ((threadIdx.x & 31) == 0) {
-            typename RecOf<T>::type w = ld_record(z, mc);
-            while (!ready(w, epoch) && k < limit) {
-                w = ld_record(z, mc);
-                ++k;
-            }
-        }
-        k = __shfl_sync(0xffffffffu, k, 0) + 1;
+    for (unsigned int k = 0; pending && k < limit; ++k) {
 #pragma unroll
         for (int j = 0; j < 4; ++j)
             if (!ready(q[j], epoch)) q[j] = ld_record(z, cc[j]);
@@ -293,6 +272,7 @@ __device__ __forceinline__ bool await_records(const T* z, const int32_t cc[4], u
 #pragma unroll
         for (int j = 0; j < 4; ++j) pending = pending || !ready(q[j], epoch);
     }
+    __syncwarp();
     return !pending;
 }
 
@@ -304,7 +284,7 @@ __global__ void k_wait_selftest(const float* z, unsigned int epoch, unsigned int
     Rec32 q[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) q[j] = ld_record(z, cc[j]);
-    const bool ok = await_records<float>(z, cc, epoch, q, limit, true);
+    const bool ok = __all_sync(0xffffffffu, await_records<float>(z, cc, epoch, q, limit));
     if ((threadIdx.x & 31) == 0) *timed_out = ok ? 0 : 1;
 }
 
@@ -403,13 +383,12 @@ __device__ __forceinline__ void issue_records(int4 c4, const T* z, int32_t pad, 
 // lane's columns were fetched ahead and its records q requested by issue_records, so their L2
 // round trip is the step's only wait. Once every lane has read the buffer, lane 0 starts the copy
 // of step `next` (the next step of this slice or the first of the warp's next slice; < 0: none).
-// `fwd`: the sweep's direction, which tells the wait which pending record to poll.
 template <typename T>
 __device__ __forceinline__ bool slot_products(const T* __restrict__ vals, int4 c4, const T* z,
                                               unsigned int epoch, int lane, Stage<T>& st,
-                                              int64_t next, typename RecOf<T>::type q[4], T P[4][3], bool fwd) {
+                                              int64_t next, typename RecOf<T>::type q[4], T P[4][3]) {
     const int32_t cc[4] = {c4.x, c4.y, c4.z, c4.w};
-    bool ok = await_records<T>(z, cc, epoch, q, kSpinLimit, fwd);
+    bool ok = await_records<T>(z, cc, epoch, q, kSpinLimit);
     ok = mbar_wait(st.bar, st.phase) && ok;
     st.phase ^= 1u;
     const T* V = st.buf + 4 * lane;
@@ -604,7 +583,7 @@ __device__ __forceinline__ double sweep(const PsellDev& A, unsigned int epoch, c
             const uint32_t mine = head_bits(m0.head, lane);
             const int last = lane + 1 < nrows ? nth_set(m0.head, lane + 1) - 1 : 127;
             T P[4][3];
-            ok = slot_products(vals, c0, z, epoch, lane, st, next_slice, q, P, FWD) && ok;
+            ok = slot_products(vals, c0, z, epoch, lane, st, next_slice, q, P) && ok;
             // in-lane running sums, restarted at each row start; the lane's carry-out is the sum
             // of its slots after its last row start (all 4 when none starts here)
             T s0 = 0, s1 = 0, s2 = 0;
@@ -653,7 +632,7 @@ __device__ __forceinline__ double sweep(const PsellDev& A, unsigned int epoch, c
                 R q[4];
                 issue_records<T>(cg4, z, A.pad, q);
                 T P[4][3];
-                ok = slot_products(vals, cg4, z, epoch, lane, st, g + 1 < m0.g1 ? g + 1 : next_slice, q, P, FWD) && ok;
+                ok = slot_products(vals, cg4, z, epoch, lane, st, g + 1 < m0.g1 ? g + 1 : next_slice, q, P) && ok;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) { a0 += P[j][0]; a1 += P[j][1]; a2 += P[j][2]; }
             }

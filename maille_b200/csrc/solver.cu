@@ -588,11 +588,16 @@ int32_t create_impl(const MailleElasticProblem* p, MailleGpuHandle** out, Maille
         // 4 reduction slots for every block of the persistent grid and of the norm kernels
         // (grids capped at 8 and 4 blocks per SM)
         h->persist_grid = std::min(h->persist_grid, 8 * device_sms());
-        // small systems: a grid sized to the work (one block of 8 warps per 8 slices of K, at
-        // least half the SMs), so that each of the iteration's grid barriers spans fewer blocks
-        // (the large-strain block, 587 slices: 74 blocks, 8 % faster than 296)
-        h->persist_grid = std::min<int64_t>(
-            h->persist_grid, std::max<int64_t>(device_sms() / 2, (h->sk.h.nslices() + 7) / 8));
+        // systems whose matrix and factor hold less than 200 MB: at most a block per SM, sized to the work
+        // (one block of 8 warps per 8 slices of K, at least half the SMs), so that the sweeps' levels and
+        // the grid barriers span fewer warps; larger ones are paced by the bytes in flight. Microseconds
+        // an iteration with 74 / 148 / 296 blocks: Tet4 20^3 (19 MB) 75 / 74 / 88, 26^3 (41 MB) 83 / 79 / 89,
+        // 40^3 (147 MB) 151 / 124 / 132, Tet10 20^3 mixed (147 MB) 190 / 148 / 151; Tet4 48^3 (254 MB) - /
+        // 154 / 152, Tet10 28^3 mixed (396 MB) - / 231 / 209
+        const int64_t steps = h->sk.h.steps() + h->pl.h.steps() + h->pu.h.steps();
+        if (steps * kStepSlots * (9 * (is_mixed(h.get()) ? 4 : 8) + 4) < 200000000)
+            h->persist_grid = std::min<int64_t>(
+                {h->persist_grid, device_sms(), std::max<int64_t>(device_sms() / 2, (h->sk.h.nslices() + 7) / 8)});
         // MAILLE_PERSIST_GRID: fewer co-resident blocks than the occupancy allows (a tuning and
         // measurement knob: the phases' time against the warps in flight and the barrier cost)
         if (const int blocks = env_int("MAILLE_PERSIST_GRID", 0); blocks > 0)
