@@ -116,11 +116,21 @@ __device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
 __device__ __forceinline__ void st_release(unsigned int* p, unsigned int v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-__device__ __forceinline__ bool wait_ready(const unsigned int* f, unsigned int epoch) {
-    if (ld_acquire(f) >= epoch) return true;
+// Waits until the ready flags of a lane's 4 columns (stride G, group g) have reached `epoch`, re-reading
+// the stale ones together.
+__device__ __forceinline__ bool wait_ready4(const unsigned int* flags, const int32_t cc[4], int G, int g,
+                                            unsigned int epoch) {
+    unsigned int f[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) f[j] = ld_acquire(flags + (int64_t)cc[j] * G + g);
     for (unsigned int k = 0; k < kBatchSpin; ++k) {
-        __nanosleep(64);
-        if (ld_acquire(f) >= epoch) return true;
+        bool pending = false;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) pending = pending || f[j] < epoch;
+        if (!pending) return true;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (f[j] < epoch) f[j] = ld_acquire(flags + (int64_t)cc[j] * G + g);
     }
     return false;
 }
@@ -160,11 +170,7 @@ __device__ __forceinline__ void step_acc(const M* __restrict__ vals, const int32
     constexpr int AB = group_align<T, Q>();
     const int4 c4 = __ldg(reinterpret_cast<const int4*>(col + gs * Gm::SS + slot0));
     const int32_t cc[4] = {c4.x, c4.y, c4.z, c4.w};
-    if (flags) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (ok) ok = wait_ready(flags + (int64_t)cc[j] * Gm::G + g, epoch);
-    }
+    if (flags && ok) ok = wait_ready4(flags, cc, Gm::G, g, epoch);
     const M* V = vals + gs * 9 * Gm::SS + slot0;
     if constexpr (sizeof(M) == 8) {
 #pragma unroll
