@@ -804,7 +804,7 @@ int32_t solve_batch(MailleGpuBatch* b, const double* f, MailleBatchResult* res) 
         if (f) {
             for (size_t k = 0; k < nf; ++k)
                 if (!std::isfinite(f[k])) return fail({MAILLE_INVALID_INPUT, "non-finite load"});
-            CK(cudaMemcpyAsync(b->f, f, nf * sizeof(double), cudaMemcpyHostToDevice, st));
+            host_upload(b->f, f, nf * sizeof(double), st);
             b->f_cur = b->f;
         } else {
             b->f_cur = b->f0;
@@ -863,7 +863,7 @@ int32_t solve_batch(MailleGpuBatch* b, const double* f, MailleBatchResult* res) 
         CK(cudaMemcpyAsync(b->h_status.data(), b->state.status, b->n_inst * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
         CK(cudaMemcpyAsync(b->h_rr.data(), b->state.rr, ncol * sizeof(double), cudaMemcpyDeviceToHost, st));
         CK(cudaMemcpyAsync(b->h_bb.data(), b->state.bb, ncol * sizeof(double), cudaMemcpyDeviceToHost, st));
-        if (res && res->u) CK(cudaMemcpyAsync(res->u, b->u_out, nf * sizeof(double), cudaMemcpyDeviceToHost, st));
+        if (res && res->u) host_download(res->u, b->u_out, nf * sizeof(double), st);
         CK(cudaEventRecord(b->ev[3], st));
         CK(cudaStreamSynchronize(st));
         int32_t status = MAILLE_OK;
@@ -939,9 +939,9 @@ int32_t refactor_batch(MailleGpuBatch* b, const double* young, const double* poi
     Error err{MAILLE_OK, ""};
     try {
         CK(cudaSetDevice(b->device));
-        if (young) CK(cudaMemcpyAsync(b->young, young, b->n_elems * sizeof(double), cudaMemcpyHostToDevice, b->st));
+        if (young) host_upload(b->young, young, b->n_elems * sizeof(double), b->st);
         if (poisson)
-            CK(cudaMemcpyAsync(b->poisson, poisson, b->n_elems * sizeof(double), cudaMemcpyHostToDevice, b->st));
+            host_upload(b->poisson, poisson, b->n_elems * sizeof(double), b->st);
         if (numeric(b, err) != MAILLE_OK) return fail(err);
         if (b->cfg.valid()) fill_values(b);
         CK(cudaStreamSynchronize(b->st));

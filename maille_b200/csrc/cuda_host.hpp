@@ -51,6 +51,11 @@ int32_t trim_device_memory(int device);
 // its host address); slots are reused, never returned to the driver.
 void* pinned_slot_alloc(size_t bytes);
 void pinned_slot_free(void* p);
+// Copies between the device and host memory, enqueued on st. A large copy from or to pageable memory is
+// shared by several threads (memory.cu): an upload has read the host memory when it returns, a
+// download has written it; smaller ones and page-locked memory are plain cudaMemcpyAsync.
+void host_upload(void* dev, const void* host, size_t bytes, cudaStream_t st);
+void host_download(void* host, const void* dev, size_t bytes, cudaStream_t st);
 // Streaming multiprocessors of the current device (cudaDevAttrMultiProcessorCount, cached per
 // device): grid caps are multiples of it.
 int device_sms();
@@ -64,7 +69,7 @@ T* dalloc(size_t n) {
 template <typename T>
 T* dupload(const T* src, size_t n, cudaStream_t st) {
     T* d = dalloc<T>(n);
-    if (n && src) CK(cudaMemcpyAsync(d, src, n * sizeof(T), cudaMemcpyHostToDevice, st));
+    if (n && src) host_upload(d, src, n * sizeof(T), st);
     return d;
 }
 

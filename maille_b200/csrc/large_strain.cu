@@ -458,9 +458,9 @@ int32_t ls_run(MailleGpuLargeStrain* s, MailleLargeStrainResult* res) {
     }
     CK(cudaGetLastError());
     if (res) {
-        if (res->u) CK(cudaMemcpyAsync(res->u, s->ckpt, s->increments * n3 * sizeof(double), cudaMemcpyDeviceToHost, st));
+        if (res->u) host_download(res->u, s->ckpt, s->increments * n3 * sizeof(double), st);
         if (res->reactions)
-            CK(cudaMemcpyAsync(res->reactions, s->react, s->increments * n3 * sizeof(double), cudaMemcpyDeviceToHost, st));
+            host_download(res->reactions, s->react, s->increments * n3 * sizeof(double), st);
     }
     CK(cudaStreamSynchronize(st));
     s->ran = true;

@@ -660,7 +660,7 @@ int32_t solve_impl(MailleGpuHandle* h, const double* f, MailleElasticResult* res
         const Symbolic& s = h->sym;
         const int64_t n3 = 3 * h->n_nodes;
         if (f) {
-            CK(cudaMemcpyAsync(h->f, f, n3 * sizeof(double), cudaMemcpyHostToDevice, st));
+            host_upload(h->f, f, n3 * sizeof(double), st);
             if (!all_finite(h, h->f, n3)) return fail({MAILLE_INVALID_INPUT, "non-finite load"});
             h->f_cur = h->f;
         } else {
@@ -708,15 +708,13 @@ int32_t solve_impl(MailleGpuHandle* h, const double* f, MailleElasticResult* res
         CK(cudaGetLastError());
         CK(cudaEventRecord(h->ev[6], st));
         if (res) {
-            if (res->u) CK(cudaMemcpyAsync(res->u, h->u_full, n3 * sizeof(double), cudaMemcpyDeviceToHost, st));
+            if (res->u) host_download(res->u, h->u_full, n3 * sizeof(double), st);
             if (res->reactions)
-                CK(cudaMemcpyAsync(res->reactions, h->react, n3 * sizeof(double), cudaMemcpyDeviceToHost, st));
+                host_download(res->reactions, h->react, n3 * sizeof(double), st);
             if (res->gauss_stress)
-                CK(cudaMemcpyAsync(res->gauss_stress, h->gauss, (size_t)h->n_elems * ng * 9 * sizeof(double),
-                                   cudaMemcpyDeviceToHost, st));
+                host_download(res->gauss_stress, h->gauss, (size_t)h->n_elems * ng * 9 * sizeof(double), st);
             if (res->von_mises)
-                CK(cudaMemcpyAsync(res->von_mises, h->vm, (size_t)h->n_elems * ng * sizeof(double),
-                                   cudaMemcpyDeviceToHost, st));
+                host_download(res->von_mises, h->vm, (size_t)h->n_elems * ng * sizeof(double), st);
         }
         CK(cudaEventRecord(h->ev[7], st));
         CK(cudaStreamSynchronize(st));
@@ -774,7 +772,7 @@ int32_t backward_impl(MailleGpuHandle* h, const double* dJdu, double* dJdE, doub
         cudaStream_t st = h->st;
         const int64_t n3 = 3 * h->n_nodes;
         // adjoint right-hand side g at free DOFs; lambda = 0 at fixed DOFs (no coupling term)
-        CK(cudaMemcpyAsync(h->y_full, dJdu, n3 * sizeof(double), cudaMemcpyHostToDevice, st));
+        host_upload(h->y_full, dJdu, n3 * sizeof(double), st);
         if (!all_finite(h, h->y_full, n3)) return fail({MAILLE_INVALID_INPUT, "non-finite dJ/du"});
         launch_build_rhs(h->sym.nb, h->perm, h->fixmask, h->y_full, nullptr, h->b64, st);
         if (!h->lambda_full) {
@@ -795,9 +793,9 @@ int32_t backward_impl(MailleGpuHandle* h, const double* dJdu, double* dJdE, doub
         launch_adjoint_grad(h->npe, h->n_elems, h->conn, h->ke, h->young, h->lambda_full, h->u_full,
                             h->grad, st);
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(dJdE, h->grad, h->n_elems * sizeof(double), cudaMemcpyDeviceToHost, st));
+        host_download(dJdE, h->grad, h->n_elems * sizeof(double), st);
         if (lambda)
-            CK(cudaMemcpyAsync(lambda, h->lambda_full, n3 * sizeof(double), cudaMemcpyDeviceToHost, st));
+            host_download(lambda, h->lambda_full, n3 * sizeof(double), st);
         CK(cudaStreamSynchronize(st));
     } catch (const CudaFailure& e) {
         return fail({MAILLE_CUDA_ERROR, e.what});
@@ -895,9 +893,9 @@ int32_t maille_gpu_refactor(MailleGpuHandle* h, const double* young, const doubl
     try {
         CK(cudaSetDevice(h->device));
         if (young)
-            CK(cudaMemcpyAsync(h->young, young, h->n_elems * sizeof(double), cudaMemcpyHostToDevice, h->st));
+            host_upload(h->young, young, h->n_elems * sizeof(double), h->st);
         if (poisson)
-            CK(cudaMemcpyAsync(h->poisson, poisson, h->n_elems * sizeof(double), cudaMemcpyHostToDevice, h->st));
+            host_upload(h->poisson, poisson, h->n_elems * sizeof(double), h->st);
         Error err{MAILLE_OK, ""};
         if (numeric_phase(h, err) != MAILLE_OK) return fail(err);
         h->solved = false;
@@ -933,13 +931,13 @@ int32_t maille_gpu_multiply(MailleGpuHandle* h, const double* x, double* y) {
     try {
         CK(cudaSetDevice(h->device));
         const int64_t n3 = 3 * h->n_nodes;
-        CK(cudaMemcpyAsync(h->y_full, x, n3 * sizeof(double), cudaMemcpyHostToDevice, h->st));
+        host_upload(h->y_full, x, n3 * sizeof(double), h->st);
         launch_build_rhs(h->sym.nb, h->perm, h->fixmask, h->y_full, nullptr, h->p64, h->st);
         launch_spmv<double>(h->sk.dev(), h->Ks64, h->p64, h->ap64, h->spmv_grid, h->st);
         CK(cudaMemsetAsync(h->react, 0, n3 * sizeof(double), h->st));
         launch_gather_u(h->n_nodes, h->inv, h->fixed, h->react, h->ap64, h->y_full, h->st);
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(y, h->y_full, n3 * sizeof(double), cudaMemcpyDeviceToHost, h->st));
+        host_download(y, h->y_full, n3 * sizeof(double), h->st);
         CK(cudaStreamSynchronize(h->st));
         h->solved = false;
     } catch (const CudaFailure& e) {
@@ -962,10 +960,8 @@ int32_t maille_gpu_nodal_stresses(MailleGpuHandle* h, double* stress, double* vo
         launch_nodal_stresses(h->npe, h->n_nodes, h->inc_ptr, h->inc, h->gauss, h->node_stress,
                               h->node_vm, h->st);
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(stress, h->node_stress, (size_t)h->n_nodes * 6 * sizeof(double),
-                           cudaMemcpyDeviceToHost, h->st));
-        CK(cudaMemcpyAsync(von_mises, h->node_vm, (size_t)h->n_nodes * sizeof(double),
-                           cudaMemcpyDeviceToHost, h->st));
+        host_download(stress, h->node_stress, (size_t)h->n_nodes * 6 * sizeof(double), h->st);
+        host_download(von_mises, h->node_vm, (size_t)h->n_nodes * sizeof(double), h->st);
         CK(cudaStreamSynchronize(h->st));
     } catch (const CudaFailure& e) {
         return fail({MAILLE_CUDA_ERROR, e.what});

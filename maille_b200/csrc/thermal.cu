@@ -1654,12 +1654,12 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
         const double t_dl0 = now_ms();
         if (res) {
             if (res->temperatures)
-                CK(cudaMemcpy(res->temperatures, temps, (size_t)(steps + 1) * n * sizeof(double), cudaMemcpyDeviceToHost));
+                host_download(res->temperatures, temps, (size_t)(steps + 1) * n * sizeof(double), st);
             if (res->reactions)
-                CK(cudaMemcpy(res->reactions, react, (size_t)(steps + 1) * n * sizeof(double), cudaMemcpyDeviceToHost));
+                host_download(res->reactions, react, (size_t)(steps + 1) * n * sizeof(double), st);
             if (want_flux)
-                CK(cudaMemcpy(res->heat_fluxes, flux, (size_t)(steps + 1) * ne * ng * 6 * sizeof(double),
-                              cudaMemcpyDeviceToHost));
+                host_download(res->heat_fluxes, flux, (size_t)(steps + 1) * ne * ng * 6 * sizeof(double), st);
+            CK(cudaStreamSynchronize(st));
             int64_t total = 0;
             double worst = 0.0;
             for (int32_t s = 0; s < steps; ++s) {
