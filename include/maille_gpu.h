@@ -391,8 +391,9 @@ void maille_gpu_large_strain_destroy(MailleGpuLargeStrain* s);
  * assembly.rs:413-433), then per increment
  *   (C/dt + theta K) T_{n+1} = (C/dt - (1 - theta) K) T_n + F
  * with the left matrix assembled and IC(0)-factorised once (FreeSystem::new, model.rs:1442-1499;
- * Pcg::new) and each increment solved by IC(0)-PCG from a zero start to ||r|| <= rel_tol ||b||
- * (Pcg::solve, iterative.rs:210-248); reactions R = C (T_{n+1} - T_n)/dt + K (theta T_{n+1} +
+ * Pcg::new) and each increment solved by IC(0)-PCG to ||r|| <= rel_tol ||b|| (Pcg::solve,
+ * iterative.rs:210-248; after the first increment from the projection of the earlier ones, with the
+ * RCM ordering from a zero start as the reference); reactions R = C (T_{n+1} - T_n)/dt + K (theta T_{n+1} +
  * (1 - theta) T_n) - F on imposed nodes and the heat fluxes q = -k grad T (heat_fluxes,
  * element.rs:480-506) of every increment. Imposed temperatures replace the initial field at
  * their nodes from t = 0. The whole step runs on the device: one host synchronisation at the

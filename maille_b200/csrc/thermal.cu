@@ -534,6 +534,9 @@ __global__ void __launch_bounds__(kT) k_heat_rhs(SellDev R, const double* __rest
     }
 }
 
+// Earlier increments that a PCG starts from.
+constexpr int kHeatHist = 8;
+
 // Arguments of the persistent PCG kernel of one increment. T is the storage type of the
 // iteration's matrices and vectors: double in the plain form, float in the mixed form, whose
 // solution accumulates in x64 (FP64) through reliable updates against the FP64 matrix A64v.
@@ -564,6 +567,12 @@ struct HeatPcg {
     double* r64;                     // [nb + 1] the true residual b - A x64
     double delta;                    // reliable update when ||r|| fell below delta x its last true value
     CoarseDev<T> c;                  // the preconditioner's coarse correction (c.nn = 0: none)
+    // start from earlier increments: the last hist of them lie in a ring of `ring` slots, the newest in
+    // slot - 1; this one goes to `slot` (ring = 0: zero start, nothing kept)
+    int32_t hist, ring, slot;
+    double *hb, *hx;                 // [ring][nb + 1] their right-hand sides b_k and solutions x_k
+    double* hgram;                   // [kHeatHist][kHeatHist] b_k . b_l of the slots
+    double* x0;                      // [nb + 1] the start
 };
 
 __device__ __forceinline__ unsigned long long heat_clock() {
@@ -818,11 +827,60 @@ __device__ __forceinline__ void st2(float* p, double a, double b) {
     *reinterpret_cast<float2*>(p) = make_float2((float)a, (float)b);
 }
 
-// IC(0)-PCG of one increment from x = 0 (Pcg::solve, iterative.rs:210-248) in one cooperative
-// launch: SpMV, the x / r update, the dataflow preconditioner and the p update, each closed by a
-// grid barrier (four per iteration). (Fusing the two updates into the SpMV and the sweeps saves
-// two barriers but puts more loads on the sweeps' critical path; measured slower.) Every
-// reduction is per-block partials in fixed slots summed in slot order by every block.
+// Coefficients g of sum_k g_k b_k closest to b in the 2-norm, over the `hist` slots before `slot` of the
+// ring, from the inner products: c_k = b_k . b, a.hgram. Cholesky of the Gram matrix of the scaled b_k,
+// newest first; a b_k that lies in the span of newer ones to 3e-7 (the pivot, its squared distance,
+// below 1e-13, which the products' rounding reaches) is left out, and so is a zero or non-finite
+// one. One thread; g is indexed by the slot.
+template <typename T>
+__device__ void start_coefficients(const HeatPcg<T>& a, const double* c, double* g) {
+    __shared__ double L[kHeatHist][kHeatHist], y[kHeatHist], scale[kHeatHist];
+    auto slot = [&](int i) { return (a.slot - 1 - i + 2 * a.ring) % a.ring; };  // i-th newest
+    for (int i = 0; i < a.hist; ++i) {
+        const int si = slot(i);
+        const double n2 = __ldcg(a.hgram + si * kHeatHist + si);
+        scale[i] = n2 > 0.0 ? 1.0 / sqrt(n2) : 0.0;
+        double t = c[si] * scale[i], d = n2 * scale[i] * scale[i];
+        for (int j = 0; j < i; ++j) {
+            double l = __ldcg(a.hgram + si * kHeatHist + slot(j)) * scale[i] * scale[j];
+            for (int m = 0; m < j; ++m) l -= L[i][m] * L[j][m];
+            l = L[j][j] > 0.0 ? l * L[j][j] : 0.0;  // the inverse pivot, 0 of one left out
+            L[i][j] = l;
+            t -= l * y[j];
+            d -= l * l;
+        }
+        const double inv = d > 1e-13 ? 1.0 / sqrt(d) : 0.0;
+        if (inv == 0.0)
+            for (int j = 0; j < i; ++j) L[i][j] = 0.0;
+        L[i][i] = inv;
+        y[i] = inv > 0.0 ? t * inv : 0.0;
+    }
+    for (int i = a.hist - 1; i >= 0; --i) {
+        double t = y[i];
+        for (int j = i + 1; j < a.hist; ++j) t -= L[j][i] * y[j];
+        y[i] = t * L[i][i];
+    }
+    for (int i = 0; i < a.hist; ++i) g[slot(i)] = y[i] * scale[i];
+}
+
+// the PCG's state of row i at the start x0: residual r0 = b - A x0, no correction yet
+template <typename T>
+__device__ __forceinline__ void start_row(const HeatPcg<T>& a, int64_t i, double x0, double r0, double& rr) {
+    a.x[i] = (T)0;
+    a.r[i] = (T)r0;
+    if constexpr (sizeof(T) == 4) {
+        a.x64[i] = x0;
+        a.r64[i] = r0;
+    }
+    rr += r0 * r0;
+}
+
+// IC(0)-PCG of one increment (Pcg::solve, iterative.rs:210-248) in one cooperative
+// launch, from x = 0 or, after earlier increments of the step, from their projection: SpMV, the x / r
+// update, the dataflow preconditioner and the p update, each closed by a grid barrier (four per
+// iteration). (Fusing the two updates into the SpMV and the sweeps saves two barriers but puts more
+// loads on the sweeps' critical path; measured slower.) Every reduction is per-block partials in
+// fixed slots summed in slot order by every block.
 // MIXED: FP32 matrices and vectors with FP64 scalars and reductions; whenever the FP32 residual
 // fell by delta since the last true one (and at the end), x64 += x, x = 0 and r64 = b - A64 x64 in
 // FP64, r = r64 (the reliable update of the elastic mixed form); the stopping test is on r64.
@@ -851,20 +909,61 @@ __global__ void __launch_bounds__(kT, 2) k_heat_pcg(HeatPcg<T> a) {
         }
     };
     unsigned long long epoch = a.epoch0;
-    double loc = 0.0;
+    // ||b||, and b against the earlier increments' right-hand sides
+    __shared__ double start[2 * kHeatHist];  // c_k = b_k . b, then the coefficients, by slot
+    double loc = 0.0, dots[kHeatHist] = {};
     for (int64_t i = tid; i < a.nb; i += nth) {
         const double bi = a.b[i];
-        a.x[i] = (T)0;
-        a.r[i] = (T)bi;
-        if constexpr (MIXED) {
-            a.x64[i] = 0.0;
-            a.r64[i] = bi;
-        }
         loc += bi * bi;
+#pragma unroll
+        for (int k = 0; k < kHeatHist; ++k)
+            if (k < a.hist) dots[k] += a.hb[(int64_t)k * (a.nb + 1) + i] * bi;
     }
     heat_publish(loc, a.partials, 3, sh);
+#pragma unroll
+    for (int k = 0; k < kHeatHist; ++k)
+        if (k < a.hist) heat_publish(dots[k], a.partials, 4 + k, sh);
     grid.sync();
     const double bnorm = sqrt(heat_total(a.partials, 3));
+    // The start x0 = sum_k g_k x_k: since A x_k = b_k, the least residual over the span of the earlier
+    // solutions comes from the b_k alone; the PCG then starts from its true residual b - A x0. The
+    // residual against ||b|| at the 2nd, 5th and 10th increment: 0.05, 1e-3, 2e-7 (Tet10, backward
+    // Euler), 0.5, 0.03, 1e-4 (Tet4, Crank-Nicolson). The
+    // iterations fall from 40 to 18 over ten increments of Tet10 40^3 (112 -> 83 ms) and from 24 to 16 over twelve of Tet4
+    // 23x30x17 (17.8 -> 15.2 ms). (Keeping only what each increment added, with the oldest
+    // dropped or the last replaced, loses the basis once the ring is full; four kept: 3e-6, 2e-3.)
+    if (a.hist > 0) {
+        for (int k = 0; k < a.hist; ++k) {
+            const double c = heat_total(a.partials, 4 + k);
+            if (threadIdx.x == 0) start[k] = c;
+        }
+        if (threadIdx.x == 0) start_coefficients(a, start, start + kHeatHist);
+        __syncthreads();
+        for (int64_t i = tid; i < a.nb; i += nth) {
+            double x = 0.0;
+            for (int k = 0; k < a.hist; ++k) x += start[kHeatHist + k] * a.hx[(int64_t)k * (a.nb + 1) + i];
+            a.x0[i] = x;
+        }
+        grid.sync();
+    }
+    loc = 0.0;
+    if (a.hist > 0) {
+        const int lane = threadIdx.x & 31, S = 32 / a.A.lpr, r = lane / a.A.lpr, q = lane % a.A.lpr;
+        const int32_t w0 = (int32_t)(tid >> 5), nw = (int32_t)(nth >> 5);
+        const double* vals;
+        if constexpr (MIXED) vals = a.A64v;
+        else vals = a.Av;
+        for (int32_t sl = w0; sl < a.A.nslices; sl += nw) {
+            const double acc = slice_row_dot_t<2>(a.A, vals, sl, (const double*)a.x0, lane);
+            const int32_t row = a.A.rowid[(int64_t)sl * S + r];
+            if (q == 0 && row >= 0) start_row(a, row, __ldcg(a.x0 + row), a.b[row] - acc, loc);
+        }
+    } else {
+        for (int64_t i = tid; i < a.nb; i += nth) start_row(a, i, 0.0, a.b[i], loc);
+    }
+    heat_publish(loc, a.partials, 1, sh);
+    grid.sync();
+    const double rr0 = heat_total(a.partials, 1);
     // z = (L L^T)^-1 r by the sweeps, the coarse correction's y = E^-1 P^T r beside them (the barrier
     // between its restriction and its gather is waited for behind the sweeps); this thread's share
     // of r . (z + P y)
@@ -908,10 +1007,10 @@ __global__ void __launch_bounds__(kT, 2) k_heat_pcg(HeatPcg<T> a) {
             }
         }
     };
-    double maxr = bnorm;  // mixed: the last true residual norm
+    double maxr = sqrt(rr0);  // mixed: the last true residual norm
     int32_t status = 0, it = 0;
-    double rel = 0.0;
-    if (bnorm > 0.0) {
+    double rel = bnorm > 0.0 ? sqrt(rr0) / bnorm : 0.0;
+    if (bnorm > 0.0 && !(sqrt(rr0) <= a.tol * bnorm)) {
         loc = precondition();
         heat_publish(loc, a.partials, 2, sh);
         grid.sync();
@@ -1030,10 +1129,30 @@ __global__ void __launch_bounds__(kT, 2) k_heat_pcg(HeatPcg<T> a) {
             mark(3);
         }
     }
+    // x = x0 + the correction (in the mixed form x64 holds it already), and the pair that later increments
+    // start from; every block is past its last read of x
+    if (a.ring > 0)
+        for (int64_t i = tid; i < a.nb; i += nth) {
+            double x;
+            if constexpr (MIXED) {
+                x = __ldcg(a.x64 + i);
+            } else {
+                x = __ldcg(a.x + i);
+                if (a.hist > 0) a.x[i] = x += __ldcg(a.x0 + i);
+            }
+            const int64_t j = (int64_t)a.slot * (a.nb + 1) + i;
+            a.hb[j] = a.b[i];
+            a.hx[j] = x;
+        }
     if (lead) {
         *a.status = status;
         *a.iterations = it;
         *a.rel = rel;
+        if (a.ring > 0) {
+            for (int k = 0; k < a.hist; ++k)
+                a.hgram[a.slot * kHeatHist + k] = a.hgram[k * kHeatHist + a.slot] = start[k];
+            a.hgram[a.slot * (kHeatHist + 1)] = bnorm * bnorm;
+        }
     }
 }
 
@@ -1591,7 +1710,22 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pcg_fn, kT, csmem));
         const int grid = sms * std::min(per_sm, 2);
         if (grid <= 0) return th_fail(MAILLE_CUDA_ERROR, "the PCG kernel does not fit on the device");
-        double* partials = mem.take(dalloc<double>((size_t)4 * grid));
+        double* partials = mem.take(dalloc<double>((size_t)(4 + kHeatHist) * grid));
+        // The earlier increments that each one starts from; RCM keeps the zero start, for the reference's
+        // iteration counts, and so does a device without room for them (17 vectors at most: a tenth of what a
+        // Tet10 step holds already)
+        int32_t ring = ordering != MAILLE_ORDER_RCM ? std::min<int32_t>(kHeatHist, steps - 1) : 0;
+        double* earlier = nullptr;
+        if (ring > 0) {
+            try {
+                earlier = mem.take(dalloc<double>((2 * ring + 1) * nv + kHeatHist * kHeatHist));
+            } catch (const CudaFailure&) {
+                cudaGetLastError();
+                ring = 0;
+            }
+        }
+        double *hb = earlier, *hx = earlier + ring * nv, *x0 = earlier + 2 * ring * nv, *hgram = earlier + (2 * ring + 1) * nv;
+        if (ring > 0) CK(cudaMemsetAsync(x0, 0, nv * sizeof(double), st));
         // MAILLE_PHASE_TIMING: device time of the PCG phases (block 0), printed at the end
         unsigned long long* timing = nullptr;
         if (const char* e = std::getenv("MAILLE_PHASE_TIMING"); e && std::atoi(e) != 0) {
@@ -1609,11 +1743,14 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
             counted();
             k_heat_gate<<<1, 1, 0, st>>>(d_cancel, s > 1 ? d_status + (s - 2) : nullptr, d_status + (s - 1));
             counted();
+            // the oldest pair makes room for the newest
+            const int32_t hist = std::min(s - 1, ring), slot = ring > 0 ? (s - 1) % ring : 0;
             if (!mixed) {
                 HeatPcg<double> a{nb, sk.dev(), sl.dev(), su.dev(), bwd_slice, Av, Lv, Uv, D, b, x, r, pp, ap,
                                   yrec, zrec, partials, timeout, (unsigned long long)s << 32, tol, max_iter,
                                   d_status + (s - 1), d_iters + (s - 1), d_rel + (s - 1), timing,
-                                  nullptr, nullptr, nullptr, 0.0, coarse.dev64()};
+                                  nullptr, nullptr, nullptr, 0.0, coarse.dev64(), hist, ring, slot, hb, hx,
+                                 hgram, x0};
                 void* args[] = {&a};
                 CK(cudaLaunchCooperativeKernel(pcg_fn, dim3(grid), dim3(kT), args, csmem, st));
             } else {
@@ -1622,7 +1759,8 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
                 HeatPcg<float> a{nb, sk.dev(), sl.dev(), su.dev(), bwd_slice, Av32, Lv32, Uv32, D32, b, x32, r32,
                                  p32, ap32, yrec32, zrec32, partials, timeout, epoch0, tol, max_iter,
                                  d_status + (s - 1), d_iters + (s - 1), d_rel + (s - 1), timing,
-                                 Av, x, r64, coarse.active() ? kCoarseDelta : kHeatDelta, coarse.dev32()};
+                                 Av, x, r64, coarse.active() ? kCoarseDelta : kHeatDelta, coarse.dev32(), hist, ring, slot, hb, hx,
+                                 hgram, x0};
                 void* args[] = {&a};
                 CK(cudaLaunchCooperativeKernel(pcg_fn, dim3(grid), dim3(kT), args, csmem, st));
             }

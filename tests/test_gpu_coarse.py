@@ -118,3 +118,18 @@ def test_a_batch_takes_the_correction(gpu, monkeypatch, rhs, precision, tol, err
     for a, b in zip(out["0"].displacements, out["1"].displacements):
         assert rel(b, a) < 2 * err
     assert out["1"].iterations.max() < out["0"].iterations.max()
+
+
+@pytest.mark.parametrize("increments", [1, 2, 9, 12])
+@pytest.mark.parametrize("theta,precision", [(1.0, MAILLE_FP64), (0.5, MAILLE_FP64), (1.0, MAILLE_MIXED)])
+def test_increments_start_from_the_earlier_ones(gpu, oracle_lib, increments, theta, precision):
+    # one, two, as many as are kept plus one, and more than that: the oracle's history (1e-9 of the largest
+    # temperature, as the thermal parity tests), and never more iterations than the first increment's
+    from maille_b200 import thermal as th
+    p = mg.thermal_cube(6, True, increments=increments, time_period=0.02 * increments, theta=theta)
+    ref = oracle_lib.thermal_transient(p, solver=2)
+    s, out = th.solve_problem(p, f=ref["f"], precision=precision)
+    assert s == 0
+    assert np.abs(out["temps"] - ref["temps"]).max() < 1e-9 * np.abs(ref["temps"]).max()
+    assert np.abs(out["reactions"] - ref["reactions"]).max() < 1e-8 * np.abs(ref["reactions"]).max()
+    assert (out["iterations"] <= out["iterations"][0]).all()
