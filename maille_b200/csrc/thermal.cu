@@ -55,7 +55,8 @@ namespace cg = cooperative_groups;
 namespace maille {
 namespace {
 
-constexpr int kT = 256;  // threads per block of every kernel here
+constexpr int kT = 256;   // threads per block of every kernel here but
+constexpr int kTP = 384;  // the persistent PCG's: one block per SM
 
 inline void counted() { g_kernel_launches.fetch_add(1, std::memory_order_relaxed); }
 inline int grid_of(int64_t n) {
@@ -885,8 +886,8 @@ __device__ __forceinline__ void start_row(const HeatPcg<T>& a, int64_t i, double
 // fell by delta since the last true one (and at the end), x64 += x, x = 0 and r64 = b - A64 x64 in
 // FP64, r = r64 (the reliable update of the elastic mixed form); the stopping test is on r64.
 template <typename T, bool MIXED>
-__global__ void __launch_bounds__(kT, 2) k_heat_pcg(HeatPcg<T> a) {
-    __shared__ double sh[kT / 32];
+__global__ void __launch_bounds__(kTP, 1) k_heat_pcg(HeatPcg<T> a) {
+    __shared__ double sh[kTP / 32];
     extern __shared__ __align__(16) unsigned char coarse_mem[];  // y of the coarse correction
     cg::grid_group grid = cg::this_grid();
     const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
@@ -929,8 +930,8 @@ __global__ void __launch_bounds__(kT, 2) k_heat_pcg(HeatPcg<T> a) {
     // solutions comes from the b_k alone; the PCG then starts from its true residual b - A x0. The
     // residual against ||b|| at the 2nd, 5th and 10th increment: 0.05, 1e-3, 2e-7 (Tet10, backward
     // Euler), 0.5, 0.03, 1e-4 (Tet4, Crank-Nicolson). The
-    // iterations fall from 40 to 18 over ten increments of Tet10 40^3 (112 -> 83 ms) and from 24 to 16 over twelve of Tet4
-    // 23x30x17 (17.8 -> 15.2 ms). (Keeping only what each increment added, with the oldest
+    // iterations fall from 40 to 18 over ten increments of Tet10 40^3 (112 -> 83 ms) and from 24 to 16 over
+    // twelve of Tet4 23x30x17 (17.8 -> 15.2 ms). (Keeping only what each increment added, with the oldest
     // dropped or the last replaced, loses the basis once the ring is full; four kept: 3e-6, 2e-3.)
     if (a.hist > 0) {
         for (int k = 0; k < a.hist; ++k) {
@@ -1527,13 +1528,16 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
         tmp.release();
         {
             // lanes per row: MAILLE_THERMAL_LPR_A (the SpMV layouts; 0 picks from the mean row
-            // length), MAILLE_THERMAL_LPR_LU (the triangles; 2 measured best on Tet10 40^3 against
-            // 1 and 4: the sweeps are latency-bound, 16 rows a slice balance slices against steps)
+            // length), MAILLE_THERMAL_LPR_LU (the triangles). A step of 2 lanes a row holds 8 slots, of 4 lanes
+            // 16: Tet4 rows (7 in a triangle) fit one step of 2; Tet10 rows (13, and 32 at corners) take fewer
+            // dependent steps with 4, at more padding, which pays while the factor stays near the L2.
+            // Ten increments with 2 / 4, ms: Tet10 16^3 22.1 / 20.0, 24^3 (3.2 M entries) 33.9 / 31.2, 40^3 (14.7 M)
+            // 83.6 / 89.7; Tet4 23x30x17 12.4 / 12.7, 40^3 16.2 / 17.0. 8: 40^3 118, Tet4 20.7
             auto env = [](const char* k, int d) {
                 const char* e = std::getenv(k);
                 return e ? std::atoi(e) : d;
             };
-            const int lpr_a = env("MAILLE_THERMAL_LPR_A", 0), lpr_lu = env("MAILLE_THERMAL_LPR_LU", 2);
+            const int lpr_a = env("MAILLE_THERMAL_LPR_A", 0), lpr_lu = env("MAILLE_THERMAL_LPR_LU", npe == 10 && sym.blocks < 6000000 ? 4 : 2);
             std::thread tk([&] { build_sell(sym, SELL_FULL, lpr_a, sk.h); });
             std::thread tl([&] { build_sell(sym, SELL_LOWER, lpr_lu, sl.h); });
             build_sell(sym, SELL_UPPER, lpr_lu, su.h);
@@ -1701,14 +1705,19 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
                                                                 flux + (size_t)s * ne * ng * 6);
         };
         // the persistent kernel: every block co-resident
-        // two blocks of 256 threads per SM (128 registers a thread): 3 or 4 blocks (80 or 64
-        // registers) spill and make every grid barrier dearer, measured slower in every phase
+        // One block of 12 warps per SM (168 registers a thread, no spills), and down to half the SMs where
+        // a warp would have less than 2 slices of K: fewer warps for the levels and the barriers to span.
+        // Ten increments, ms, with 2 x 256 threads (128 registers, spills) / 256 / 384 a SM / 384 on half the
+        // SMs, 2 lanes a triangle row: Tet10 40^3 83.2 / 97.2 / 81.4 / 123, 24^3 36.5 / 31.9 / 32.8 / 36.8, 16^3
+        // 23.1 / 20.1 / 22.1 / 21.2, Tet4 40^3 17.7 / 15.5 / 15.8 / 15.8, Tet4 23x30x17 (twelve) 15.0 / 12.5 /
+        // 13.6 / 12.5. 3 and 4 blocks of 256 spill more: 93.6 and 102 at 40^3. Mixed form, 2 x 256 / as chosen:
+        // 40^3 78.8 / 80.3, 31^3 50.0 / 47.5, 24^3 34.8 / 28.8, 8^3 19.5 / 17.1
         int per_sm = 0, sms = 0, dev = p->device;
         void* pcg_fn = mixed ? (void*)k_heat_pcg<float, true> : (void*)k_heat_pcg<double, false>;
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         const size_t csmem = coarse.active() ? (size_t)coarse.dev64().nn * (mixed ? 4 : 8) : 0;  // y
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pcg_fn, kT, csmem));
-        const int grid = sms * std::min(per_sm, 2);
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pcg_fn, kTP, csmem));
+        const int grid = per_sm <= 0 ? 0 : (int)std::min<int64_t>(sms, std::max<int64_t>(sms / 2, (sk.h.nslices() + 23) / 24));
         if (grid <= 0) return th_fail(MAILLE_CUDA_ERROR, "the PCG kernel does not fit on the device");
         double* partials = mem.take(dalloc<double>((size_t)(4 + kHeatHist) * grid));
         // The earlier increments that each one starts from; RCM keeps the zero start, for the reference's
@@ -1752,7 +1761,7 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
                                   nullptr, nullptr, nullptr, 0.0, coarse.dev64(), hist, ring, slot, hb, hx,
                                  hgram, x0};
                 void* args[] = {&a};
-                CK(cudaLaunchCooperativeKernel(pcg_fn, dim3(grid), dim3(kT), args, csmem, st));
+                CK(cudaLaunchCooperativeKernel(pcg_fn, dim3(grid), dim3(kTP), args, csmem, st));
             } else {
                 // 32-bit tags: increment s starts after the sweeps every earlier increment can take
                 const unsigned long long epoch0 = (unsigned long long)(s - 1) * ((unsigned long long)max_iter + 2);
@@ -1762,7 +1771,7 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
                                  Av, x, r64, coarse.active() ? kCoarseDelta : kHeatDelta, coarse.dev32(), hist, ring, slot, hb, hx,
                                  hgram, x0};
                 void* args[] = {&a};
-                CK(cudaLaunchCooperativeKernel(pcg_fn, dim3(grid), dim3(kT), args, csmem, st));
+                CK(cudaLaunchCooperativeKernel(pcg_fn, dim3(grid), dim3(kTP), args, csmem, st));
             }
             counted();
             k_heat_scatter<<<grid_of(n), kT, 0, st>>>(n, inv, fixed, imp, x, temps + (size_t)s * n);
