@@ -1,5 +1,6 @@
 // coarse_dev.cuh -- device side of the coarse correction (coarse.cuh), for the persistent PCG kernels:
-// z += P E^-1 P^T r in three phases separated by grid barriers of the caller:
+// z += P E^-1 P^T r in three phases separated by barriers of the caller (of its grid, or of the blocks that
+// form a coarse team, coarse_team_barrier):
 //   coarse_restrict  each warp sums w_a(x_i) r_i over a chunk of one cell's rows, for the cell's 8
 //                    corners (r is read once; a chunk's partial sums go to its own slots, so the
 //                    result does not depend on the order the warps run in);
@@ -74,22 +75,32 @@ __device__ __forceinline__ void coarse_halve(T* v, int bit, int lane) {
 // r is padded to 4 entries a row when DOF is 3, plain when it is 1. `warp` of `nwarps` in the grid.
 template <typename T, int DOF>
 __device__ __noinline__ void coarse_restrict(const CoarseDev<T> c, const T* r, int32_t warp, int32_t nwarps) {
+    constexpr int U = sizeof(T) * DOF > 12 ? 2 : 4;  // rows a lane has in flight
     const int lane = threadIdx.x & 31;
     for (int32_t k = warp; k < c.nchunks; k += nwarps) {
         const int4 range = __ldg(c.chunk + k);
         T s[8 * DOF];
 #pragma unroll
         for (int q = 0; q < 8 * DOF; ++q) s[q] = T(0);
-        for (int32_t p = range.x + lane; p < range.y; p += 32) {
-            T f[3], w[8], v[DOF];
-            uint32_t row;
-            coarse_row(c.ws, p, f, row);
-            coarse_load_r<DOF>(r, (int64_t)(row & kCoarseRow), v);
-            coarse_weights(f, w);
+        for (int32_t p = range.x + lane; p < range.y; p += 32 * U) {
+            T f[U][3], v[U][DOF];
+            uint32_t row[U];
 #pragma unroll
-            for (int a = 0; a < 8; ++a)
+            for (int u = 0; u < U; ++u)
+                if (p + 32 * u < range.y) coarse_row(c.ws, p + 32 * u, f[u], row[u]);
 #pragma unroll
-                for (int d = 0; d < DOF; ++d) s[a * DOF + d] += w[a] * v[d];
+            for (int u = 0; u < U; ++u)
+                if (p + 32 * u < range.y) coarse_load_r<DOF>(r, (int64_t)(row[u] & kCoarseRow), v[u]);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (p + 32 * u < range.y) {
+                    T w[8];
+                    coarse_weights(f[u], w);
+#pragma unroll
+                    for (int a = 0; a < 8; ++a)
+#pragma unroll
+                        for (int d = 0; d < DOF; ++d) s[a * DOF + d] += w[a] * v[u][d];
+                }
         }
         // lane bits 4, 3, 2 choose the corner's z, y, x; bits 1, 0 are summed
         coarse_halve<8 * DOF>(s, 16, lane);
@@ -140,19 +151,47 @@ __device__ __noinline__ double coarse_apply(const CoarseDev<T> c, int32_t warp, 
     constexpr int V = 16 / (int)sizeof(T);
     const int lane = threadIdx.x & 31;
     double loc = 0.0;
-    for (int32_t e = warp; e < c.m; e += nwarps) {
-        const T* row = c.inv + (int64_t)e * c.ld;
-        T s = T(0);  // ld is a multiple of 64, zero beyond m in the matrix and in rc
+    // two rows at a time: 8 KB a warp in flight
+    for (int32_t e = warp; e < c.m; e += 2 * nwarps) {
+        const bool two = e + nwarps < c.m;
+        const T *row0 = c.inv + (int64_t)e * c.ld, *row1 = row0 + (two ? (int64_t)nwarps * c.ld : 0);
+        T s[2] = {T(0), T(0)};  // ld is a multiple of 64, zero beyond m in the matrix and in rc
 #pragma unroll 8
-        for (int32_t q = lane * V; q < c.ld; q += 32 * V) s = coarse_dot16(row + q, c.rc + q, s);
+        for (int32_t q = lane * V; q < c.ld; q += 32 * V) {
+            s[0] = coarse_dot16(row0 + q, c.rc + q, s[0]);
+            s[1] = coarse_dot16(row1 + q, c.rc + q, s[1]);
+        }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) {
-            c.y[DOF == 3 ? 4 * (int64_t)(e / 3) + e % 3 : (int64_t)e] = s;
-            loc += (double)__ldcg(c.rc + e) * (double)s;
+        for (int j = 0; j < 2; ++j) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
+            const int32_t i = e + j * nwarps;
+            if (lane == 0 && (j == 0 || two)) {
+                c.y[DOF == 3 ? 4 * (int64_t)(i / 3) + i % 3 : (int64_t)i] = s[j];
+                loc += (double)__ldcg(c.rc + i) * (double)s[j];
+            }
         }
     }
     return loc;
+}
+
+// Barrier among the blocks of a coarse team (co-resident with the grid): every block adds one to `arrived`
+// and waits, at most `limit` reads, until it reaches `target`; on giving up raises `timeout`, which the
+// caller reads after its next grid barrier.
+__device__ __forceinline__ void coarse_team_barrier(int32_t* arrived, int32_t target, int32_t* timeout,
+                                                    unsigned int limit) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(arrived, 1);
+        int32_t n = 0;
+        unsigned int k = 0;
+        do {
+            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(n) : "l"(arrived) : "memory");
+        } while (n < target && ++k < limit);
+        if (n < target) atomicExch(timeout, 1);
+    }
+    __syncthreads();
 }
 
 // P y of a row (DOF 3) from y in shared memory (4 per coarse node), zero at fixed components

@@ -155,6 +155,8 @@ struct MailleGpuHandle {
     int32_t* dfail = nullptr;  // [2]
     int spmv_grid = 1;
     int persist_grid = 0;             // co-resident grid of the persistent PCG kernel
+    int persist_warps = 8;            // warps in each of its blocks
+    int team_blocks = 0;              // those of its blocks that are the coarse team
     int persist_chunk = 64;           // iterations per persistent launch
     unsigned long long* timing = nullptr;  // per-phase ns when MAILLE_PHASE_TIMING is set
     int32_t* claim = nullptr;              // [4]; claim[2]: the sweeps' timeout flag

@@ -3,7 +3,7 @@
 // One launch runs up to `chunk` iterations of Pcg::solve (iterative.rs:222-243): the SpMV, the
 // x/r update with the stopping test (fused into the IC(0) forward sweep in the mixed form: each
 // row takes x += alpha p, r -= alpha ap right before it is swept), the forward and backward
-// sweeps and the p update.
+// sweeps, beside them on blocks of their own the coarse correction (coarse_dev.cuh), and the p update.
 // Phases are separated by grid-wide barriers; every block sums the per-block partials of a
 // reduction in the same fixed order, so alpha, beta and the stopping decisions are bit-identical
 // in every block and the whole grid takes the same branches. The mixed form adds the reliable
@@ -51,7 +51,9 @@ extern std::atomic<long long> g_kernel_launches;
 
 namespace {
 
-constexpr int kPW = 8;                        // warps per block
+// Warps per block, one block per SM: 12 (168 registers a thread) keep more bytes in flight, 8 (255, no
+// spills) shorten the chain of a small system's levels. solver.cu chooses.
+constexpr int kSmallWarps = 8, kLargeWarps = 12;
 constexpr unsigned int kSpinLimit = 1u << 22;  // rounds of a wait before a timeout (seconds)
 
 template <typename T>
@@ -148,6 +150,9 @@ __device__ __forceinline__ void lanes_sum(T& a0, T& a1, T& a2) {
     }
 }
 
+__device__ __forceinline__ int32_t grid_warp() { return (int32_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); }
+__device__ __forceinline__ int32_t grid_warps() { return (int32_t)((gridDim.x * blockDim.x) >> 5); }
+
 // block partial of a grid reduction into partials[slot * G + block]
 __device__ __forceinline__ void publish(double v, double* partials, int slot, double* sh) {
     const double t = block_sum(v, sh);
@@ -169,9 +174,9 @@ __device__ __forceinline__ double spmv_phase(const SellDev& A, const M* vals, co
                                              const double* b = nullptr) {
     const int lane = threadIdx.x & 31, r = lane / LPR, q = lane % LPR;
     constexpr int S = 32 / LPR;
-    const int32_t nw = (int32_t)(gridDim.x * kPW);
+    const int32_t nw = grid_warps();
     double loc = 0.0;
-    for (int32_t sl = (int32_t)(blockIdx.x * kPW + (threadIdx.x >> 5)); sl < A.nslices; sl += nw) {
+    for (int32_t sl = grid_warp(); sl < A.nslices; sl += nw) {
         const int32_t row = A.rowid[(int64_t)sl * S + r];
         T a0 = 0, a1 = 0, a2 = 0;
         const int64_t g0 = A.off[sl], g1 = A.off[sl + 1];
@@ -552,11 +557,11 @@ __device__ __forceinline__ int4 lane_cols(const PsellDev& A, int64_t g, int lane
 template <typename T, bool FWD, bool FUSED = false>
 __device__ __forceinline__ double sweep(const PsellDev& A, unsigned int epoch, const T* vals,
                                         const T* D, int32_t nb, const T* r, T* z, Stage<T>& st,
-                                        bool& ok, const XrUpdate<T>& upd = XrUpdate<T>{}) {
+                                        bool& ok, int32_t nw, const XrUpdate<T>& upd = XrUpdate<T>{}) {
     const int lane = threadIdx.x & 31;
-    const int32_t nw = (int32_t)(gridDim.x * kPW), n = A.nslices;
+    const int32_t n = A.nslices;
     double loc = 0.0;
-    int32_t k = (int32_t)(blockIdx.x * kPW + (threadIdx.x >> 5));
+    int32_t k = grid_warp();
     if (k >= n) return loc;
     SliceMeta m0 = slice_meta(A, k), m1 = slice_meta(A, k + nw);
     int4 c0 = lane_cols(A, m0.g0, lane);
@@ -660,8 +665,8 @@ __device__ __forceinline__ double spmv_staged(const SellDev& A, const float* __r
     const int lane = threadIdx.x & 31, r = lane / LPR, q = lane % LPR;
     constexpr int S = 32 / LPR;
     constexpr uint32_t kBytes = 9 * kStepSlots * sizeof(float);
-    const int32_t nw = (int32_t)(gridDim.x * kPW), n = A.nslices;
-    int32_t sl = (int32_t)(blockIdx.x * kPW + (threadIdx.x >> 5));
+    const int32_t nw = grid_warps(), n = A.nslices;
+    int32_t sl = grid_warp();
     double loc = 0.0;
     if (sl >= n) return loc;
     // staging cursor of lane 0: the next step to copy, walking the warp's slices
@@ -737,8 +742,16 @@ __device__ __forceinline__ unsigned long long gtime() {
     return t;
 }
 
-template <typename T, int LPRK, bool MIXED>
-__global__ void __launch_bounds__(kPW * 32, 2) k_pcg(PcgArgs<T> a, int init) {
+// Blocks 0 .. sweep_blocks - 1 sweep; the others, the coarse team, meanwhile bring the coarse correction
+// from r to y = E^-1 P^T r, with barriers of their own; everything else runs on the whole grid. (Done by the
+// whole grid behind the backward sweep, restriction before it, the correction cost 20 us an iteration
+// whatever the system's size, in blocks of 8 warps at 128 registers, two a SM. Calls with that / this, ms:
+// large strain Tet4 64x16x16 154 / 115, loads Tet4 13x11x12 6.9 / 5.6, Tet10 mixed 21x24x18 29.7 / 22.7, SIMP
+// Tet4 48^3 29.9 / 25.7, Tet4 20^3 7.3 / 6.3, Tet10 27x19x23 27.9 / 25.0, 40^3 mixed 79.1 / 78.1. With the
+// restriction on the whole grid before the sweeps instead of on the team: 139 and 8.1 at the first and the
+// fifth.)
+template <typename T, int LPRK, bool MIXED, int kPW>
+__global__ void __launch_bounds__(kPW * 32, 1) k_pcg(PcgArgs<T> a, int init) {
     __shared__ double sh[kPW];
     __shared__ uint64_t bars[kPW];
     __shared__ uint64_t spmv_bars[2 * kPW];  // the two staging buffers of the mixed form's SpMV
@@ -770,7 +783,15 @@ __global__ void __launch_bounds__(kPW * 32, 2) k_pcg(PcgArgs<T> a, int init) {
             t_last = t;
         }
     };
-    int* timeout = reinterpret_cast<int*>(a.claim + 2);
+    int32_t *timeout = a.claim + 2, *arrived = a.claim + 3;
+    const int32_t team_blocks = (int32_t)gridDim.x - a.sweep_blocks;
+    const bool team = (int32_t)blockIdx.x >= a.sweep_blocks;
+    // P^T r by the team
+    auto restrict_gather = [&]() {
+        coarse_restrict<T, 3>(a.c, a.r, gwarp - a.sweep_blocks * kPW, team_blocks * kPW);
+        coarse_team_barrier(arrived, team_blocks, timeout, kSpinLimit);
+        coarse_gather<T, 3>(a.c, tid - (int64_t)a.sweep_blocks * blockDim.x, (int64_t)team_blocks * blockDim.x);
+    };
     int it = 0;
     while (!v.done && (init ? it < 1 : it < a.chunk)) {
         double loc;
@@ -799,7 +820,7 @@ __global__ void __launch_bounds__(kPW * 32, 2) k_pcg(PcgArgs<T> a, int init) {
             // FP64 sweep's extra registers cost more than the pass; measured both ways).
             if constexpr (MIXED) {
                 v.epoch += 1;
-                loc = sweep<T, true, true>(a.L, v.epoch, a.Lv, a.D, a.nb, a.r, a.z, stage, ok,
+                loc = sweep<T, true, true>(a.L, v.epoch, a.Lv, a.D, a.nb, a.r, a.z, stage, ok, nwarps,
                                            XrUpdate<T>{v.alpha, a.x, a.r, a.p, a.ap});
                 if (!ok) atomicExch(timeout, 1);
                 publish(loc, a.partials, 1, sh);
@@ -884,32 +905,35 @@ __global__ void __launch_bounds__(kPW * 32, 2) k_pcg(PcgArgs<T> a, int init) {
                 need_fwd = true;  // the fused sweep ran on the recurrence residual: again on the true one
             }
         }
-        // z = (L L^T)^-1 r (Csr::precondition, iterative.rs:173-188): dataflow sweeps
+        // z = (L L^T)^-1 r (Csr::precondition, iterative.rs:173-188): dataflow sweeps, and beside them, on the
+        // team's blocks, the coarse correction's y = E^-1 P^T r
+        bool gathered = false;
         if (need_fwd) {
             v.epoch += 1;
-            sweep<T, true>(a.L, v.epoch, a.Lv, a.D, a.nb, a.r, a.z, stage, ok);
+            if (!team) {
+                sweep<T, true>(a.L, v.epoch, a.Lv, a.D, a.nb, a.r, a.z, stage, ok, a.sweep_blocks * kPW);
+            } else {
+                restrict_gather();
+                gathered = true;
+            }
             grid.sync();
             mark(3);
         }
-        // the coarse correction's restriction of r runs before the backward sweep and is gathered after
-        // it, so the grid barrier between the two is waited for behind the sweep
-        cg::grid_group::arrival_token restricted{};
-        if (a.c.nn) {
-            coarse_restrict<T, 3>(a.c, a.r, gwarp, nwarps);
-            restricted = grid.barrier_arrive();
-        }
         v.epoch += 1;
-        loc = sweep<T, false>(a.U, v.epoch, a.Uv, a.D, a.nb, a.r, a.z, stage, ok);
-        if (a.c.nn) {
-            grid.barrier_wait(std::move(restricted));
-            coarse_gather<T, 3>(a.c, tid, nthreads);
-            grid.sync();
-            loc += coarse_apply<T, 3>(a.c, gwarp, nwarps);
+        if (!team) {
+            loc = sweep<T, false>(a.U, v.epoch, a.Uv, a.D, a.nb, a.r, a.z, stage, ok, a.sweep_blocks * kPW);
+        } else {
+            if (!gathered) {
+                restrict_gather();
+                coarse_team_barrier(arrived, 2 * team_blocks, timeout, kSpinLimit);
+            }
+            loc = coarse_apply<T, 3>(a.c, gwarp - a.sweep_blocks * kPW, team_blocks * kPW);
         }
         if (!ok) atomicExch(timeout, 1);
         publish(loc, a.partials, 3, sh);
         grid.sync();
         mark(4);
+        if (blockIdx.x == 0 && threadIdx.x == 0) *arrived = 0;  // used again behind the next grid barrier
         if (__ldcg(timeout)) {
             v.done = 1;
             v.status = 3;
@@ -962,18 +986,21 @@ __global__ void __launch_bounds__(kPW * 32, 2) k_pcg(PcgArgs<T> a, int init) {
 }
 
 // dynamic shared memory of the persistent kernel: one staged step of factor values per warp
-template <typename T>
-constexpr size_t stage_bytes() {
+constexpr size_t stage_bytes(int warps) {
     // one step of FP64 values (9 KB) per warp; two FP32 steps in the mixed form's staged SpMV
-    return (size_t)kPW * 9 * kStepSlots * 8;
+    return (size_t)warps * 9 * kStepSlots * 8;
 }
 
-template <typename T, bool MIXED>
+template <typename T, bool MIXED, int kPW>
 void* pick(int lprk) {
-    if (lprk == 1) return (void*)k_pcg<T, 1, MIXED>;
-    if (lprk == 2) return (void*)k_pcg<T, 2, MIXED>;
-    if (lprk == 4) return (void*)k_pcg<T, 4, MIXED>;
+    if (lprk == 1) return (void*)k_pcg<T, 1, MIXED, kPW>;
+    if (lprk == 2) return (void*)k_pcg<T, 2, MIXED, kPW>;
+    if (lprk == 4) return (void*)k_pcg<T, 4, MIXED, kPW>;
     return nullptr;
+}
+template <typename T, bool MIXED>
+void* pick(int lprk, int warps) {
+    return warps == kLargeWarps ? pick<T, MIXED, kLargeWarps>(lprk) : pick<T, MIXED, kSmallWarps>(lprk);
 }
 
 }  // namespace
@@ -997,32 +1024,32 @@ void wait_selftest(const unsigned int tags[4], unsigned int epoch, unsigned int 
 // Grid size of the persistent kernel: every block co-resident (0 when the layout's lanes-per-
 // row combination has no instance).
 template <typename T, bool MIXED>
-int pcg_persistent_grid(int lprk) {
-    void* f = pick<T, MIXED>(lprk);
+int pcg_persistent_grid(int lprk, int warps) {
+    void* f = pick<T, MIXED>(lprk, warps);
     if (!f) return 0;
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const size_t smem = stage_bytes<T>();
+    const size_t smem = stage_bytes(warps);
     if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, kPW * 32, smem);
-    return sms * per_sm;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, warps * 32, smem);
+    return sms * std::min(per_sm, 1);
 }
 
 template <typename T, bool MIXED>
-cudaError_t launch_pcg_persistent(const PcgArgs<T>& a, int grid, bool init, cudaStream_t st) {
-    void* f = pick<T, MIXED>(a.K.lpr);
+cudaError_t launch_pcg_persistent(const PcgArgs<T>& a, int grid, int warps, bool init, cudaStream_t st) {
+    void* f = pick<T, MIXED>(a.K.lpr, warps);
     if (!f) return cudaErrorInvalidValue;
     PcgArgs<T> copy = a;
     int in = init ? 1 : 0;
     void* args[] = {&copy, &in};
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-    return cudaLaunchCooperativeKernel(f, dim3(grid), dim3(kPW * 32), args, stage_bytes<T>(), st);
+    return cudaLaunchCooperativeKernel(f, dim3(grid), dim3(warps * 32), args, stage_bytes(warps), st);
 }
 
-template int pcg_persistent_grid<double, false>(int);
-template int pcg_persistent_grid<float, true>(int);
-template cudaError_t launch_pcg_persistent<double, false>(const PcgArgs<double>&, int, bool, cudaStream_t);
-template cudaError_t launch_pcg_persistent<float, true>(const PcgArgs<float>&, int, bool, cudaStream_t);
+template int pcg_persistent_grid<double, false>(int, int);
+template int pcg_persistent_grid<float, true>(int, int);
+template cudaError_t launch_pcg_persistent<double, false>(const PcgArgs<double>&, int, int, bool, cudaStream_t);
+template cudaError_t launch_pcg_persistent<float, true>(const PcgArgs<float>&, int, int, bool, cudaStream_t);
 
 }  // namespace maille

@@ -123,6 +123,7 @@ PcgArgs<T> pcg_args(MailleGpuHandle* h, const T* Kv, const T* Lv, const T* Uv, c
     a.partials = h->partials;
     a.timing = h->timing;
     a.claim = h->claim;
+    a.sweep_blocks = h->persist_grid - h->team_blocks;
     if constexpr (sizeof(T) == 4) a.c = h->coarse.dev32();
     else a.c = h->coarse.dev64();
     return a;
@@ -136,10 +137,10 @@ int32_t run_pcg_persistent(MailleGpuHandle* h, int32_t* iterations, int32_t* upd
     auto launch = [&](bool init) {
         if (mixed) {
             auto a = pcg_args<float>(h, h->Ks32, h->Ls32, h->Us32, h->D32, h->x32, h->r32, h->z32, h->p32, h->ap32);
-            CK((launch_pcg_persistent<float, true>(a, h->persist_grid, init, st)));
+            CK((launch_pcg_persistent<float, true>(a, h->persist_grid, h->persist_warps, init, st)));
         } else {
             auto a = pcg_args<double>(h, h->Ks64, h->Ls64, h->Us64, h->D64, h->x64, h->r64, h->z64, h->p64, h->ap64);
-            CK((launch_pcg_persistent<double, false>(a, h->persist_grid, init, st)));
+            CK((launch_pcg_persistent<double, false>(a, h->persist_grid, h->persist_warps, init, st)));
         }
     };
     CK(cudaMemsetAsync(h->claim, 0, 4 * sizeof(int32_t), st));
@@ -583,25 +584,32 @@ int32_t create_impl(const MailleElasticProblem* p, MailleGpuHandle** out, Maille
         h->spmv_grid = grid_for_slices(h->sk.h.nslices());
         h->claim = dalloc<int32_t>(4);
         CK(cudaMemsetAsync(h->claim, 0, 4 * sizeof(int32_t), st));
-        h->persist_grid = is_mixed(h.get()) ? pcg_persistent_grid<float, true>(h->sk.h.lpr)
-                                            : pcg_persistent_grid<double, false>(h->sk.h.lpr);
-        // 4 reduction slots for every block of the persistent grid and of the norm kernels
-        // (grids capped at 8 and 4 blocks per SM)
-        h->persist_grid = std::min(h->persist_grid, 8 * device_sms());
-        // systems whose matrix and factor hold less than 200 MB: at most a block per SM, sized to the work
-        // (one block of 8 warps per 8 slices of K, at least half the SMs), so that the sweeps' levels and
-        // the grid barriers span fewer warps; larger ones are paced by the bytes in flight. Microseconds
-        // an iteration with 74 / 148 / 296 blocks: Tet4 20^3 (19 MB) 75 / 74 / 88, 26^3 (41 MB) 83 / 79 / 89,
-        // 40^3 (147 MB) 151 / 124 / 132, Tet10 20^3 mixed (147 MB) 190 / 148 / 151; Tet4 48^3 (254 MB) - /
-        // 154 / 152, Tet10 28^3 mixed (396 MB) - / 231 / 209
-        const int64_t steps = h->sk.h.steps() + h->pl.h.steps() + h->pu.h.steps();
-        if (steps * kStepSlots * (9 * (is_mixed(h.get()) ? 4 : 8) + 4) < 200000000)
-            h->persist_grid = std::min<int64_t>(
-                {h->persist_grid, device_sms(), std::max<int64_t>(device_sms() / 2, (h->sk.h.nslices() + 7) / 8)});
+        // Below 45000 rows: blocks of 8 warps, sized to the work (one per 8 slices of K, at least half the SMs),
+        // so that the sweeps' levels and the grid barriers span fewer warps; larger systems are paced by the
+        // bytes in flight: 12 warps on every SM. A call's ms with 8 / 12: Tet4 12^3 5.1 / 5.3, 26^3 9.0 / 10.1,
+        // 32^3 (36 k rows) 12.1 / 13.2, 36^3 (49 k) 16.9 / 15.0, 40^3 19.4 / 18.8, 48^3 26.1 / 24.7, mixed 40^3
+        // 17.2 / 16.6; Tet10 12^3 7.8 / 8.5, 18^3 (49 k) 13.6 / 14.2, 33^3 58.5 / 55.7, mixed 15^3 9.0 / 9.5, 18^3
+        // 12.5 / 12.6, 20^3 15.3 / 15.3, 28^3 32.8 / 30.5
+        const bool small = h->sym.nb < 45000;
+        h->persist_warps = small ? 8 : 12;
+        h->persist_grid = is_mixed(h.get()) ? pcg_persistent_grid<float, true>(h->sk.h.lpr, h->persist_warps)
+                                            : pcg_persistent_grid<double, false>(h->sk.h.lpr, h->persist_warps);
+        const int full = h->persist_grid;
+        if (small)
+            h->persist_grid = std::min<int64_t>(full, std::max<int64_t>(device_sms() / 2, (h->sk.h.nslices() + 7) / 8));
         // MAILLE_PERSIST_GRID: fewer co-resident blocks than the occupancy allows (a tuning and
         // measurement knob: the phases' time against the warps in flight and the barrier cost)
         if (const int blocks = env_int("MAILLE_PERSIST_GRID", 0); blocks > 0)
             h->persist_grid = std::min(h->persist_grid, blocks);
+        // the coarse correction's team: a quarter of the SMs. A call's ms with 30 / 37 / 45 of 148: loads Tet10
+        // mixed 21x24x18 25.1 / 23.3 / 23.3, SIMP Tet4 48^3 30.8 / 28.9 / 28.7, Tet10 27x19x23 25.1 / 25.4 / 25.6, 40^3
+        // mixed 78.7 / 77.7 / 78.9, Tet4 20^3 6.5 / 6.5 / 6.6
+        if (h->coarse.active()) {
+            h->team_blocks = std::max(1, full / 4);
+            h->persist_grid = std::min(full, h->persist_grid + h->team_blocks);
+        }
+        // 4 reduction slots for every block of the persistent grid and of the norm kernels (capped at 4 blocks
+        // per SM)
         h->partials = dalloc<double>((size_t)4 * 8 * device_sms());
         if (env_int("MAILLE_PHASE_TIMING", 0)) {
             h->timing = dalloc<unsigned long long>(8);

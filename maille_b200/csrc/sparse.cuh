@@ -81,17 +81,19 @@ struct PcgArgs {
     const double* b64;
     double *x64, *r64;
     PcgScalars* s;
-    int32_t* claim;  // claim[2]: the sweeps' timeout flag
+    int32_t* claim;  // [2]: the sweeps' timeout flag, [3]: arrivals at the coarse team's barrier
+    int32_t sweep_blocks;  // the blocks before this one sweep, the others (none without a coarse correction) are
+                           // the coarse team
     double* partials;       // [4 * grid]
     CoarseDev<T> c;         // the preconditioner's coarse correction (c.nn = 0: none)
     unsigned long long* timing;  // optional [8] ns per phase (block 0): spmv, axpy, update, fwd, bwd, p
 };
 template <typename T, bool MIXED>
-int pcg_persistent_grid(int lprk);
+int pcg_persistent_grid(int lprk, int warps);
 // Self-test of the sweeps' bounded wait (persist.cu): awaits 4 FP32 records with tags `tags` for
 // `epoch` within `limit` rounds; *timed_out = 1 when the wait ran out. Throws CudaFailure.
 void wait_selftest(const unsigned int tags[4], unsigned int epoch, unsigned int limit, int32_t* timed_out);
 template <typename T, bool MIXED>
-cudaError_t launch_pcg_persistent(const PcgArgs<T>& a, int grid, bool init, cudaStream_t st);
+cudaError_t launch_pcg_persistent(const PcgArgs<T>& a, int grid, int warps, bool init, cudaStream_t st);
 
 }  // namespace maille

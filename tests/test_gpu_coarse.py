@@ -133,3 +133,25 @@ def test_increments_start_from_the_earlier_ones(gpu, oracle_lib, increments, the
     assert np.abs(out["temps"] - ref["temps"]).max() < 1e-9 * np.abs(ref["temps"]).max()
     assert np.abs(out["reactions"] - ref["reactions"]).max() < 1e-8 * np.abs(ref["reactions"]).max()
     assert (out["iterations"] <= out["iterations"][0]).all()
+
+
+@pytest.mark.parametrize("cells,precision,tol", [((33, 35, 36), MAILLE_FP64, 1e-12), ((36, 35, 36), MAILLE_FP64, 1e-12),
+                                                 ((36, 35, 36), MAILLE_MIXED, 1e-10)])
+@pytest.mark.parametrize("blocks", [None, "1", "500"])
+def test_the_team_beside_the_sweeps_at_both_block_sizes(gpu, monkeypatch, cells, precision, tol, blocks):
+    # either side of 45000 rows, with one sweeping block and with more than fit, against IC(0) alone: two
+    # solutions at relative residual tol differ by at most 2 cond(K) tol, cond < 1e5 (about 4 n^2 = 5e3
+    # times the moduli's ratio of 4)
+    p = box(cells, tuple(0.1 * c for c in cells), False)
+    m = mb.Model.from_arrays(p.coords, p.conn, p.young, p.poisson, p.fixed, p.imposed, p.loads,
+                             (p.p_elem, p.p_face, p.p_value))
+    m.with_solver(mb.SolverKind.ITERATIVE).with_tolerance(tol).with_precision(precision)
+    m.ordering = MAILLE_ORDER_MULTICOLOR
+    if blocks:
+        monkeypatch.setenv("MAILLE_PERSIST_GRID", blocks)
+    u = {}
+    for knob in ("0", "1"):
+        monkeypatch.setenv("MAILLE_COARSE", knob)
+        u[knob] = m.solve()
+    assert rel(u["1"].displacements, u["0"].displacements) < 2e5 * tol
+    assert u["1"].info["iterations"] < u["0"].info["iterations"]
