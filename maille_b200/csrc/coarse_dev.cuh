@@ -75,7 +75,7 @@ __device__ __forceinline__ void coarse_halve(T* v, int bit, int lane) {
 // r is padded to 4 entries a row when DOF is 3, plain when it is 1. `warp` of `nwarps` in the grid.
 template <typename T, int DOF>
 __device__ __noinline__ void coarse_restrict(const CoarseDev<T> c, const T* r, int32_t warp, int32_t nwarps) {
-    constexpr int U = sizeof(T) * DOF > 12 ? 2 : 4;  // rows a lane has in flight
+    constexpr int U = DOF == 1 ? 1 : 2;  // rows a lane has in flight; more cost the sweeps registers
     const int lane = threadIdx.x & 31;
     for (int32_t k = warp; k < c.nchunks; k += nwarps) {
         const int4 range = __ldg(c.chunk + k);
@@ -151,12 +151,12 @@ __device__ __noinline__ double coarse_apply(const CoarseDev<T> c, int32_t warp, 
     constexpr int V = 16 / (int)sizeof(T);
     const int lane = threadIdx.x & 31;
     double loc = 0.0;
-    // two rows at a time: 8 KB a warp in flight
+    // two rows at a time: 4 KB a warp in flight
     for (int32_t e = warp; e < c.m; e += 2 * nwarps) {
         const bool two = e + nwarps < c.m;
         const T *row0 = c.inv + (int64_t)e * c.ld, *row1 = row0 + (two ? (int64_t)nwarps * c.ld : 0);
         T s[2] = {T(0), T(0)};  // ld is a multiple of 64, zero beyond m in the matrix and in rc
-#pragma unroll 8
+#pragma unroll 4
         for (int32_t q = lane * V; q < c.ld; q += 32 * V) {
             s[0] = coarse_dot16(row0 + q, c.rc + q, s[0]);
             s[1] = coarse_dot16(row1 + q, c.rc + q, s[1]);

@@ -552,7 +552,8 @@ struct HeatPcg {
     T *x, *r, *p, *ap;               // [nb + 1]; the plain form's x is the solution
     Rec *yrec, *zrec;                // [nb + 1] sweep records (value, tag); entry nb always ready
     double* partials;                // [4 * grid]
-    int32_t* timeout;                // set when a record wait ran out
+    int32_t* timeout;                // [0] set when a wait gave up, [1] arrivals at the coarse team's barrier
+    int32_t sweep_blocks;            // the blocks from this one on are the coarse team (none without a correction)
     unsigned long long epoch0;       // the launch's sweeps tag their records epoch0 + 1, + 2, ...
     double tol;
     int32_t max_iter;
@@ -759,7 +760,7 @@ template <typename T>
 __device__ __forceinline__ double heat_sweeps(const HeatPcg<T>& a, unsigned long long epoch) {
     const int lane = threadIdx.x & 31;
     const int32_t w0 = (int32_t)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    const int32_t nw = (int32_t)(((int64_t)gridDim.x * blockDim.x) >> 5);
+    const int32_t nw = a.sweep_blocks * (int32_t)(blockDim.x >> 5);
     const int32_t nl = a.Lo.nslices, nt = a.Lo.nslices + a.Up.nslices;
     bool ok = true;
     double rz = 0.0;
@@ -965,24 +966,22 @@ __global__ void __launch_bounds__(kTP, 1) k_heat_pcg(HeatPcg<T> a) {
     heat_publish(loc, a.partials, 1, sh);
     grid.sync();
     const double rr0 = heat_total(a.partials, 1);
-    // z = (L L^T)^-1 r by the sweeps, the coarse correction's y = E^-1 P^T r beside them (the barrier
-    // between its restriction and its gather is waited for behind the sweeps); this thread's share
-    // of r . (z + P y)
+    // z = (L L^T)^-1 r by the sweeps and, beside them on the team's blocks, the coarse correction's y =
+    // E^-1 P^T r; this thread's share of r . (z + P y). (By the whole grid, restriction before the sweeps and
+    // the rest behind them, ten increments, ms, that / this: Tet10 40^3 81.2 / 75.6, 24^3 30.7 / 26.4, Tet4
+    // 40^3 14.6 / 11.6, 23x30x17, twelve, 12.6 / 10.3.)
+    const bool team = (int32_t)blockIdx.x >= a.sweep_blocks;
     auto precondition = [&]() {
-        cg::grid_group::arrival_token restricted{};
-        const int32_t warp = (int32_t)(tid >> 5), warps = (int32_t)(nth >> 5);
-        if (a.c.nn) {
-            coarse_restrict<T, 1>(a.c, a.r, warp, warps);
-            restricted = grid.barrier_arrive();
-        }
-        double rz = heat_sweeps(a, ++epoch);
-        if (a.c.nn) {
-            grid.barrier_wait(std::move(restricted));
-            coarse_gather<T, 1>(a.c, tid, nth);
-            grid.sync();
-            rz += coarse_apply<T, 1>(a.c, warp, warps);
-        }
-        return rz;
+        epoch += 1;
+        if (!team) return heat_sweeps(a, epoch);
+        const int32_t blocks = (int32_t)gridDim.x - a.sweep_blocks, warps = blocks * (kTP / 32);
+        const int64_t first = (int64_t)a.sweep_blocks * kTP;
+        const int32_t warp = (int32_t)((tid - first) >> 5);
+        coarse_restrict<T, 1>(a.c, a.r, warp, warps);
+        coarse_team_barrier(a.timeout + 1, blocks, a.timeout, kSpinLimit);
+        coarse_gather<T, 1>(a.c, tid - first, (int64_t)blocks * kTP);
+        coarse_team_barrier(a.timeout + 1, 2 * blocks, a.timeout, kSpinLimit);
+        return coarse_apply<T, 1>(a.c, warp, warps);
     };
     // p = z + P y + beta p, two entries per thread and pass
     auto update_p = [&](double beta) {
@@ -1015,6 +1014,7 @@ __global__ void __launch_bounds__(kTP, 1) k_heat_pcg(HeatPcg<T> a) {
         loc = precondition();
         heat_publish(loc, a.partials, 2, sh);
         grid.sync();
+        if (lead) a.timeout[1] = 0;  // used again behind the next grid barrier
         double rz = heat_total(a.partials, 2);
         update_p(0.0);
         grid.sync();
@@ -1118,6 +1118,7 @@ __global__ void __launch_bounds__(kTP, 1) k_heat_pcg(HeatPcg<T> a) {
             heat_publish(loc, a.partials, 2, sh);
             grid.sync();
             mark(2);
+            if (lead) a.timeout[1] = 0;
             if (__ldcg(a.timeout)) {
                 status = 3;
                 break;
@@ -1680,8 +1681,8 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
         for (int32_t l = sym.levels - 1; l >= 0; --l)
             for (int32_t q = su.h.level_slices[l]; q < su.h.level_slices[l + 1]; ++q) bwd.push_back(q);
         int32_t* bwd_slice = mem.take(dupload(bwd.data(), bwd.size(), st));
-        int32_t* timeout = mem.take(dalloc<int32_t>(1));
-        CK(cudaMemsetAsync(timeout, 0, sizeof(int32_t), st));
+        int32_t* timeout = mem.take(dalloc<int32_t>(2));
+        CK(cudaMemsetAsync(timeout, 0, 2 * sizeof(int32_t), st));
         counted();
         k_heat_const<<<grid_of(nv), kT, 0, st>>>(nb, npe, ne, perm, inc_ptr, inc, conn, fixed, imp, f, left, right, g);
         CK(cudaGetLastError());
@@ -1717,7 +1718,13 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         const size_t csmem = coarse.active() ? (size_t)coarse.dev64().nn * (mixed ? 4 : 8) : 0;  // y
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pcg_fn, kTP, csmem));
-        const int grid = per_sm <= 0 ? 0 : (int)std::min<int64_t>(sms, std::max<int64_t>(sms / 2, (sk.h.nslices() + 23) / 24));
+        int grid = per_sm <= 0 ? 0 : (int)std::min<int64_t>(sms, std::max<int64_t>(sms / 2, (sk.h.nslices() + 23) / 24));
+        // the coarse correction's team: an eighth of the SMs. Ten increments, ms, with 15 / 24 / 37 blocks of 148:
+        // Tet10 40^3 75.0 / 77.3 / 80.1, 24^3 26.1 / 27.1 / 28.2, Tet4 64^3 34.1 / 29.7 / 30.8, 40^3 11.5 / 11.7 / 12.3,
+        // 23x30x17 (twelve) 10.2 / 10.6 / 10.8
+        const int team = coarse.active() ? sms / 8 : 0;
+        grid = grid > 0 ? std::min(sms, grid + team) : 0;
+        const int sweep_blocks = grid - team;
         if (grid <= 0) return th_fail(MAILLE_CUDA_ERROR, "the PCG kernel does not fit on the device");
         double* partials = mem.take(dalloc<double>((size_t)(4 + kHeatHist) * grid));
         // The earlier increments that each one starts from; RCM keeps the zero start, for the reference's
@@ -1756,7 +1763,7 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
             const int32_t hist = std::min(s - 1, ring), slot = ring > 0 ? (s - 1) % ring : 0;
             if (!mixed) {
                 HeatPcg<double> a{nb, sk.dev(), sl.dev(), su.dev(), bwd_slice, Av, Lv, Uv, D, b, x, r, pp, ap,
-                                  yrec, zrec, partials, timeout, (unsigned long long)s << 32, tol, max_iter,
+                                  yrec, zrec, partials, timeout, sweep_blocks, (unsigned long long)s << 32, tol, max_iter,
                                   d_status + (s - 1), d_iters + (s - 1), d_rel + (s - 1), timing,
                                   nullptr, nullptr, nullptr, 0.0, coarse.dev64(), hist, ring, slot, hb, hx,
                                  hgram, x0};
@@ -1766,7 +1773,7 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
                 // 32-bit tags: increment s starts after the sweeps every earlier increment can take
                 const unsigned long long epoch0 = (unsigned long long)(s - 1) * ((unsigned long long)max_iter + 2);
                 HeatPcg<float> a{nb, sk.dev(), sl.dev(), su.dev(), bwd_slice, Av32, Lv32, Uv32, D32, b, x32, r32,
-                                 p32, ap32, yrec32, zrec32, partials, timeout, epoch0, tol, max_iter,
+                                 p32, ap32, yrec32, zrec32, partials, timeout, sweep_blocks, epoch0, tol, max_iter,
                                  d_status + (s - 1), d_iters + (s - 1), d_rel + (s - 1), timing,
                                  Av, x, r64, coarse.active() ? kCoarseDelta : kHeatDelta, coarse.dev32(), hist, ring, slot, hb, hx,
                                  hgram, x0};
