@@ -170,8 +170,8 @@ int32_t maille_gpu_backward(MailleGpuHandle* h, const double* dJdu, double* dJdE
 
 /* Numeric refactorisation on the handle's topology: new per-element materials ([n_elems] each,
  * NULL keeps the current ones), then element integration, assembly and IC(0) again, as the
- * reference rebuilds FreeSystem when the matrix changes (model.rs:1011). The ordering, pattern
- * and scatter map are reused; the next solve uses the new matrix. */
+ * reference rebuilds FreeSystem when the matrix changes (model.rs:1011). The ordering and
+ * the pattern are reused; the next solve uses the new matrix. */
 int32_t maille_gpu_refactor(MailleGpuHandle* h, const double* young, const double* poisson);
 
 /* y = K x with the assembled free-DOF matrix (Csr::multiply, iterative.rs:131-142): x and y are

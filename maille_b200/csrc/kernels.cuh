@@ -1,6 +1,6 @@
 // kernels.cuh -- sm_100a kernels of the linear-elastic solve path.
 //
-// Data layout in HBM (new = solver numbering of the kept nodes, see setup.cpp):
+// Data layout in HBM (new = solver numbering of the kept nodes, see ordering.cu):
 //   * K and F (the IC(0) factor) are assembled and factorised on one full 3x3-block CSR pattern:
 //     row_ptr (int64), col (int32), 9 consecutive entries per block, row-major. F holds L below
 //     the diagonal, L^T above it and D = L_II^-1 on the diagonal. The iteration kernels read

@@ -34,7 +34,6 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
-#include <utility>
 
 #include <cooperative_groups.h>
 

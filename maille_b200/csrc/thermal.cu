@@ -5,7 +5,7 @@
 // per increment; right-hand sides, reactions and heat fluxes stay on the device, so a whole step
 // of many increments is enqueued without a host synchronisation.
 //
-// Data layout in HBM (solver numbering = the multicolour order of the free nodes, setup.cpp):
+// Data layout in HBM (solver numbering = the multicolour order of the free nodes, ordering.cu):
 //   * element matrices as node pairs a <= b, pair-major: left[pair * n_elems + e], the element
 //     index fastest so that the element kernel's stores and the assembly's loads coalesce;
 //   * the left matrix A, the right matrix R (free-free part) and the factor F on the full
@@ -21,8 +21,8 @@
 //   * the history [(increments + 1) n_nodes] of temperatures and reactions, and of Gauss-point
 //     heat fluxes when asked for, in the caller's numbering, copied to the host once at the end.
 //
-// Roofline: every iteration kernel here is HBM-bandwidth bound (FP64 values streamed once per
-// SpMV / sweep; vectors stay in L2). The element kernel is FP64 arithmetic, once per step.
+// Roofline: the SpMV is bound by HBM (FP64 values streamed once, vectors in L2), the sweeps by the round trip
+// of each dependent level. The element kernel is FP64 arithmetic, once per step.
 
 #include <algorithm>
 #include <atomic>
@@ -34,7 +34,6 @@
 #include <string>
 #include <thread>
 #include <type_traits>
-#include <utility>
 #include <vector>
 
 #include <cooperative_groups.h>

@@ -358,7 +358,7 @@ class SolverHandle:
 
     def refactor(self, young=None, poisson=None):
         """New per-element materials on the same mesh and constraints: element integration,
-        assembly and IC(0) again, reusing the ordering and scatter map."""
+        assembly and IC(0) again, reusing the ordering and the pattern."""
         ne = self.model.mesh.conn.shape[0]
         ya = None if young is None else np.ascontiguousarray(young, np.float64).ravel()
         pa = None if poisson is None else np.ascontiguousarray(poisson, np.float64).ravel()
