@@ -938,7 +938,12 @@ __global__ void __launch_bounds__(kTP, 1) k_heat_pcg(HeatPcg<T> a) {
             const double c = heat_total(a.partials, 4 + k);
             if (threadIdx.x == 0) start[k] = c;
         }
-        if (threadIdx.x == 0) start_coefficients(a, start, start + kHeatHist);
+        if (threadIdx.x == 0) {
+            if (bnorm > 0.0)
+                start_coefficients(a, start, start + kHeatHist);
+            else  // nothing to solve for: x = 0
+                for (int k = 0; k < a.hist; ++k) start[kHeatHist + k] = 0.0;
+        }
         __syncthreads();
         for (int64_t i = tid; i < a.nb; i += nth) {
             double x = 0.0;

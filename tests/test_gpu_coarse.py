@@ -155,3 +155,14 @@ def test_the_team_beside_the_sweeps_at_both_block_sizes(gpu, monkeypatch, cells,
         u[knob] = m.solve()
     assert rel(u["1"].displacements, u["0"].displacements) < 2e5 * tol
     assert u["1"].info["iterations"] < u["0"].info["iterations"]
+
+
+def test_increments_without_load_stay_zero(gpu):
+    # imposed and initial temperatures 0 and no loads: every right-hand side is 0, so is every start
+    from maille_b200 import thermal as th
+    p = mg.thermal_cube(5, False, increments=4, time_period=0.1, theta=1.0)
+    p.imposed[:] = 0.0
+    p.initial[:] = 0.0
+    s, out = th.solve_problem(p, f=np.zeros(p.n_nodes))
+    assert s == 0
+    assert not out["temps"].any() and not out["iterations"].any()
