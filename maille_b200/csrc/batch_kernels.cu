@@ -838,6 +838,7 @@ __global__ void __launch_bounds__(256) k_batch_pcg(BatchArgs<M, T> a, int passes
                         } else {
                             // reliable update when converged by the recurrence, when the residual
                             // fell by delta since the last update, or at the cap
+                            if (coarse) st.maxr2[s] = fmax(st.maxr2[s], rrv);  // kCoarseDelta
                             flag = small || rrv < a.delta2 * st.maxr2[s] || capped;
                         }
                     }
@@ -924,6 +925,9 @@ __global__ void __launch_bounds__(256) k_batch_pcg(BatchArgs<M, T> a, int passes
                         bool conv = false;
                         if (lane < R && ((fm >> lane) & 1u)) {
                             const int64_t s = (int64_t)inst * R + lane;
+                            const double recurrence = __ldcg(st.rr + s);
+                            // beta = 0 (kCoarseDrift)
+                            if (coarse && !(fabs(rt - recurrence) <= kCoarseDrift * recurrence)) st.rz[s] = INFINITY;
                             st.maxr2[s] = rt;
                             st.rr[s] = rt;
                             conv = rt <= a.tol2 * st.bb[s];

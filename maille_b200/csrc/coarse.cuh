@@ -76,8 +76,16 @@ struct CoarseBatchDev {
 };
 constexpr int kCoarseTileRows = 16;
 
-// Mixed forms with the correction: reliable update when the FP32 residual fell by this factor.
+// Mixed forms with the correction: a reliable update when the FP32 residual fell by kCoarseDelta from the
+// largest it has had since the last update (slender parts raise it by decades before it falls, and the
+// recurrence drifts with the largest); when the true residual's square then differs from the recurrence's by
+// more than kCoarseDrift of it, the direction starts anew (beta = 0): p is conjugate to the lost residual,
+// and kept, it stalled the iteration. Iterations at tol 1e-10, IC(0) alone / p kept, 0.01 from the last true
+// residual / always anew / as here: bar 10x10x60 1030 / singular / 46 / 44, 6x6x48 1082 / not in 10000 / 37 / 35,
+// 4x4x32 648 / 672 / 35 / 34, Tet10 3x3x24 1119 / not / 38 / 36, quarter-cylinder shell 30x2x30 1130 / not / 83 /
+// 82, plate 40x2x40 2199 / not / 70 / 68, cube Tet4 20^3 274 / 40 / 43 / 40.
 constexpr double kCoarseDelta = 0.01;
+constexpr double kCoarseDrift = 1e-4;
 
 // The correction of one system (one or several instances): plan and numeric state.
 class Coarse {

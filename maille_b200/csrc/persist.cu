@@ -854,6 +854,7 @@ __global__ void __launch_bounds__(kPW * 32, 1) k_pcg(PcgArgs<T> a, int init) {
             }
             v.rr = grid_total(a.partials, 1);
             const bool small = sqrt(v.rr) <= v.tol * sqrt(v.bb);
+            if (MIXED && a.c.nn) v.maxr = fmax(v.maxr, sqrt(v.rr));  // kCoarseDelta
             if (!MIXED) {
                 if (small) {
                     v.done = 1;
@@ -883,6 +884,8 @@ __global__ void __launch_bounds__(kPW * 32, 1) k_pcg(PcgArgs<T> a, int init) {
                 publish(loc, a.partials, 2, sh);
                 grid.sync();
                 v.rr_true = grid_total(a.partials, 2);
+                // p is not conjugate to a residual that the recurrence has lost: beta = 0 (kCoarseDrift)
+                if (a.c.nn && !(fabs(v.rr_true - v.rr) <= kCoarseDrift * v.rr)) v.rz = INFINITY;
                 v.maxr = sqrt(v.rr_true);
                 v.updates += 1;
                 if (sqrt(v.rr_true) <= v.tol * sqrt(v.bb)) {

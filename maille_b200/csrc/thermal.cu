@@ -1011,7 +1011,7 @@ __global__ void __launch_bounds__(kTP, 1) k_heat_pcg(HeatPcg<T> a) {
             }
         }
     };
-    double maxr = sqrt(rr0);  // mixed: the last true residual norm
+    double maxr = sqrt(rr0);  // mixed: the last true residual norm, or with the correction the largest since then
     int32_t status = 0, it = 0;
     double rel = bnorm > 0.0 ? sqrt(rr0) / bnorm : 0.0;
     if (bnorm > 0.0 && !(sqrt(rr0) <= a.tol * bnorm)) {
@@ -1075,6 +1075,7 @@ __global__ void __launch_bounds__(kTP, 1) k_heat_pcg(HeatPcg<T> a) {
             mark(1);
             double rn = sqrt(heat_total(a.partials, 1));
             if constexpr (MIXED) {
+                if (a.c.nn) maxr = fmax(maxr, rn);  // kCoarseDelta
                 if (rn <= a.tol * bnorm || rn < a.delta * maxr || it >= a.max_iter) {
                     // reliable update: fold x into x64, the true residual against the FP64 matrix
                     for (int64_t i = tid; i < a.nb; i += nth) {
@@ -1099,7 +1100,11 @@ __global__ void __launch_bounds__(kTP, 1) k_heat_pcg(HeatPcg<T> a) {
                     }
                     heat_publish(loc, a.partials, 1, sh);
                     grid.sync();
+                    const double recurrence = rn;
                     rn = sqrt(heat_total(a.partials, 1));
+                    // beta = 0 (kCoarseDrift)
+                    if (a.c.nn && !(fabs(rn * rn - recurrence * recurrence) <= kCoarseDrift * (recurrence * recurrence)))
+                        rz = INFINITY;
                     maxr = rn;
                     rel = rn / bnorm;
                     if (rn <= a.tol * bnorm) break;
