@@ -100,7 +100,8 @@ struct MailleGpuBatch {
     cudaStream_t st = nullptr;
     cudaEvent_t ev[8] = {};
     int32_t n_inst = 0, npe = 0, n_rhs = 0, R = 0, precision = MAILLE_FP64, max_iter = kDefaultMaxIter;
-    double tol = kDefaultTol, delta = 0.1;
+    double tol = kDefaultTol;
+    double delta = 0.1, coarse_delta = kCoarseDelta;  // of the reliable updates, without and with the correction
     int64_t n_nodes = 0, n_elems = 0;
     std::vector<int64_t> node_off, elem_off;
     std::vector<uint8_t> h_fixed;
@@ -451,7 +452,6 @@ BatchArgs<M, T> batch_args(MailleGpuBatch* b) {
     a.n_rhs = b->n_rhs;
     a.max_iter = b->max_iter;
     a.tol2 = b->tol * b->tol;
-    a.delta2 = b->delta * b->delta;
     a.K = b->lk.dev();
     a.L = b->ll.dev();
     a.U = b->lu.dev();
@@ -483,6 +483,8 @@ BatchArgs<M, T> batch_args(MailleGpuBatch* b) {
     a.cancel = b->d_cancel;
     a.timing = b->timing;
     if (b->cfg.threads % 128 == 0) a.c = b->coarse.batch<T>();  // its product works in groups of 4 warps
+    const double delta = a.c.nodes ? b->coarse_delta : b->delta;
+    a.delta2 = delta * delta;
     return a;
 }
 
@@ -605,7 +607,7 @@ int32_t create_batch(const MailleBatchProblem* p, MailleGpuBatch** out) {
     b->precision = p->precision;
     b->tol = p->rel_tol > 0 ? p->rel_tol : kDefaultTol;
     b->max_iter = p->max_iter > 0 ? p->max_iter : kDefaultMaxIter;
-    if (const char* e = std::getenv("MAILLE_RELIABLE_DELTA")) b->delta = std::atof(e);
+    if (const char* e = std::getenv("MAILLE_RELIABLE_DELTA")) b->delta = b->coarse_delta = std::atof(e);
     b->node_off.assign(p->node_offset, p->node_offset + p->n_instances + 1);
     b->elem_off.assign(p->elem_offset, p->elem_offset + p->n_instances + 1);
     b->n_nodes = b->node_off.back();
@@ -769,8 +771,6 @@ int32_t create_batch(const MailleBatchProblem* p, MailleGpuBatch** out) {
             inst.p = dupload(b->row_inst.data(), b->row_inst.size(), st);
             b->coarse.plan(3, b->mixed(), s.nb, s.blocks, b->coords, b->perm, b->fixmask, b->row_ptr, b->col,
                            static_cast<const int32_t*>(inst.p), box, rows, st, b->R);
-            // as in the single solve (24 x 3 mixed: 9.7, 8.9 and 8.7 ms at 0.1, 0.01 and 0.003)
-            if (b->coarse.active() && !std::getenv("MAILLE_RELIABLE_DELTA")) b->delta = kCoarseDelta;
         }
         CK(cudaEventRecord(b->ev[5], st));
         if (numeric(b.get(), err) != MAILLE_OK) return fail(err);

@@ -112,3 +112,21 @@ def test_the_mixed_thermal_step_along_a_bar(gpu, oracle_lib):
     assert s == 0
     assert np.abs(out["temps"] - ref["temps"]).max() < 1e-9 * np.abs(ref["temps"]).max()
     assert (out["iterations"] <= 2 * plain["iterations"]).all()
+
+
+@pytest.mark.parametrize("threads", ["64", "192"])
+def test_a_batch_in_blocks_without_the_correction_is_ic0s(gpu, monkeypatch, threads):
+    # the correction's product works in groups of 4 warps: other block sizes run IC(0) alone, with its own
+    # threshold of the reliable updates, so the same bits as with the correction switched off
+    probs = [bar((3, 3, 18)), bar((4, 4, 16), draw=1)]
+    loads = [np.stack([p.loads, np.roll(p.loads, -1)], 1) for p in probs]
+    for k, v in (("Q", "2"), ("SUB", "1"), ("TASK", "4"), ("THREADS", threads)):
+        monkeypatch.setenv("MAILLE_BATCH_" + k, v)
+    out = {}
+    for knob in ("0", "1"):
+        monkeypatch.setenv("MAILLE_COARSE", knob)
+        with mb.BatchSolver(probs, loads, tol=1e-10, precision=MAILLE_MIXED) as b:
+            out[knob] = b.solve()
+    assert out["0"].info["status_code"] == 0
+    assert np.array_equal(out["0"].iterations, out["1"].iterations)
+    assert all(np.array_equal(x, y) for x, y in zip(out["0"].displacements, out["1"].displacements))
