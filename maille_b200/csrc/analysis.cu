@@ -149,6 +149,17 @@ __global__ void __launch_bounds__(kT) k_graph_lists(int npe, const int32_t* __re
     }
 }
 
+// *any = 1 when an element names a node twice
+__global__ void k_repeats(int npe, int64_t ne, const int32_t* __restrict__ conn, int32_t* __restrict__ any) {
+    GRID_STRIDE(e, ne) {
+        const int32_t* c = conn + e * npe;
+        bool twice = false;
+        for (int a = 1; a < npe; ++a)
+            for (int b = 0; b < a; ++b) twice = twice || c[a] == c[b];
+        if (twice) *any = 1;
+    }
+}
+
 // keys (I << sh) | J of every ordered pair of distinct kept nodes of an element, ~0 for the others
 __global__ void k_graph_keys(int npe, int64_t ne, const int32_t* __restrict__ conn,
                              const int32_t* __restrict__ kept_of, int sh, uint64_t* __restrict__ keys) {
@@ -358,20 +369,22 @@ void gpu_graph(int npe, int64_t n_elems, const int32_t* conn, const int64_t* inc
     out.off = dalloc<int64_t>((size_t)nk + 1);
     out.deg = dalloc<int32_t>((size_t)nk + 1);
     Scratch tmp(st);
-    int32_t* overflow = tmp.take<int32_t>(1);
-    CK(cudaMemsetAsync(overflow, 0, sizeof(int32_t), st));
+    int32_t* overflow = tmp.take<int32_t>(2);  // [1]: an element names a node twice
+    CK(cudaMemsetAsync(overflow, 0, 2 * sizeof(int32_t), st));
     CK(cudaMemsetAsync(out.deg + nk, 0, sizeof(int32_t), st));
     k_graph_count<<<warps_of(nk), kT, 0, st>>>(npe, conn, inc_ptr, inc, kept_of, kept, nk, out.deg, overflow);
+    k_repeats<<<grid_of(n_elems), kT, 0, st>>>(npe, n_elems, conn, overflow + 1);
     CK(cudaGetLastError());
     size_t bytes = 0;
     CK(cub::DeviceScan::ExclusiveSum(nullptr, bytes, out.deg, out.off, (int)(nk + 1), st));
     CK(cub::DeviceScan::ExclusiveSum(tmp.take<unsigned char>(bytes), bytes, out.deg, out.off, (int)(nk + 1), st));
-    counted(3);
-    int32_t over = 0;
-    CK(cudaMemcpyAsync(&over, overflow, sizeof(over), cudaMemcpyDeviceToHost, st));
+    counted(4);
+    int32_t flags[2] = {0, 0};
+    CK(cudaMemcpyAsync(flags, overflow, sizeof(flags), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(&out.m, out.off + nk, sizeof(out.m), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    if (!over) {
+    out.repeats = flags[1] != 0;
+    if (!flags[0]) {
         out.adj = dalloc<int32_t>((size_t)std::max<int64_t>(1, out.m));
         k_graph_lists<<<warps_of(nk), kT, 0, st>>>(npe, conn, inc_ptr, inc, kept_of, kept, nk, out.off, out.adj);
         CK(cudaGetLastError());

@@ -47,6 +47,7 @@ struct GraphDev {
     int64_t* off = nullptr;  // [nk + 1]
     int32_t* adj = nullptr;  // [m]
     int32_t* deg = nullptr;  // [nk]
+    bool repeats = false;    // an element names a node twice
     cudaStream_t st = nullptr;  // its last user
     GraphDev() = default;
     GraphDev(const GraphDev&) = delete;

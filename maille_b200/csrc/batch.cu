@@ -107,6 +107,7 @@ struct MailleGpuBatch {
     std::vector<uint8_t> h_fixed;
     std::vector<double> h_imposed, h_f0;
     bool any_imposed = false;
+    bool repeats = false;  // an element names a node twice
     Symbolic sym;
     std::vector<int32_t> row_inst;
     SideStream side;  // the coarse correction's set-up runs beside the factorisation
@@ -313,7 +314,7 @@ int32_t factorize(MailleGpuBatch* b, Error& err, int32_t* dfail, F meanwhile) {
 int32_t numeric(MailleGpuBatch* b, Error& err) {
     ElemIn in{b->n_elems, b->coords, b->conn, b->young, b->poisson};
     launch_elem_stiffness(b->npe, in, b->ke, b->st);
-    launch_assemble(b->npe, b->pattern(), AssembleIn{b->perm, b->inc_ptr, b->inc, b->conn, b->inv}, b->ke, b->K, b->st);
+    launch_assemble(b->npe, b->pattern(), AssembleIn{b->perm, b->inc_ptr, b->inc, b->conn, b->inv, b->repeats}, b->ke, b->K, b->st);
     CK(cudaGetLastError());
     CK(cudaEventRecord(b->ev[6], b->st));
     int32_t* dfail = dalloc<int32_t>(1);
@@ -671,6 +672,7 @@ int32_t create_batch(const MailleBatchProblem* p, MailleGpuBatch** out) {
             const int32_t nk = gpu_keep(3, b->n_nodes, b->fixed, st, kept_of, kept);
             int32_t *order = tmp.take<int32_t>(nk), *rank = tmp.take<int32_t>(nk);
             gpu_graph(b->npe, b->n_elems, b->conn, b->inc_ptr, b->inc, kept_of, kept, nk, st, graph);
+            b->repeats = graph.repeats;
             gpu_ordering(graph, kOrderIndex, st, order, s.level_ptr);
             s.levels = (int32_t)s.level_ptr.size() - 1;
             s.nb = nk;

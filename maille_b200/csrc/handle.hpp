@@ -166,7 +166,8 @@ struct MailleGpuHandle {
     Pattern pattern() const {
         return Pattern{sym.nb, row_ptr, col, diag, tpos, fixmask};
     }
-    AssembleIn assembly() const { return AssembleIn{perm, inc_ptr, inc, conn, inv}; }
+    bool repeats = false;  // an element names a node twice
+    AssembleIn assembly() const { return AssembleIn{perm, inc_ptr, inc, conn, inv, repeats}; }
     ~MailleGpuHandle();
 };
 

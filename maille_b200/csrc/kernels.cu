@@ -120,9 +120,11 @@ __global__ void __launch_bounds__(kThreads) k_elem_stiffness(ElemIn in, double* 
 // (in shared memory) and are added to the row's sums there, 32 entries at a time. Every entry is thus
 // summed in element order, the same in K_IJ and K_JI, with no map from element pairs to slots
 // (whose sort took longer than the assembly: 38.4 M pairs on Tet10 40^3). A row of more than kAsmCols
-// blocks is taken in windows. Bound by the gather of the element blocks, each read twice.
+// blocks is taken in windows. Bound by the gather of the element blocks, each read twice. REPEATS: an
+// element may name a node twice; the blocks of its nodes are then added one node after the other (all at
+// once, two lanes would add to one sum).
 constexpr int kAsmCols = 72;
-template <int NPE>
+template <int NPE, bool REPEATS>
 __global__ void __launch_bounds__(kThreads) k_assemble(Pattern pt, AssembleIn in, const double* __restrict__ ke,
                                                        double* __restrict__ K) {
     constexpr int NP = NPE * (NPE + 1) / 2;
@@ -182,10 +184,19 @@ __global__ void __launch_bounds__(kThreads) k_assemble(Pattern pt, AssembleIn in
             }
 #pragma unroll
             for (int k = 0; k < G; ++k) {
+                if constexpr (REPEATS) {
+                    for (int n1 = 0; n1 < NPE; ++n1) {
 #pragma unroll
-                for (int h = 0; h < V; ++h)
-                    if (at[k][h] >= 0) sum[at[k][h]] += x[k][h];
-                __syncwarp();
+                        for (int h = 0; h < V; ++h)
+                            if (at[k][h] >= 0 && (32 * h + lane) / 9 == n1) sum[at[k][h]] += x[k][h];
+                        __syncwarp();
+                    }
+                } else {
+#pragma unroll
+                    for (int h = 0; h < V; ++h)
+                        if (at[k][h] >= 0) sum[at[k][h]] += x[k][h];
+                    __syncwarp();
+                }
             }
         }
         for (int t = lane; t < nc * 9; t += 32) {
@@ -761,8 +772,9 @@ void launch_elem_stiffness(int npe, const ElemIn& in, double* ke_up, cudaStream_
 void launch_assemble(int npe, const Pattern& pt, const AssembleIn& in, const double* ke, double* K, cudaStream_t st) {
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
     const unsigned grid = blocks_for(pt.nb, kWarps, INT32_MAX);
-    if (npe == 4) k_assemble<4><<<grid, kThreads, 0, st>>>(pt, in, ke, K);
-    else k_assemble<10><<<grid, kThreads, 0, st>>>(pt, in, ke, K);
+    auto kernel = in.repeats ? (npe == 4 ? k_assemble<4, true> : k_assemble<10, true>)
+                             : (npe == 4 ? k_assemble<4, false> : k_assemble<10, false>);
+    kernel<<<grid, kThreads, 0, st>>>(pt, in, ke, K);
 }
 
 void launch_factor_level(const Pattern& pt, int32_t r0, int32_t r1, const double* K, double* F,

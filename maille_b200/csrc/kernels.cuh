@@ -43,11 +43,13 @@ struct Pattern {
     const uint8_t* fixmask;
 };
 
-// What the assembly reads beside the pattern: row -> node, the incidence of the nodes, node -> row.
+// What the assembly reads beside the pattern: row -> node, the incidence of the nodes, node -> row, and
+// whether an element names a node twice.
 struct AssembleIn {
     const int32_t* perm;
     const int64_t* inc_ptr;
     const int32_t *inc, *conn, *inv;
+    bool repeats;
 };
 
 // A model's values as the caller gave them (device copies; imposed and f may be null): launch_check_model.

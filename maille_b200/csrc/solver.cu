@@ -481,6 +481,7 @@ int32_t create_impl(const MailleElasticProblem* p, MailleGpuHandle** out, Maille
             const int32_t nk = gpu_keep(3, p->n_nodes, h->fixed, st, kept_of, kept);
             int32_t *order = tmp.take<int32_t>(nk), *rank = tmp.take<int32_t>(nk);
             gpu_graph(h->npe, h->n_elems, h->conn, h->inc_ptr, h->inc, kept_of, kept, nk, st, graph);
+            h->repeats = graph.repeats;
             tmark("graph");
             h->perm = dalloc<int32_t>(nk);
             h->inv = dalloc<int32_t>(p->n_nodes);

@@ -313,9 +313,10 @@ __global__ void __launch_bounds__(kT) k_heat_elem(HeatElemIn in, double* __restr
 
 // The left and right matrices on the free-node pattern: one warp per row walks the elements incident to
 // its node in element order (k_assemble of kernels.cu on scalars): lane b finds the column of the
-// element's node b and adds the pair's two entries to the row's sums in shared memory.
+// element's node b and adds the pair's two entries to the row's sums in shared memory; one lane after the
+// other when an element may name a node twice (REPEATS).
 constexpr int kHeatCols = 128;
-template <int NPE>
+template <int NPE, bool REPEATS>
 __global__ void __launch_bounds__(kT) k_heat_assemble(int32_t nb, int64_t ne, const int32_t* __restrict__ perm,
                                                       const int64_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc,
                                                       const int32_t* __restrict__ conn, const int32_t* __restrict__ inv,
@@ -358,18 +359,23 @@ __global__ void __launch_bounds__(kT) k_heat_assemble(int32_t nb, int64_t ne, co
             const int32_t j = J;
             const double lv = l, rv = r;
             if (q + 1 < q1) load(q + 1, pos, J, l, r);
+            int lo = nc;
             if (j >= 0) {
-                int lo = 0, hi = nc;
+                int hi = nc;
+                lo = 0;
                 while (lo < hi) {
                     const int mid = (lo + hi) >> 1;
                     if (rc[mid] < j) lo = mid + 1; else hi = mid;
                 }
-                if (lo < nc && rc[lo] == j) {
+                if (lo < nc && rc[lo] != j) lo = nc;
+            }
+            for (int b = 0; b < (REPEATS ? NPE : 1); ++b) {
+                if (lo < nc && (!REPEATS || lane == b)) {
                     sum[lo].x += lv;
                     sum[lo].y += rv;
                 }
+                __syncwarp();
             }
-            __syncwarp();
         }
         for (int t = lane; t < nc; t += 32) {
             A[rb + c0 + t] = sum[t].x;
@@ -1570,12 +1576,9 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
         counted();
         {
             const unsigned rows_grid = (unsigned)(((int64_t)nb * 32 + kT - 1) / kT);
-            if (npe == 4)
-                k_heat_assemble<4><<<rows_grid, kT, 0, st>>>(nb, ne, perm, inc_ptr, inc, conn, inv, pt.row_ptr, pt.col, left,
-                                                             right, A, R);
-            else
-                k_heat_assemble<10><<<rows_grid, kT, 0, st>>>(nb, ne, perm, inc_ptr, inc, conn, inv, pt.row_ptr, pt.col,
-                                                              left, right, A, R);
+            auto kernel = graph.repeats ? (npe == 4 ? k_heat_assemble<4, true> : k_heat_assemble<10, true>)
+                                        : (npe == 4 ? k_heat_assemble<4, false> : k_heat_assemble<10, false>);
+            kernel<<<rows_grid, kT, 0, st>>>(nb, ne, perm, inc_ptr, inc, conn, inv, pt.row_ptr, pt.col, left, right, A, R);
         }
         CK(cudaGetLastError());
         CK(cudaEventRecord(ev[6], st));
