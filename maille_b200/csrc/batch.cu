@@ -160,7 +160,9 @@ struct MailleGpuBatch {
     BatchShape shape() const { return BatchShape{R, cfg.Q, cfg.SUB}; }
     Pattern pattern() const { return Pattern{sym.nb, row_ptr, col, diag, tpos, fixmask}; }
     size_t vec_len() const { return ((size_t)sym.nb + 1) * R * 3; }
+    // no configuration: the next solve chooses one
     void release_config() {
+        cfg = BatchConfig{};
         for (BLayout* l : {&lk, &ll, &lu}) l->release();
         for (void* q : {Kv, Lv, Uv, D, (void*)K64, (void*)task_off, (void*)task_inst, (void*)inst_task,
                         (void*)uslot, (void*)inst_uslot, (void*)bwd_seq, (void*)part_k, (void*)part_u})
@@ -594,7 +596,9 @@ bool choose_config(MailleGpuBatch* b, Error& err, bool& tuned) {
     return true;
 }
 
-int32_t create_batch(const MailleBatchProblem* p, MailleGpuBatch** out) {
+// Throws DeviceMemoryFull when there was no room with the coarse correction; with IC(0) alone (coarse = false)
+// that is a CUDA error like any other.
+int32_t create_once(const MailleBatchProblem* p, MailleGpuBatch** out, bool coarse) {
     Error err{MAILLE_OK, ""};
     if (!out) return fail({MAILLE_INVALID_INPUT, "null handle pointer"});
     *out = nullptr;
@@ -760,7 +764,7 @@ int32_t create_batch(const MailleBatchProblem* p, MailleGpuBatch** out) {
             b->timing = dalloc<unsigned long long>(8);
             CK(cudaMemsetAsync(b->timing, 0, 8 * sizeof(unsigned long long), st));
         }
-        if (env_int("MAILLE_COARSE", 1) != 0) {
+        if (coarse && env_int("MAILLE_COARSE", 1) != 0) {
             std::vector<double> box(6 * (size_t)b->n_inst);
             std::vector<int64_t> rows(b->n_inst, 0);
             for (int32_t k = 0; k < b->n_inst; ++k)
@@ -779,11 +783,24 @@ int32_t create_batch(const MailleBatchProblem* p, MailleGpuBatch** out) {
         CK(cudaStreamSynchronize(st));
         b->h_ctrl.assign(8, 0);
         b->sym.ms = t1 - t0;
+    } catch (const DeviceMemoryFull& e) {
+        if (coarse) throw;
+        return fail({MAILLE_CUDA_ERROR, e.what});
     } catch (const CudaFailure& e) {
         return fail({MAILLE_CUDA_ERROR, e.what});
     }
     *out = b.release();
     return MAILLE_OK;
+}
+
+// A device without room for the coarse correction gets IC(0) alone.
+int32_t create_batch(const MailleBatchProblem* p, MailleGpuBatch** out) {
+    try {
+        return create_once(p, out, true);
+    } catch (const DeviceMemoryFull&) {
+    }
+    trim_device_memory(p->device);
+    return create_once(p, out, false);
 }
 
 int32_t solve_batch(MailleGpuBatch* b, const double* f, MailleBatchResult* res) {
@@ -799,7 +816,22 @@ int32_t solve_batch(MailleGpuBatch* b, const double* f, MailleBatchResult* res) 
         if (!b->cfg.valid()) {
             const double t0 = now_ms();
             b->f_cur = b->f0;
-            if (!choose_config(b, err, tuned)) return fail(err);
+            bool chosen = false;
+            try {
+                chosen = choose_config(b, err, tuned);
+            } catch (const DeviceMemoryFull&) {
+                if (!b->coarse.active()) throw;
+            }
+            if (!chosen && err.status == MAILLE_OK) {  // the coarse correction makes room for the layouts
+                CK(cudaStreamSynchronize(st));
+                b->release_config();
+                std::vector<void*> all;
+                b->coarse.gather(all);
+                device_free_all(all);
+                trim_device_memory(b->device);
+                chosen = choose_config(b, err, tuned);
+            }
+            if (!chosen) return fail(err);
             ms_tune = now_ms() - t0;
         }
         CK(cudaEventRecord(b->ev[0], st));

@@ -106,7 +106,7 @@ class Coarse {
     CoarseDev<double> dev64(int inst = 0) const { return dev<double>(inst); }
     template <typename T>
     CoarseBatchDev<T> batch() const;
-    // the device buffers, handed over to be freed together
+    // the device buffers, handed over to be freed together; the correction is inactive afterwards
     void gather(std::vector<void*>& out);
 
   private:

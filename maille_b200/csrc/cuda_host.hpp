@@ -24,6 +24,8 @@ struct NvtxRange {
 struct CudaFailure {
     std::string what;
 };
+// device_alloc found no room. What holds a coarse correction (coarse.cuh) gives it up and tries again.
+struct DeviceMemoryFull : CudaFailure {};
 
 #define CK(call)                                                                             \
     do {                                                                                     \

@@ -113,7 +113,7 @@ struct MailleGpuHandle {
     int precision = MAILLE_FP64;
     double tol = kDefaultTol;
     int32_t max_iter = kDefaultMaxIter;
-    double delta = 0.3;  // reliable update when the FP32 residual fell by this factor
+    double delta = 0.3, coarse_delta = kCoarseDelta;  // of the reliable updates, without and with the correction
     std::vector<uint8_t> h_fixed;
     bool any_imposed = false;
     // device: inputs (caller numbering)
@@ -173,8 +173,9 @@ struct MailleGpuHandle {
 
 namespace maille {
 
-// create: analysis, upload, element integration, assembly, IC(0) (FreeSystem::new + Pcg::new)
-int32_t handle_create(const MailleElasticProblem* p, MailleGpuHandle** out, MailleElasticResult* res);
+// create: analysis, upload, element integration, assembly, IC(0) (FreeSystem::new + Pcg::new).
+// coarse = false: IC(0) alone
+int32_t handle_create(const MailleElasticProblem* p, MailleGpuHandle** out, MailleElasticResult* res, bool coarse = true);
 // assembly of the element matrices in h->ke, IC(0) with the shift ladder, sliced copies
 int32_t handle_assemble_factor(MailleGpuHandle* h, Error& err);
 // b64 = f_cur - K_fc imposed at free DOFs (solver numbering); K_fc from h->ke

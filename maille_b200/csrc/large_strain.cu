@@ -535,7 +535,8 @@ int32_t ls_set_materials(MailleGpuLargeStrain* s, const double* young, const dou
     return MAILLE_OK;
 }
 
-int32_t ls_create(const MailleLargeStrainProblem* p, MailleGpuLargeStrain** out) {
+// Throws DeviceMemoryFull when there was no room beside the coarse correction.
+int32_t ls_create_once(const MailleLargeStrainProblem* p, MailleGpuLargeStrain** out, bool coarse) {
     if (!out) return ls_fail(MAILLE_INVALID_INPUT, "null handle pointer");
     *out = nullptr;
     if (!p) return ls_fail(MAILLE_INVALID_INPUT, "null problem");
@@ -560,7 +561,7 @@ int32_t ls_create(const MailleLargeStrainProblem* p, MailleGpuLargeStrain** out)
     ep.ordering = MAILLE_ORDER_AUTO;
     ep.device = p->device;
     auto s = std::make_unique<MailleGpuLargeStrain>();
-    int32_t status = maille::handle_create(&ep, &s->h, nullptr);
+    int32_t status = maille::handle_create(&ep, &s->h, nullptr, coarse);
     if (status != MAILLE_OK) return status;
     s->saved_imposed = s->h->imposed;
     s->increments = p->increments;
@@ -603,11 +604,23 @@ int32_t ls_create(const MailleLargeStrainProblem* p, MailleGpuLargeStrain** out)
         s->h_norms = static_cast<double*>(pinned_slot_alloc(4 * sizeof(double)));
         status = ls_set_materials(s.get(), nullptr, nullptr);
         if (status != MAILLE_OK) return status;
+    } catch (const maille::DeviceMemoryFull& e) {
+        if (s->h->coarse.active()) throw;
+        return ls_fail(MAILLE_CUDA_ERROR, e.what);
     } catch (const CudaFailure& e) {
         return ls_fail(MAILLE_CUDA_ERROR, e.what);
     }
     *out = s.release();
     return MAILLE_OK;
+}
+
+int32_t ls_create(const MailleLargeStrainProblem* p, MailleGpuLargeStrain** out) {
+    try {
+        return ls_create_once(p, out, true);
+    } catch (const maille::DeviceMemoryFull&) {
+    }
+    maille::trim_device_memory(p->device);
+    return ls_create_once(p, out, false);
 }
 
 }  // namespace

@@ -60,7 +60,12 @@ DevicePool& pool_of_current_device() {
 void* device_alloc(size_t bytes) {
     DevicePool& d = pool_of_current_device();
     void* p = nullptr;
-    CK(cudaMallocFromPoolAsync(&p, bytes, d.pool, d.stream));
+    const cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, d.pool, d.stream);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        throw DeviceMemoryFull{{"cudaMallocFromPoolAsync of " + std::to_string(bytes) + " bytes: " + cudaGetErrorString(e)}};
+    }
+    CK(e);
     CK(cudaStreamSynchronize(d.stream));
     return p;
 }

@@ -186,7 +186,7 @@ int32_t run_pcg(MailleGpuHandle* h, int32_t* iterations, int32_t* updates, doubl
     CK(cudaMemsetAsync(h->x64, 0, n4 * sizeof(double), st));
     CK(cudaMemcpyAsync(h->r64, h->b64, n4 * sizeof(double), cudaMemcpyDeviceToDevice, st));
     launch_norm2<double>(n4, h->b64, h->partials, h->dticket, &h->scal->bb, st);
-    launch_pcg_init(h->scal, h->tol, h->max_iter, mixed ? h->delta : 0.0, st);
+    launch_pcg_init(h->scal, h->tol, h->max_iter, !mixed ? 0.0 : h->coarse.active() ? h->coarse_delta : h->delta, st);
     if (mixed) {
         for (float* q : {h->x32, h->p32, h->ap32}) CK(cudaMemsetAsync(q, 0, n4 * sizeof(float), st));
         launch_cast(n4, h->b64, h->r32, st);
@@ -357,7 +357,9 @@ int env_int(const char* name, int dflt) {
     return e ? std::atoi(e) : dflt;
 }
 
-int32_t create_impl(const MailleElasticProblem* p, MailleGpuHandle** out, MailleElasticResult* res) {
+// Throws DeviceMemoryFull when there was no room with the coarse correction; with IC(0) alone (coarse = false)
+// that is a CUDA error like any other.
+int32_t create_once(const MailleElasticProblem* p, MailleGpuHandle** out, MailleElasticResult* res, bool coarse) {
     NvtxRange nvtx("maille create: analysis, upload, assembly, IC(0)");
     Error err{MAILLE_OK, ""};
     if (!out) return fail({MAILLE_INVALID_INPUT, "null handle pointer"});
@@ -382,7 +384,7 @@ int32_t create_impl(const MailleElasticProblem* p, MailleGpuHandle** out, Maille
     h->precision = p->precision;
     h->tol = p->rel_tol > 0 ? p->rel_tol : kDefaultTol;
     h->max_iter = p->max_iter > 0 ? p->max_iter : kDefaultMaxIter;
-    if (const char* e = std::getenv("MAILLE_RELIABLE_DELTA")) h->delta = std::atof(e);
+    if (const char* e = std::getenv("MAILLE_RELIABLE_DELTA")) h->delta = h->coarse_delta = std::atof(e);
     const int64_t n3 = 3 * p->n_nodes;
     h->h_fixed.assign(n3, 0);
     int64_t nfixed = 0;
@@ -529,13 +531,9 @@ int32_t create_impl(const MailleElasticProblem* p, MailleGpuHandle** out, Maille
         // the coarse correction, with the multicolour orderings (RCM stands for the reference's own
         // iteration counts). MAILLE_COARSE=0: IC(0) alone (a measurement knob)
         boxer.join();
-        if (ordering != MAILLE_ORDER_RCM && env_int("MAILLE_COARSE", 1) != 0)
+        if (coarse && ordering != MAILLE_ORDER_RCM && env_int("MAILLE_COARSE", 1) != 0)
             h->coarse.plan(3, is_mixed(h.get()), s.nb, s.blocks, h->coords, h->perm, h->fixmask, h->row_ptr, h->col,
                            nullptr, box, {(int64_t)s.nb}, st);
-        // with the correction an iteration takes the residual down by about 0.7: fewer reliable updates do
-        // (Tet10 40^3: 17, 10, 5 and 4 updates at 0.3, 0.1, 0.01 and 0.003, 68 iterations and the same
-        // true residual at each; the solve 31.2, 28.2, 26.0 and 25.5 ms)
-        if (h->coarse.active() && !std::getenv("MAILLE_RELIABLE_DELTA")) h->delta = kCoarseDelta;
         tmark("coarse plan");
         CK(cudaEventRecord(h->ev[11], st));  // pattern and layouts on the device
         // numeric buffers
@@ -632,11 +630,41 @@ int32_t create_impl(const MailleElasticProblem* p, MailleGpuHandle** out, Maille
             res->ms_assembly = elapsed(h->ev[1], h->ev[2]);
             res->ms_factor = elapsed(h->ev[2], h->ev[3]);
         }
+    } catch (const DeviceMemoryFull& e) {
+        if (coarse) throw;
+        return fail({MAILLE_CUDA_ERROR, e.what});
     } catch (const CudaFailure& e) {
         return fail({MAILLE_CUDA_ERROR, e.what});
     }
     *out = h.release();
     return MAILLE_OK;
+}
+
+// A device without room for the coarse correction gets IC(0) alone.
+int32_t create_impl(const MailleElasticProblem* p, MailleGpuHandle** out, MailleElasticResult* res, bool coarse = true) {
+    try {
+        return create_once(p, out, res, coarse);
+    } catch (const DeviceMemoryFull&) {
+    }
+    trim_device_memory(p->device);
+    return create_once(p, out, res, false);
+}
+
+// Device memory for a handle in use: the coarse correction makes room for it.
+template <typename T>
+T* late_alloc(MailleGpuHandle* h, size_t n) {
+    try {
+        return dalloc<T>(n);
+    } catch (const DeviceMemoryFull&) {
+        if (!h->coarse.active()) throw;
+    }
+    CK(cudaStreamSynchronize(h->st));
+    std::vector<void*> all;
+    h->coarse.gather(all);
+    device_free_all(all);
+    h->team_blocks = 0;
+    trim_device_memory(h->device);
+    return dalloc<T>(n);
 }
 
 const char* status_message(int32_t status, int32_t iters, double rel) {
@@ -708,10 +736,8 @@ int32_t solve_impl(MailleGpuHandle* h, const double* f, MailleElasticResult* res
         }
         if (h->bd.orphans) launch_orphan_reactions(h->n_nodes, h->inc_ptr, h->fixed, h->f_cur, h->react, st);
         const int ng = gauss_points(h->npe);
-        if (!h->gauss) {
-            h->gauss = dalloc<double>((size_t)h->n_elems * ng * 9);
-            h->vm = dalloc<double>((size_t)h->n_elems * ng);
-        }
+        if (!h->gauss) h->gauss = late_alloc<double>(h, (size_t)h->n_elems * ng * 9);
+        if (!h->vm) h->vm = late_alloc<double>(h, (size_t)h->n_elems * ng);
         ElemIn in{h->n_elems, h->coords, h->conn, h->young, h->poisson};
         launch_stresses(h->npe, in, h->u_full, h->gauss, h->vm, st);
         CK(cudaGetLastError());
@@ -784,10 +810,8 @@ int32_t backward_impl(MailleGpuHandle* h, const double* dJdu, double* dJdE, doub
         host_upload(h->y_full, dJdu, n3 * sizeof(double), st);
         if (!all_finite(h, h->y_full, n3)) return fail({MAILLE_INVALID_INPUT, "non-finite dJ/du"});
         launch_build_rhs(h->sym.nb, h->perm, h->fixmask, h->y_full, nullptr, h->b64, st);
-        if (!h->lambda_full) {
-            h->lambda_full = dalloc<double>(n3);
-            h->grad = dalloc<double>(h->n_elems);
-        }
+        if (!h->lambda_full) h->lambda_full = late_alloc<double>(h, n3);
+        if (!h->grad) h->grad = late_alloc<double>(h, h->n_elems);
         // K is symmetric: the same PCG and factor solve K lambda = g (u stays in u_full)
         int32_t iters = 0, outer = 0;
         double rel = 0.0;
@@ -816,8 +840,8 @@ int32_t backward_impl(MailleGpuHandle* h, const double* dJdu, double* dJdE, doub
 
 namespace maille {
 void set_last_error(const std::string& message) { g_last_error = message; }
-int32_t handle_create(const MailleElasticProblem* p, MailleGpuHandle** out, MailleElasticResult* res) {
-    return create_impl(p, out, res);
+int32_t handle_create(const MailleElasticProblem* p, MailleGpuHandle** out, MailleElasticResult* res, bool coarse) {
+    return create_impl(p, out, res, coarse);
 }
 int32_t handle_assemble_factor(MailleGpuHandle* h, Error& err) { return assemble_factor(h, err); }
 void handle_build_rhs(MailleGpuHandle* h) { build_rhs(h); }
@@ -962,10 +986,8 @@ int32_t maille_gpu_nodal_stresses(MailleGpuHandle* h, double* stress, double* vo
         return fail({MAILLE_INVALID_INPUT, "nodal stresses need the Gauss stresses of a solve"});
     try {
         CK(cudaSetDevice(h->device));
-        if (!h->node_stress) {
-            h->node_stress = dalloc<double>((size_t)h->n_nodes * 6);
-            h->node_vm = dalloc<double>((size_t)h->n_nodes);
-        }
+        if (!h->node_stress) h->node_stress = late_alloc<double>(h, (size_t)h->n_nodes * 6);
+        if (!h->node_vm) h->node_vm = late_alloc<double>(h, (size_t)h->n_nodes);
         launch_nodal_stresses(h->npe, h->n_nodes, h->inc_ptr, h->inc, h->gauss, h->node_stress,
                               h->node_vm, h->st);
         CK(cudaGetLastError());

@@ -1395,7 +1395,9 @@ int32_t check_thermal(const MailleThermalProblem* p, std::string& why) {
     return MAILLE_OK;
 }
 
-int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* res) {
+// Throws DeviceMemoryFull when there was no room with the coarse correction; with IC(0) alone (allow_coarse =
+// false) that is a CUDA error like any other.
+int32_t thermal_once(const MailleThermalProblem* p, MailleThermalResult* res, bool allow_coarse) {
     NvtxRange nvtx("maille thermal transient");
     std::string why;
     if (const int32_t s = check_thermal(p, why); s != MAILLE_OK) return th_fail(s, why);
@@ -1431,6 +1433,7 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
     cudaEvent_t ev[7] = {};
     DevBufs mem;
     Coarse coarse;
+    bool planned = false;  // the coarse correction took memory
     SideStream side;  // declared after the buffers its work uses: it is waited for before they go
     Slices sk, sl, su;
     sk.kind = SELL_FULL;
@@ -1565,9 +1568,11 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
         su.upload(pt, nb, st);
         boxer.join();
         if (const char* e = std::getenv("MAILLE_COARSE");
-            ordering != MAILLE_ORDER_RCM && !(e && std::atoi(e) == 0) && coarse_pays(p, box, nb))
+            allow_coarse && ordering != MAILLE_ORDER_RCM && !(e && std::atoi(e) == 0) && coarse_pays(p, box, nb)) {
+            planned = true;
             coarse.plan(1, p->precision == MAILLE_MIXED, nb, pt.blocks, coords, perm, nullptr, pt.row_ptr, pt.col, nullptr,
                         box, {(int64_t)nb}, st);
+        }
         // assembly of the left and right matrices on the free-node pattern
         double* A = mem.take(dalloc<double>((size_t)pt.blocks));
         double* R = mem.take(dalloc<double>((size_t)pt.blocks));
@@ -1864,10 +1869,22 @@ int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* re
                                                          ": iterations " + std::to_string(h_iters[s]) +
                                                          ", relative residual " + std::to_string(h_rel[s]));
         }
+    } catch (const DeviceMemoryFull& e) {
+        if (planned) throw;
+        return th_fail(MAILLE_CUDA_ERROR, e.what);
     } catch (const CudaFailure& e) {
         return th_fail(MAILLE_CUDA_ERROR, e.what);
     }
     return MAILLE_OK;
+}
+
+int32_t thermal_transient(const MailleThermalProblem* p, MailleThermalResult* res) {
+    try {
+        return thermal_once(p, res, true);
+    } catch (const DeviceMemoryFull&) {
+    }
+    trim_device_memory(p->device);
+    return thermal_once(p, res, false);
 }
 
 // nodal_source (assembly.rs:476-484) of a uniform source q over element e on its rule
