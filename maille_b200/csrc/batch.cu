@@ -651,9 +651,12 @@ int32_t create_once(const MailleBatchProblem* p, MailleGpuBatch** out, bool coar
         CK(cudaEventRecord(b->ev[4], st));
         // the packed mesh: node ids offset by the instance's first node
         std::vector<int32_t> conn32((size_t)b->n_elems * b->npe);
+        std::vector<uint8_t> used(b->n_nodes, 0);  // nodes that an element names
         for (int32_t k = 0; k < b->n_inst; ++k)
-            for (int64_t e = b->elem_off[k] * b->npe; e < b->elem_off[k + 1] * b->npe; ++e)
+            for (int64_t e = b->elem_off[k] * b->npe; e < b->elem_off[k + 1] * b->npe; ++e) {
                 conn32[e] = (int32_t)(p->conn[e] + b->node_off[k]);
+                used[conn32[e]] = 1;
+            }
         b->coords = dupload(p->coords, n3, st);
         b->conn = dupload(conn32.data(), conn32.size(), st);
         b->young = dupload(p->young, b->n_elems, st);
@@ -768,7 +771,7 @@ int32_t create_once(const MailleBatchProblem* p, MailleGpuBatch** out, bool coar
             std::vector<double> box(6 * (size_t)b->n_inst);
             std::vector<int64_t> rows(b->n_inst, 0);
             for (int32_t k = 0; k < b->n_inst; ++k)
-                coarse_box(p->coords, b->node_off[k], b->node_off[k + 1], box.data() + 6 * (size_t)k);
+                coarse_box(p->coords, used.data(), b->node_off[k], b->node_off[k + 1], box.data() + 6 * (size_t)k);
             for (int32_t k : b->row_inst) rows[k]++;
             struct DevTemp {
                 void* p = nullptr;

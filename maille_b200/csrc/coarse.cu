@@ -18,6 +18,7 @@
 #include <atomic>
 #include <climits>
 #include <cmath>
+#include <cstring>
 
 #include <cub/cub.cuh>
 
@@ -48,6 +49,29 @@ inline void counted(int n = 1) { g_kernel_launches.fetch_add(n, std::memory_orde
 
 #define GRID_STRIDE(t, n) \
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < (n); t += (int64_t)gridDim.x * blockDim.x)
+
+// ext: the largest keys of -x, -y, -z, x, y, z over the nodes of an element, in keys (an order-preserving
+// image of the doubles, complemented for the minima; all zero before)
+__global__ void __launch_bounds__(kT) k_box(int64_t n, const double* __restrict__ xyz, const int64_t* __restrict__ inc_ptr,
+                                            unsigned long long* __restrict__ ext) {
+    unsigned long long m[6] = {};
+    GRID_STRIDE(v, n) {
+        if (inc_ptr[v] == inc_ptr[v + 1]) continue;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const unsigned long long bits = (unsigned long long)__double_as_longlong(xyz[3 * v + a]);
+            const unsigned long long key = bits >> 63 ? ~bits : bits | (1ull << 63);
+            m[a] = max(m[a], ~key);
+            m[3 + a] = max(m[3 + a], key);
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < 6; ++a) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m[a] = max(m[a], __shfl_xor_sync(0xffffffffu, m[a], o));
+        if ((threadIdx.x & 31) == 0) atomicMax(&ext[a], m[a]);
+    }
+}
 
 // cell, fractions and code of every row
 __global__ void k_place(int32_t nb, const double* __restrict__ xyz, const int32_t* __restrict__ perm,
@@ -533,16 +557,33 @@ struct Temp {
 
 }  // namespace
 
-void coarse_box(const double* xyz, int64_t n0, int64_t n1, double box[6]) {
+void coarse_box(const double* xyz, const uint8_t* used, int64_t n0, int64_t n1, double box[6]) {
     for (int a = 0; a < 3; ++a) {
         box[a] = INFINITY;
         box[3 + a] = -INFINITY;
     }
     for (int64_t v = n0; v < n1; ++v)
-        for (int a = 0; a < 3; ++a) {
+        for (int a = 0; a < 3 && used[v]; ++a) {
             box[a] = std::min(box[a], xyz[3 * v + a]);
             box[3 + a] = std::max(box[3 + a], xyz[3 * v + a]);
         }
+}
+
+void coarse_box(const double* xyz, const int64_t* inc_ptr, int64_t n_nodes, cudaStream_t st, double box[6]) {
+    Temp ext(6 * sizeof(unsigned long long));
+    unsigned long long h[6];
+    CK(cudaMemsetAsync(ext.p, 0, sizeof(h), st));
+    const unsigned blocks = std::min<unsigned>(grid_of(n_nodes), 4 * (unsigned)device_sms());
+    k_box<<<blocks, kT, 0, st>>>(n_nodes, xyz, inc_ptr, ext.as<unsigned long long>());
+    CK(cudaGetLastError());
+    counted();
+    CK(cudaMemcpyAsync(h, ext.p, sizeof(h), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    for (int a = 0; a < 6; ++a) {
+        const unsigned long long key = a < 3 ? ~h[a] : h[a];
+        const unsigned long long bits = key >> 63 ? key & ~(1ull << 63) : ~key;
+        std::memcpy(&box[a], &bits, sizeof(double));
+    }
 }
 
 // About cubic cells; as many coarse nodes as a cube of 3 rows^0.44 cells has, at most 11^3 (elastic).

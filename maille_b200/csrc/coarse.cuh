@@ -138,8 +138,11 @@ constexpr uint32_t kCoarseBase = (1u << 28) - 1u;
 // Cell order: the row in the low 29 bits, fixed mask above.
 constexpr uint32_t kCoarseRow = (1u << 29) - 1u;
 
-// Host bounding box of the nodes [n0, n1) of xyz into box[6] (min x, y, z, max x, y, z).
-void coarse_box(const double* xyz, int64_t n0, int64_t n1, double box[6]);
+// Bounding box (min x, y, z, max x, y, z) of the nodes that an element names: a node of none, however far, would
+// only take cells from the part. used: such nodes among [n0, n1), in host memory. inc_ptr: their incidence, on
+// the device, enqueued on st and waited for.
+void coarse_box(const double* xyz, const uint8_t* used, int64_t n0, int64_t n1, double box[6]);
+void coarse_box(const double* xyz, const int64_t* inc_ptr, int64_t n_nodes, cudaStream_t st, double box[6]);
 // Cells per axis for `rows` rows of `dof` unknowns in the box.
 void coarse_cells(int dof, const double box[6], int64_t rows, int32_t k[3]);
 

@@ -402,14 +402,6 @@ int32_t create_once(const MailleElasticProblem* p, MailleGpuHandle** out, Maille
     // same permutation: the same algorithms on the same graph).
     const bool host_ordering = env_int("MAILLE_HOST_ORDERING", 0) != 0;
     const int ordering = p->ordering == MAILLE_ORDER_AUTO ? kOrderIndex : p->ordering;
-    std::vector<double> box(6, 0.0);  // of the nodes, for the coarse grid
-    std::thread boxer([&] { coarse_box(p->coords, 0, p->n_nodes, box.data()); });
-    struct Joiner {
-        std::thread& t;
-        ~Joiner() {
-            if (t.joinable()) t.join();
-        }
-    } joiner{boxer};
     // MAILLE_SETUP_TIMING: wall time of the device-side set-up steps (stream synchronised)
     const bool stage_timing = std::getenv("MAILLE_SETUP_TIMING") != nullptr;
     double t_mark = now_ms();
@@ -530,10 +522,12 @@ int32_t create_once(const MailleElasticProblem* p, MailleGpuHandle** out, Maille
         }
         // the coarse correction, with the multicolour orderings (RCM stands for the reference's own
         // iteration counts). MAILLE_COARSE=0: IC(0) alone (a measurement knob)
-        boxer.join();
-        if (coarse && ordering != MAILLE_ORDER_RCM && env_int("MAILLE_COARSE", 1) != 0)
+        if (coarse && ordering != MAILLE_ORDER_RCM && env_int("MAILLE_COARSE", 1) != 0) {
+            std::vector<double> box(6);
+            coarse_box(h->coords, h->inc_ptr, p->n_nodes, st, box.data());
             h->coarse.plan(3, is_mixed(h.get()), s.nb, s.blocks, h->coords, h->perm, h->fixmask, h->row_ptr, h->col,
                            nullptr, box, {(int64_t)s.nb}, st);
+        }
         tmark("coarse plan");
         CK(cudaEventRecord(h->ev[11], st));  // pattern and layouts on the device
         // numeric buffers

@@ -1420,15 +1420,6 @@ int32_t thermal_once(const MailleThermalProblem* p, MailleThermalResult* res, bo
     const int ordering = p->ordering == MAILLE_ORDER_AUTO ? kOrderIndex : p->ordering;
     const char* host_env = std::getenv("MAILLE_HOST_ORDERING");
     const bool host_ordering = host_env && std::atoi(host_env) != 0;
-    std::vector<double> box(6, 0.0);  // of the nodes, for the coarse grid
-    std::thread boxer([&] { coarse_box(p->coords, 0, n, box.data()); });
-    struct Joiner {
-        std::thread& t;
-        ~Joiner() {
-            if (t.joinable()) t.join();
-        }
-    } joiner{boxer};
-
     cudaStream_t st = nullptr;
     cudaEvent_t ev[7] = {};
     DevBufs mem;
@@ -1566,7 +1557,8 @@ int32_t thermal_once(const MailleThermalProblem* p, MailleThermalResult* res, bo
         sk.upload(pt, nb, st);
         sl.upload(pt, nb, st);
         su.upload(pt, nb, st);
-        boxer.join();
+        std::vector<double> box(6);
+        coarse_box(coords, inc_ptr, n, st, box.data());
         if (const char* e = std::getenv("MAILLE_COARSE");
             allow_coarse && ordering != MAILLE_ORDER_RCM && !(e && std::atoi(e) == 0) && coarse_pays(p, box, nb)) {
             planned = true;
