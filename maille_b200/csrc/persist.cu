@@ -292,6 +292,12 @@ __global__ void k_wait_selftest(const float* z, unsigned int epoch, unsigned int
     if ((threadIdx.x & 31) == 0) *timed_out = ok ? 0 : 1;
 }
 
+// Self-test of the coarse team's barrier: one block arrives, `target` blocks are awaited with at most `limit`
+// reads; *timed_out = 1 when the wait ran out (as it must for a target of 2).
+__global__ void k_barrier_selftest(int32_t* arrived, int32_t target, unsigned int limit, int32_t* timed_out) {
+    coarse_team_barrier(arrived, target, timed_out, limit);
+}
+
 // publishes row `row` of the sweep output for sweep `epoch`
 __device__ __forceinline__ void publish_row(float* z, int32_t row, float a, float b, float d, unsigned int epoch) {
     st_rec(z, row, a, b, d, epoch);
@@ -1007,18 +1013,24 @@ void* pick(int lprk, int warps) {
 
 }  // namespace
 
-// Runs k_wait_selftest on 4 FP32 records whose tags are `tags` for `epoch` with at most `limit`
-// rounds; *timed_out tells whether the wait ran out. Throws CudaFailure on a CUDA error.
-void wait_selftest(const unsigned int tags[4], unsigned int epoch, unsigned int limit, int32_t* timed_out) {
+// Runs k_wait_selftest on 4 FP32 records whose tags are `tags` for `epoch` and k_barrier_selftest for `blocks`
+// blocks, each with at most `limit` rounds; *timed_out: 1 when both waits ran out, 0 when neither did, 2
+// when they differ. Throws CudaFailure on a CUDA error.
+void wait_selftest(const unsigned int tags[4], unsigned int epoch, int32_t blocks, unsigned int limit,
+                   int32_t* timed_out) {
     float host[16] = {};
     for (int j = 0; j < 4; ++j) std::memcpy(&host[4 * j + 3], &tags[j], sizeof(unsigned int));
     float* z = dalloc<float>(16);
-    int32_t* flag = dalloc<int32_t>(1);
+    int32_t* flag = dalloc<int32_t>(3);  // the records' verdict, the barrier's, its arrivals
     CK(cudaMemcpy(z, host, sizeof(host), cudaMemcpyHostToDevice));
-    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+    CK(cudaMemset(flag, 0, 3 * sizeof(int32_t)));
+    g_kernel_launches.fetch_add(2, std::memory_order_relaxed);
     k_wait_selftest<<<1, 32>>>(z, epoch, limit, flag);
+    k_barrier_selftest<<<1, 64>>>(flag + 2, blocks, limit, flag + 1);
     CK(cudaGetLastError());
-    CK(cudaMemcpy(timed_out, flag, sizeof(int32_t), cudaMemcpyDeviceToHost));
+    int32_t h[2];
+    CK(cudaMemcpy(h, flag, sizeof(h), cudaMemcpyDeviceToHost));
+    *timed_out = h[0] == h[1] ? h[0] : 2;
     dfree(z);
     dfree(flag);
 }

@@ -1001,7 +1001,7 @@ int32_t maille_gpu_wait_selftest(int32_t device, int32_t stale, int32_t* timed_o
         CK(cudaSetDevice(device));
         const unsigned int epoch = 7;
         const unsigned int tags[4] = {epoch, epoch, stale ? epoch - 1 : epoch, epoch + 1};
-        wait_selftest(tags, epoch, 4096, timed_out);
+        wait_selftest(tags, epoch, stale ? 2 : 1, 4096, timed_out);
     } catch (const CudaFailure& e) {
         return fail({MAILLE_CUDA_ERROR, e.what});
     }

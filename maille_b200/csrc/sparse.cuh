@@ -90,9 +90,11 @@ struct PcgArgs {
 };
 template <typename T, bool MIXED>
 int pcg_persistent_grid(int lprk, int warps);
-// Self-test of the sweeps' bounded wait (persist.cu): awaits 4 FP32 records with tags `tags` for
-// `epoch` within `limit` rounds; *timed_out = 1 when the wait ran out. Throws CudaFailure.
-void wait_selftest(const unsigned int tags[4], unsigned int epoch, unsigned int limit, int32_t* timed_out);
+// Self-test of the PCG's bounded waits (persist.cu): awaits 4 FP32 records with tags `tags` for `epoch` and, in
+// one block, the coarse team's barrier of `blocks` blocks, within `limit` rounds; *timed_out = 1 when both
+// waits ran out, 0 when neither did, 2 when they differ. Throws CudaFailure.
+void wait_selftest(const unsigned int tags[4], unsigned int epoch, int32_t blocks, unsigned int limit,
+                   int32_t* timed_out);
 template <typename T, bool MIXED>
 cudaError_t launch_pcg_persistent(const PcgArgs<T>& a, int grid, int warps, bool init, cudaStream_t st);
 

@@ -34,3 +34,13 @@ def test_a_wait_on_a_record_nothing_writes_times_out_and_the_context_stays_usabl
     m.with_solver(mb.SolverKind.ITERATIVE)
     f = m.solve()
     assert np.all(np.isfinite(f.displacements)) and f.info["iterations"] > 0
+
+
+def test_the_barrier_of_the_coarse_team_gives_up_with_the_records(gpu):
+    # the same call waits at the barrier of the blocks that form the coarse correction's team, for a block
+    # that never arrives: 1 says that both waits ran out, 0 that neither did (2: one of them)
+    L = _lib.load()
+    before = L.maille_gpu_kernel_launches()
+    assert selftest(L, 1) == 1
+    assert L.maille_gpu_kernel_launches() == before + 2
+    assert selftest(L, 0) == 0
