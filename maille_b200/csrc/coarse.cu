@@ -8,9 +8,10 @@
 //    corner pairs (a, b), two pairs a lane, into the chunk's own slots;
 //  * k_pair_sums, k_dense: every entry of E sums the slots of the cell pairs that touch it, in order;
 //  * k_panel, k_trail: E^-1 by block symmetric sweeps (Beaton's sweep operator, 64 unknowns a
-//    step, lower tiles only): m^3 flops, no pivoting (E is positive definite). An unknown whose
-//    pivot falls to 1e-12 of its own diagonal (a coarse node without support, or dependent on
-//    others) leaves the space: its row and column of the inverse are zero;
+//    step, lower tiles only), every update a square by the tile's Cholesky factor: m^3 flops, no pivoting
+//    (E with its ridge, kRidge64, is positive definite).
+//    An unknown whose pivot falls below a tenth of the ridge (a coarse node without support) leaves the
+//    space: its row and column of the inverse are zero;
 //  * k_mirror: -A, both triangles, in the PCG's precision.
 // No floating-point atomics: repeated set-ups give the same bits.
 
@@ -38,7 +39,24 @@ constexpr int kRowChunk = 256;   // rows a restriction chunk, one row a lane at 
 constexpr int kBatchChunk = 64;  // rows a chunk of a batch, whose warp takes them one after the other
 constexpr int kPairChunk = 256;  // blocks a Galerkin chunk
 constexpr int kPairWarps = 4;    // warps a block of k_pairs
-constexpr double kDrop = 1e-12;  // pivot test, relative to the unknown's diagonal of E
+// E + ridge diag(E) is what is inverted. Where a part has fewer layers of nodes than the grid has lines, or
+// touches a cell with a corner only, hats depend on one another and E is singular; its null pivots are
+// rounding times the square of the multipliers (up to 1e-9), no threshold tells them from soft modes (a bar
+// of 331:1: 1e-10), and one taken for a pivot made the correction indefinite: a bent strip of 4x1x19
+// cells (60 of 180 unknowns dependent) did not converge in 10000 iterations where IC(0) alone takes 105, and
+// takes 26 with the ridge. 1e-9 stays far above what the rounding leaves of it and below every soft mode
+// that matters (bars of 120:1 and 331:1 take 151 and 509 iterations with and without it). Rounded to FP32 an
+// inverse is definite only while its largest entries stay below 1 / 6e-8 of its smallest modes': 1e-5
+// (3x7x6 cells of 0.44:1:0.37, mixed, IC(0) alone / without / with: 1013 / not in 10000 / 100 iterations; bars
+// of 10:1, plates, shells and cubes the same). Over 260 random parts (1 to 64 cells a side, graded, bent,
+// twisted, moduli over three decades) the correction with both converges wherever IC(0) alone does, in
+// 0.38 (FP64) and 0.34 (mixed) of its iterations, never in more than 1.3 of them.
+constexpr double kRidge64 = 1e-9, kRidge32 = 1e-5;
+constexpr double kDrop = 0.1;  // a pivot below this part of its ridge is rounding
+// A row this close to a grid plane, relative to the cell, lies on it: else the hats of a plane that nodes miss
+// by a rounding carry weights of 1e-16, depend on the others, and cost the FP32 inverse its accuracy (a
+// graded plate of one cell clamped on its face: 784 iterations against 41).
+constexpr double kSnap = 1e-9;
 constexpr int64_t kMinRows = 128;
 
 inline unsigned grid_of(int64_t n) {
@@ -87,6 +105,8 @@ __global__ void k_place(int32_t nb, const double* __restrict__ xyz, const int32_
             const double t = fmin(fmax((xyz[3 * (int64_t)perm[i] + a] - g.lo[a]) * g.inv_h[a], 0.0), (double)g.k[a]);
             c[a] = min((int32_t)t, g.k[a] - 1);
             f[a] = t - (double)c[a];
+            if (f[a] < kSnap) f[a] = 0.0;
+            if (f[a] > 1.0 - kSnap) f[a] = 1.0;
         }
         const uint32_t base = (uint32_t)(c[0] + (g.k[0] + 1) * (c[1] + (g.k[1] + 1) * c[2]));
         const uint32_t mask = fixmask ? (uint32_t)fixmask[i] & 7u : 0u;
@@ -244,13 +264,13 @@ __global__ void k_pair_sums(int32_t nseg, const int32_t* __restrict__ schunk_ptr
     }
 }
 
-// A (lower tiles, zero before) = E with ones on the padded diagonal, diag = its diagonal: one thread per
+// A (lower tiles, zero before) = E with its ridge and ones on the padded diagonal, diag = its diagonal: one thread per
 // coarse node u, node v <= u within reach (`span`: cells that a block of K reaches across at most)
 // and entry of their block.
 template <int DOF>
 __global__ void k_dense(const CoarseGrid* __restrict__ grids, const int32_t* __restrict__ table,
                         const int32_t* __restrict__ schunk_ptr, const double* __restrict__ part, double* __restrict__ A,
-                        double* __restrict__ diag, int64_t diag_stride) {
+                        double* __restrict__ diag, int64_t diag_stride, double ridge) {
     constexpr int D2 = DOF * DOF;
     const CoarseGrid g = grids[blockIdx.y];
     const int32_t nx = g.k[0] + 1, ny = g.k[1] + 1, nz = g.k[2] + 1, nn = nx * ny * nz;
@@ -287,8 +307,8 @@ __global__ void k_dense(const CoarseGrid* __restrict__ grids, const int32_t* __r
             }
         }
         const int64_t r = (int64_t)DOF * u + q / DOF, c = (int64_t)DOF * v + q % DOF;
+        if (r == c) di[r] = s *= 1.0 + ridge;
         Ai[r * g.ld + c] = s;
-        if (r == c) di[r] = s;
     }
     // the padding of the last tiles: an identity
     GRID_STRIDE(t, g.ld - g.m) {
@@ -297,105 +317,151 @@ __global__ void k_dense(const CoarseGrid* __restrict__ grids, const int32_t* __r
     }
 }
 
-// Sweeps the 64 x 64 tile held by 256 threads, 4 x 4 entries a[][] each (thread (ty, tx): rows 4 ty ..,
-// columns 4 tx ..): a = -tile^-1. Four pivots at a time: the thread on the diagonal sweeps its own 4 x 4
-// entries, its row of threads broadcasts its rows through shared memory, the block forms their
-// product with the 4 x 4 inverse, and every thread takes the rank-4 update. 16 such steps instead of
-// 64 pivots: one pivot at a time took 105 us a tile, with a division, a load of its limit and a
-// barrier on every pivot's path. An unknown whose pivot falls to kDrop of its diagonal of E is
-// dropped: a zero row and column.
-struct SweepMem {
-    double rows[4][kTile], u[kTile][4], P[16], limit[kTile];
+// The inverse Cholesky factor X = L^-1 of the 64 x 64 tile L L^T held by 256 threads, 4 x 4 entries a[][] each
+// (thread (ty, tx): rows 4 ty .., columns 4 tx ..); x[][] the same entries of X. Four pivots at a time: the
+// thread on the diagonal factors its own 4 x 4 entries, its row of threads broadcasts its rows through
+// shared memory and takes its rows of X, the block forms the columns of L below, and the threads below
+// take the rank-4 updates of the tile and of X. 16 such steps instead of 64 pivots: one pivot at a
+// time took 105 us a tile, with a division, a load of its limit and a barrier on every pivot's path. An
+// unknown whose pivot falls to its limit (kDrop) is dropped: a zero row and column of X.
+struct TileMem {
+    double rows[4][kTile], x[4][kTile], u[kTile][4], M[16], limit[kTile];
 };
-__device__ __forceinline__ void sweep_tile(double a[4][4], SweepMem& m) {
+__device__ __forceinline__ void factor_tile(double a[4][4], double x[4][4], TileMem& m) {
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int p = 0; p < 4; ++p) x[q][p] = tx == ty && q == p ? 1.0 : 0.0;
     for (int b = 0; b < kTile / 4; ++b) {
         if (ty == b) {
 #pragma unroll
             for (int q = 0; q < 4; ++q)
 #pragma unroll
                 for (int p = 0; p < 4; ++p) m.rows[q][4 * tx + p] = a[q][p];
-            if (tx == b) {
+            if (tx == b) {  // M = L_bb^-1
+                double r[4];
 #pragma unroll
                 for (int t = 0; t < 4; ++t) {
-                    const double d = a[t][t], inv = d > m.limit[4 * b + t] ? 1.0 / d : 0.0;
-                    double c[4];
+                    r[t] = a[t][t] > m.limit[4 * b + t] ? rsqrt(a[t][t]) : 0.0;
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) c[q] = a[q][t] * inv;
+                    for (int q = t + 1; q < 4; ++q) a[q][t] *= r[t];
 #pragma unroll
-                    for (int q = 0; q < 4; ++q)
+                    for (int q = t + 1; q < 4; ++q)
 #pragma unroll
-                        for (int p = 0; p < 4; ++p)
-                            if (q != t && p != t) a[q][p] -= c[q] * a[t][p];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        if (q != t) a[q][t] = a[t][q] = c[q];
-                    a[t][t] = -inv;
+                        for (int p = t + 1; p <= q; ++p) a[q][p] -= a[q][t] * a[p][t];
                 }
 #pragma unroll
-                for (int q = 0; q < 4; ++q)
+                for (int t = 0; t < 4; ++t) {
+                    double c[4] = {0.0, 0.0, 0.0, 0.0};
+                    c[t] = r[t];
 #pragma unroll
-                    for (int p = 0; p < 4; ++p) m.P[4 * q + p] = a[q][p];
+                    for (int q = t + 1; q < 4; ++q) {
+                        double d = 0.0;
+#pragma unroll
+                        for (int k = t; k < q; ++k) d -= a[q][k] * c[k];
+                        c[q] = d * r[q];
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) m.M[4 * q + t] = c[q];
+                }
             }
         }
         __syncthreads();
-        {  // u = (the pivot columns of every row) tile_bb^-1, one entry a thread
-            const int r = tid >> 2, p = tid & 3;
-            double s = 0.0;
+        if (ty == b && tx <= b)  // X is lower triangular
 #pragma unroll
-            for (int t = 0; t < 4; ++t) s -= m.rows[t][r] * m.P[4 * t + p];
-            m.u[r][p] = s;
+            for (int p = 0; p < 4; ++p) {
+                const double v[4] = {x[0][p], x[1][p], x[2][p], x[3][p]};
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    double d = 0.0;
+#pragma unroll
+                    for (int k = 0; k <= q; ++k) d += m.M[4 * q + k] * v[k];
+                    m.x[q][4 * tx + p] = x[q][p] = d;
+                }
+            }
+        {  // u = the columns of L, one entry a thread
+            const int r = tid >> 2, t = tid & 3;
+            double d = 0.0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) d += m.rows[k][r] * m.M[4 * t + k];
+            m.u[r][t] = d;
         }
         __syncthreads();
-        if (tx == b) {
-            if (ty != b)
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) a[q][p] = m.u[4 * ty + q][p];
-        } else if (ty == b) {  // the pivot rows: the transposed columns
+        if (ty > b) {
+            double l[4][4];
 #pragma unroll
             for (int q = 0; q < 4; ++q)
 #pragma unroll
-                for (int p = 0; p < 4; ++p) a[q][p] = m.u[4 * tx + p][q];
-        } else {
+                for (int t = 0; t < 4; ++t) l[q][t] = m.u[4 * ty + q][t];
+            if (tx > b) {
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                double w[4], u[4];
+                for (int p = 0; p < 4; ++p)
 #pragma unroll
-                for (int p = 0; p < 4; ++p) {
-                    w[p] = m.rows[t][4 * tx + p];
-                    u[p] = m.u[4 * ty + p][t];
-                }
+                    for (int t = 0; t < 4; ++t) {
+                        const double w = m.u[4 * tx + p][t];
 #pragma unroll
-                for (int q = 0; q < 4; ++q)
+                        for (int q = 0; q < 4; ++q) a[q][p] -= l[q][t] * w;
+                    }
+            } else {
 #pragma unroll
-                    for (int p = 0; p < 4; ++p) a[q][p] -= u[q] * w[p];
+                for (int p = 0; p < 4; ++p)
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) {
+                        const double w = m.x[t][4 * tx + p];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) x[q][p] -= l[q][t] * w;
+                    }
             }
         }
-        __syncthreads();
     }
 }
 
-// Step s of the sweeps, panel: every block sweeps the pivot tile A_ss into -A_ss^-1 (each for itself: a
-// launch of its own would cost as much, and a block of k_trail that did it slowed that kernel by its
-// registers); block i then forms W_i = A_is and V_i = W_i A_ss^-1 (both transposed in the panels:
-// unknown-major), block s leaves the pivot in piv.
+// v[q][p] = sum_t P[t][4 ty + q] W[t][r_p], t0 <= t < t1, for this thread's columns 4 ty .. and rows 2 tx,
+// 2 tx + 1, 32 + ..
 constexpr int kPanelStride = kTile + 2;
+__device__ __forceinline__ void panel_product(const double* P, const double* W, int t0, int t1, int tx, int ty,
+                                              double v[4][4]) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int p = 0; p < 4; ++p) v[q][p] = 0.0;
+#pragma unroll 4
+    for (int t = t0; t < t1; ++t) {
+        const double2 w0 = *reinterpret_cast<const double2*>(W + t * kPanelStride + 2 * tx);
+        const double2 w1 = *reinterpret_cast<const double2*>(W + t * kPanelStride + 32 + 2 * tx);
+        const double2 c0 = *reinterpret_cast<const double2*>(P + t * kPanelStride + 4 * ty);
+        const double2 c1 = *reinterpret_cast<const double2*>(P + t * kPanelStride + 4 * ty + 2);
+        const double w[4] = {w0.x, w0.y, w1.x, w1.y}, c[4] = {c0.x, c0.y, c1.x, c1.y};
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int p = 0; p < 4; ++p) v[q][p] += c[q] * w[p];
+    }
+}
+
+// Step s of the sweeps, panel: every block factors the pivot tile A_ss = L L^T (each for itself: a launch of
+// its own would cost as much, and a block of k_trail that did it slowed that kernel by its registers);
+// block i then forms W_i = A_is L^-T and V_i = W_i L^-1 = A_is A_ss^-1 (both transposed in the panels:
+// unknown-major), block s leaves A_ss^-1 = L^-T L^-1 in piv. The update A_ij -= W_i W_j^T is a square: with
+// the tile's explicit inverse, A_ij -= A_is (A_ss^-1 A_sj), the inverse's own rounding, eps / pivot^2,
+// made a matrix of dependent hats indefinite (a graded part of 2x51x6 cells: eigenvalues of P X P^T K from
+// -4200 to 4300).
 __global__ void __launch_bounds__(kT) k_panel(int s, const CoarseGrid* __restrict__ grids, const double* __restrict__ A,
-                                              const double* __restrict__ diag, int64_t diag_stride,
+                                              const double* __restrict__ diag, int64_t diag_stride, double ridge,
                                               double* __restrict__ W, double* __restrict__ V, double* __restrict__ piv) {
     extern __shared__ __align__(16) double sm[];
-    __shared__ SweepMem mem;
-    double *P = sm, *Wt = sm + kTile * kPanelStride;  // P[t][c]; Wt[t][r] = W_i[r][t]
+    __shared__ TileMem mem;
+    // X[t][c] = (L^-1)[t][c], Xt its transpose, Wt[t][r] = A_is[r][t], then W_i
+    double *X = sm, *Xt = sm + kTile * kPanelStride, *Wt = sm + 2 * kTile * kPanelStride;
     const CoarseGrid& g = grids[blockIdx.y];
     const int tiles = g.ld / kTile, i = blockIdx.x;
     if (s >= tiles || i >= tiles) return;
     const double* Ai = A + g.dense0;
     const int64_t ld = g.ld, o = (int64_t)s * kTile, oi = (int64_t)i * kTile;
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    if (tid < kTile) mem.limit[tid] = kDrop * diag[blockIdx.y * diag_stride + o + tid];
-    double a[4][4];
+    if (tid < kTile) mem.limit[tid] = kDrop * ridge * diag[blockIdx.y * diag_stride + o + tid];
+    double a[4][4], x[4][4];
 #pragma unroll
     for (int q = 0; q < 4; ++q)
 #pragma unroll
@@ -410,45 +476,42 @@ __global__ void __launch_bounds__(kT) k_panel(int s, const CoarseGrid* __restric
             else Wt[h * kPanelStride + l] = Ai[(o + h) * ld + oi + l];
         }
     __syncthreads();
-    sweep_tile(a, mem);
+    factor_tile(a, x, mem);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            X[(4 * ty + q) * kPanelStride + 4 * tx + p] = x[q][p];
+            Xt[(4 * tx + p) * kPanelStride + 4 * ty + q] = x[q][p];
+        }
+    __syncthreads();
+    double v[4][4];
     if (i == s) {
+        panel_product(X, X, 4 * ty, kTile, tx, ty, v);
         double* out = piv + (int64_t)blockIdx.y * kTile * kTile;
 #pragma unroll
         for (int q = 0; q < 4; ++q)
 #pragma unroll
-            for (int p = 0; p < 4; ++p) out[(4 * ty + q) * kTile + 4 * tx + p] = a[q][p];
+            for (int p = 0; p < 4; ++p) out[(4 * ty + q) * kTile + 2 * tx + 16 * (p & 2) + (p & 1)] = v[q][p];
         return;
     }
+    auto store = [&](double* to, int64_t stride) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int p = 0; p < 4; ++p) P[(4 * ty + q) * kPanelStride + 4 * tx + p] = a[q][p];
+        for (int q = 0; q < 4; ++q) {
+            *reinterpret_cast<double2*>(to + (4 * ty + q) * stride + 2 * tx) = make_double2(v[q][0], v[q][1]);
+            *reinterpret_cast<double2*>(to + (4 * ty + q) * stride + 32 + 2 * tx) = make_double2(v[q][2], v[q][3]);
+        }
+    };
+    panel_product(Xt, Wt, 0, 4 * ty + 4, tx, ty, v);  // X is lower triangular
+    store(W + g.y0 * kTile + oi, ld);
     __syncthreads();
-    // this thread's columns t = 4 ty .. of V, rows 2 tx, 2 tx + 1, 32 + ..
-    double v[4][4] = {};
-#pragma unroll 4
-    for (int t = 0; t < kTile; ++t) {
-        const double2 w0 = *reinterpret_cast<const double2*>(Wt + t * kPanelStride + 2 * tx);
-        const double2 w1 = *reinterpret_cast<const double2*>(Wt + t * kPanelStride + 32 + 2 * tx);
-        const double2 c0 = *reinterpret_cast<const double2*>(P + t * kPanelStride + 4 * ty);
-        const double2 c1 = *reinterpret_cast<const double2*>(P + t * kPanelStride + 4 * ty + 2);
-        const double w[4] = {w0.x, w0.y, w1.x, w1.y}, c[4] = {c0.x, c0.y, c1.x, c1.y};
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-#pragma unroll
-            for (int p = 0; p < 4; ++p) v[q][p] -= c[q] * w[p];
-    }
-    double *Wo = W + g.y0 * kTile + oi, *Vo = V + g.y0 * kTile + oi;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        *reinterpret_cast<double2*>(Vo + (int64_t)(4 * ty + q) * ld + 2 * tx) = make_double2(v[q][0], v[q][1]);
-        *reinterpret_cast<double2*>(Vo + (int64_t)(4 * ty + q) * ld + 32 + 2 * tx) = make_double2(v[q][2], v[q][3]);
-    }
-    for (int e = tid; e < kTile * kTile; e += kT)
-        Wo[(int64_t)(e / kTile) * ld + e % kTile] = Wt[(e / kTile) * kPanelStride + e % kTile];
+    store(Wt, kPanelStride);
+    __syncthreads();
+    panel_product(X, Wt, 4 * ty, kTile, tx, ty, v);
+    store(V + g.y0 * kTile + oi, ld);
 }
 
-// Step s, the rest: A_ij -= V_i W_j^T on the lower tiles, A_is = V_i, A_ss = -A_ss^-1. 64 x 64 x 64 a
+// Step s, the rest: A_ij -= W_i W_j^T on the lower tiles, A_is = V_i, A_ss = -A_ss^-1. 64 x 64 x 64 a
 // block of 128 threads, 8 x 4 entries a thread from shared memory (columns 2 tx, 2 tx + 1, 32 + ..:
 // 16-byte reads without bank conflicts; 6 of them for 32 multiply-adds). Bound by the FP64 pipe once a
 // step has more tiles than the device has SMs.
@@ -473,7 +536,7 @@ __global__ void __launch_bounds__(kTrailT, 3) k_trail(int s, const CoarseGrid* _
         for (int e = tid; e < kTile * kTile; e += kTrailT) {
             const int r = e / kTile, c = e % kTile;
             double x;
-            if (i == s && j == s) x = piv[(int64_t)blockIdx.y * kTile * kTile + e];
+            if (i == s && j == s) x = -piv[(int64_t)blockIdx.y * kTile * kTile + e];
             else if (j == s) x = Vp[c * ld + oi + r];
             else x = Vp[r * ld + oj + c];
             Ai[(oi + r) * ld + oj + c] = x;
@@ -484,7 +547,7 @@ __global__ void __launch_bounds__(kTrailT, 3) k_trail(int s, const CoarseGrid* _
 #pragma unroll 4
     for (int e = tid; e < kTile * kTile / 2; e += kTrailT) {
         const int t = e / (kTile / 2), q = 2 * (e % (kTile / 2));
-        *reinterpret_cast<double2*>(sv + t * kTile + q) = *reinterpret_cast<const double2*>(Vp + t * ld + oi + q);
+        *reinterpret_cast<double2*>(sv + t * kTile + q) = *reinterpret_cast<const double2*>(Wp + t * ld + oi + q);
         *reinterpret_cast<double2*>(sw + t * kTile + q) = *reinterpret_cast<const double2*>(Wp + t * ld + oj + q);
     }
     const int tx = tid & 15, ty = tid >> 4;
@@ -840,6 +903,7 @@ void Coarse::update(const double* vals, cudaStream_t st) {
     if (!active()) return;
     const unsigned n_inst = (unsigned)grids_.size();
     const int64_t stride = (int64_t)steps_ * kTile, d2 = (int64_t)dof_ * dof_;
+    const double ridge = fp32_ ? kRidge32 : kRidge64;
     const unsigned pg = (unsigned)std::max(1, (nschunks_ + kPairWarps - 1) / kPairWarps);
     int64_t most = 1;  // (coarse node, node within reach, entry) of the largest instance
     for (const CoarseGrid& g : grids_) {
@@ -852,19 +916,19 @@ void Coarse::update(const double* vals, cudaStream_t st) {
     if (dof_ == 3) {
         k_pairs<3><<<pg, kPairWarps * 32, 0, st>>>(nschunks_, schunk_, bpos_, brow_, bcol_, pos_, vals, spart_);
         k_pair_sums<3><<<grid_of(nseg_ * 64 * d2), kT, 0, st>>>(nseg_, schunk_ptr_, spart_);
-        k_dense<3><<<dg, kT, 0, st>>>(d_grids_, table_, schunk_ptr_, spart_, A_, diag_, stride);
+        k_dense<3><<<dg, kT, 0, st>>>(d_grids_, table_, schunk_ptr_, spart_, A_, diag_, stride, ridge);
     } else {
         k_pairs<1><<<pg, kPairWarps * 32, 0, st>>>(nschunks_, schunk_, bpos_, brow_, bcol_, pos_, vals, spart_);
         k_pair_sums<1><<<grid_of(nseg_ * 64 * d2), kT, 0, st>>>(nseg_, schunk_ptr_, spart_);
-        k_dense<1><<<dg, kT, 0, st>>>(d_grids_, table_, schunk_ptr_, spart_, A_, diag_, stride);
+        k_dense<1><<<dg, kT, 0, st>>>(d_grids_, table_, schunk_ptr_, spart_, A_, diag_, stride, ridge);
     }
     CK(cudaGetLastError());
     constexpr int smem = 2 * kTile * kTile * (int)sizeof(double);
-    constexpr int psmem = 2 * kTile * kPanelStride * (int)sizeof(double);
+    constexpr int psmem = 3 * kTile * kPanelStride * (int)sizeof(double);
     CK(cudaFuncSetAttribute(k_trail, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     CK(cudaFuncSetAttribute(k_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, psmem));
     for (int s = 0; s < steps_; ++s) {
-        k_panel<<<dim3(steps_, n_inst), kT, psmem, st>>>(s, d_grids_, A_, diag_, stride, panel_w_, panel_v_, piv_);
+        k_panel<<<dim3(steps_, n_inst), kT, psmem, st>>>(s, d_grids_, A_, diag_, stride, ridge, panel_w_, panel_v_, piv_);
         k_trail<<<dim3(steps_ * (steps_ + 1) / 2, n_inst), kTrailT, smem, st>>>(s, d_grids_, A_, panel_w_, panel_v_, piv_);
     }
     const dim3 mg(2 * steps_, 2 * steps_, n_inst);

@@ -8,7 +8,8 @@
 //    displacement fields, so the smooth error modes that IC(0) leaves are in its range whatever
 //    the mesh is; piecewise rigid modes per aggregate took 1.6x the iterations (Tet4 20^3, 125
 //    parts: 77 against 47, and 237 without a correction);
-//  * E = P^T K P is the exact Galerkin matrix of the assembled FP64 K, held as its dense inverse:
+//  * E = P^T K P is the Galerkin matrix of the assembled FP64 K, with a small ridge (kRidge64), held as its
+//    dense inverse:
 //    an application is one matrix-vector product read at HBM or L2 rate, with no dependent levels.
 // Measured (B200, device solve): Tet10 40^3 mixed 827 -> 68 iterations, 264 -> 31 ms, with 12 ms more
 // set-up; Tet4 20^3 FP64 225 -> 44, 17.0 -> 4.3 ms (+1.4); SIMP Tet4 48^3 519 -> 63, 65 -> 10 ms; Tet4
