@@ -546,11 +546,13 @@ def pcg_bytes_per_iteration(blocks, nb, vb):
     return matrix + vectors
 
 
-# DRAM traffic of the persistent PCG kernel per iteration over its algorithmic bytes, from one ncu
-# capture (dram__bytes_read.sum + dram__bytes_write.sum of one 8-iteration launch, Tet10 30^3:
-# 0.587 GB against 0.560 GB, kept in the profile summary of k_pcg); traffic grows with the blocks, so
-# the ratio scales the capture to the benchmark size.
-PCG_TRAFFIC_RATIO = 0.591 / 0.560
+# DRAM traffic of the persistent PCG kernel per iteration over the bytes of pcg_bytes_parts, from one ncu
+# capture (dram__bytes_read.sum + dram__bytes_write.sum of one 8-iteration launch with one reliable
+# update, Tet10 30^3 mixed: 0.702 GB an iteration against 0.560 GB, profiles/k_pcg_mixed_tet10_30_traffic.md);
+# traffic grows with the blocks, so the ratio scales the capture to the benchmark size. The capture
+# has what pcg_bytes_parts leaves out: the coarse correction's dense inverse (0.020 GB), the row
+# weights (0.007 GB) and the reliable update's FP64 matrix.
+PCG_TRAFFIC_RATIO = 0.702 / 0.560
 
 
 def cpu_baseline(p, tol, iterations_needed, max_iter=5):
@@ -848,9 +850,8 @@ def run_ours(args):
                                                       "ms_ordering", "ms_symbolic", "ms_buffers",
                                                       "ms_assembly", "ms_factor", "ms_solve", "ms_post",
                                                       "ms_download")},
-           "phases_note": ("ms_setup is the host thread (incidence, boundary lists), which runs while the "
-                           "device takes the inputs and orders the nodes; the other phases follow one "
-                           "another (ms_ordering: the device ordering, wall time)")}
+           "phases_note": ("ms_setup is 0 (the analysis runs on the device); the other phases follow one "
+                           "another (ms_ordering: node incidence, graph and ordering, wall time)")}
 
     plain_tet4 = plain_tet4_section(torch, mb, mg, L, args.steps, args.warmup, local)
     # the same configuration at the reference's default tolerance (iterative.rs:9)
@@ -907,7 +908,9 @@ def run_ours(args):
                      "ms_per_iteration": info_m["ms_solve"] / info_m["iterations"],
                      "traffic": PCG_TRAFFIC_RATIO * it_bytes,
                      "traffic_note": "bytes per iteration, ncu DRAM bytes of a Tet10 30^3 launch "
-                                     "scaled by blocks (the k_pcg Tet10 30^3 profile summary)"},
+                                     "scaled by blocks (profiles/k_pcg_mixed_tet10_30_traffic.md); "
+                                     "bytes_per_iteration counts IC(0)-PCG alone, without the coarse "
+                                     "correction's inverse and row weights"},
         "spmv": {"kernel": "k_spmv<float> (SELL 3x3-block SpMV, FP32, standalone)",
                  "achieved": gbs32, "frac": gbs32 / hbm, "bytes_per_launch": bytes32,
                  "ms_per_launch": ms32,

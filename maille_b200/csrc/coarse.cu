@@ -446,7 +446,8 @@ __device__ __forceinline__ void panel_product(const double* P, const double* W, 
 // unknown-major), block s leaves A_ss^-1 = L^-T L^-1 in piv. The update A_ij -= W_i W_j^T is a square: with
 // the tile's explicit inverse, A_ij -= A_is (A_ss^-1 A_sj), the inverse's own rounding, eps / pivot^2,
 // made a matrix of dependent hats indefinite (a graded part of 2x51x6 cells: eigenvalues of P X P^T K from
-// -4200 to 4300).
+// -4200 to 4300). Bound by the tile's chain of 16 dependent steps; 40 us a step at 3993 unknowns, 33 with the
+// explicit inverse and its one product.
 __global__ void __launch_bounds__(kT) k_panel(int s, const CoarseGrid* __restrict__ grids, const double* __restrict__ A,
                                               const double* __restrict__ diag, int64_t diag_stride, double ridge,
                                               double* __restrict__ W, double* __restrict__ V, double* __restrict__ piv) {

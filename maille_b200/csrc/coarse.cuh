@@ -11,12 +11,15 @@
 //  * E = P^T K P is the Galerkin matrix of the assembled FP64 K, with a small ridge (kRidge64), held as its
 //    dense inverse:
 //    an application is one matrix-vector product read at HBM or L2 rate, with no dependent levels.
-// Measured (B200, device solve): Tet10 40^3 mixed 827 -> 68 iterations, 264 -> 31 ms, with 12 ms more
-// set-up; Tet4 20^3 FP64 225 -> 44, 17.0 -> 4.3 ms (+1.4); SIMP Tet4 48^3 519 -> 63, 65 -> 10 ms; Tet4
-// 6^3 63 -> 28, 4.0 -> 2.2 ms. Below 128 rows IC(0) alone stays.
-// The sum is symmetric positive definite, and the PCG's stopping test, statuses and caps are those
-// of the plain preconditioner. The RCM ordering keeps IC(0) alone: it stands for the reference's
-// own iteration counts.
+// Measured (B200, iterations and ms of the PCG alone): Tet10 40^3 mixed 827 -> 65, 264 -> 24.6 ms, with 5 ms
+// more set-up; Tet4 20^3 FP64 225 -> 43, 17.0 -> 2.4 ms; SIMP Tet4 48^3 519 -> 63, 65 -> 7.9 ms; Tet4 6^3
+// 63 -> 28. A part that its supports hold everywhere gains nothing (a plate of 200x200x1 cells clamped on its
+// face: 19 -> 23 iterations); the call is still shorter than before the correction (24.6 -> 9.5 ms).
+// Below 128 rows IC(0) alone stays.
+// The sum is symmetric positive definite: IC(0) is, and E has a ridge that keeps its inverse so in the
+// PCG's precision (kRidge64, kRidge32). The PCG's stopping test, statuses and caps are those of the plain
+// preconditioner. The RCM ordering keeps IC(0) alone: it stands for the reference's own iteration
+// counts. A device without room for the correction keeps IC(0) alone too.
 //
 // Independent instances (the batched solver) get a grid and a dense inverse each.
 #pragma once
@@ -48,7 +51,7 @@ struct CoarseDev {
     int32_t m = 0, ld = 0;
     int32_t kx = 0, ky = 0, kz = 0;
     int32_t nchunks = 0;
-    const T* w = nullptr;               // [4 nb] per row: fx, fy, fz in its cell, code (CoarseCode)
+    const T* w = nullptr;               // [4 nb] per row: fx, fy, fz in its cell, code (kCoarseBase)
     const T* ws = nullptr;              // [4 nb] the same in cell order, code = the row
     const int4* chunk = nullptr;        // [nchunks] (first, end) in the cell order, inside one cell
     const int32_t* cell_chunk = nullptr;  // [cells + 1] first chunk of each cell
@@ -95,8 +98,9 @@ class Coarse {
     // Rows, pattern and grid of the system. xyz: [3 n_nodes] device coordinates; perm: [nb] row ->
     // node; fixmask: [nb] fixed components or null; row_ptr, col: the full pattern, dof x dof blocks.
     // row_inst: [nb] instance of each row or null (one instance). box: [6 instances] min and max
-    // corners; rows_of: rows per instance; rhs: load cases of a batch (its layouts), 0: one system. Does nothing (active() stays false) when no
-    // instance is large enough. Synchronises the stream.
+    // corners; rows_of: rows per instance; rhs: load cases of a batch (its layouts), 0: one system. Does
+    // nothing (active() stays false) when no instance is large enough. Synchronises the stream. Throws
+    // DeviceMemoryFull when there is no room.
     void plan(int dof, bool fp32, int32_t nb, int64_t blocks, const double* xyz, const int32_t* perm,
               const uint8_t* fixmask, const int64_t* row_ptr, const int32_t* col, const int32_t* row_inst,
               const std::vector<double>& box, const std::vector<int64_t>& rows_of, cudaStream_t st, int rhs = 0);
@@ -133,8 +137,7 @@ class Coarse {
     double *spart_ = nullptr, *A_ = nullptr, *diag_ = nullptr, *panel_w_ = nullptr, *panel_v_ = nullptr, *piv_ = nullptr;
 };
 
-// Coarse node and fixed components of a row, packed: base node of its cell in the low 28 bits, fixed
-// mask above.
+// Code of a row: base node of its cell in the low 28 bits, fixed components above.
 constexpr uint32_t kCoarseBase = (1u << 28) - 1u;
 // Cell order: the row in the low 29 bits, fixed mask above.
 constexpr uint32_t kCoarseRow = (1u << 29) - 1u;

@@ -7,7 +7,7 @@
 //   coarse_gather    P^T r of a coarse node: the partial sums of its at most 8 cells, in order;
 //   coarse_apply     y = E^-1 P^T r, one warp per row of the dense inverse, and this thread's
 //                    share of (P^T r) . y, which is r . (P E^-1 P^T r).
-// The caller adds P y to z wherever it reads z next (CoarseHats::add).
+// The caller adds P y to z wherever it reads z next (coarse_interpolate3, coarse_interpolate1).
 #pragma once
 
 #include <cstdint>

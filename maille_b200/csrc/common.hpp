@@ -50,9 +50,12 @@ struct Symbolic {
 
 // The library's own ordering besides those of the ABI: greedy colouring visited by node index, then one
 // pass of iterated greedy (last class first). No searches: with the coarse correction the iteration
-// counts no longer depend on the visit order (Tet4 20^3 47 against 47 in RCM order with two passes,
+// counts of boxes hardly depend on the visit order (Tet4 20^3 47 against 47 in RCM order with two passes,
 // Tet10 14^3 40 / 40, Tet10 18x12x15 44 / 44, with node ids permuted at random 44 / 43 / 47), and it
-// has as few colours (14 against 15 on the Tet10 cube; 16 permuted).
+// has as few colours (14 against 15 on the Tet10 cube; 16 permuted). A call's ms, this / RCM order with two
+// passes: Tet4 20^3 5.8 / 7.7, Tet10 12^3 8.1 / 9.9; with ids permuted at random 6.1 / 8.1 and 8.8 / 10.0; over
+// 200 random parts 0.81 of the time at 1.04 of the iterations (single parts 0.5 to 1.9 of the time: how good
+// IC(0) is in one order or another, and the diagonal shift it takes).
 constexpr int kOrderIndex = 100;
 
 // Sliced 3x3-block layout of one matrix part (see sparse.cuh): K (full rows), L (strictly

@@ -2,8 +2,9 @@
 // C ABI of include/maille_gpu.h.
 //
 // create = FreeSystem::new + Pcg::new (model.rs:1442-1499, iterative.rs:201-207) on the GPU:
-//   symbolic analysis (host, setup.cpp) -> upload -> element integration -> scatter-reduce
-//   assembly -> level-scheduled block IC(0) with the reference's diagonal-shift ladder.
+//   upload -> element integration -> symbolic analysis (analysis.cu, ordering.cu; layout plans on the
+//   host, setup.cpp) -> assembly -> level-scheduled block IC(0) with the reference's diagonal-shift
+//   ladder, the coarse correction's inverse beside it.
 // solve  = FreeSystem::solve + Pcg::solve (model.rs:1502-1516, iterative.rs:210-248), then the
 //   reactions (product, model.rs:586-593) and Gauss-point stresses (model.rs:596-598).
 // The PCG runs in the persistent cooperative kernel of persist.cu: one launch for the initial
